@@ -134,9 +134,10 @@ SW2D_HD void hllc_dip_both(bool blending, double bL, double bR, double phiG, dou
     const double FR = spec_force_dip(bR, phiG, phiR / smax(phiG, kSmallReal), hR, uR);
     f.f2 = L2 * FL - L1 * FR + L1 * L2 * (phiR * R.q - phiL * L.q);
     f.f2 = f.f2 / den;
-    const double vL = x1L * L.r / smax(hL, kSmallReal);
-    const double vR = x1R * R.r / smax(hR, kSmallReal);
-    f.f3 = (f.f1 >= 0) ? f.f1 * vL : f.f1 * vR;
+    // the tangential velocity of the upwind side only: one division instead of two
+    const bool up = f.f1 >= 0;
+    const double vU = (up ? x1L : x1R) * (up ? L.r : R.r) / smax(up ? hL : hR, kSmallReal);
+    f.f3 = f.f1 * vU;
 }
 
 // swDip::hypHllc (dip/swDipHyp.cpp:759-905) and swDip::hypHllcBlending (:908-1083).  Flags

@@ -92,6 +92,47 @@ SW2D_HD double sqrt_z(double x) { return warp_all(x == 0.0) ? x : sqrt(x); }
 
 SW2D_HD double div_z(double x, double d) { return warp_all(x == 0.0) ? x : x / d; }  // d > 0
 
+// sqrt((b - 1) b u u + c c) is c itself for b == 1 (the first term is then +-0 for a finite u) and
+// c = +0 or c c normal: in radix 2 the correctly rounded square root of the rounded square of c
+// is |c| (S. Boldo, "Stupid is as stupid does: taking the square root of the square of a
+// floating-point number", 2015).  A Boussinesq coefficient of 1 is the usual map, so this takes four
+// of the eight square roots off a MUSCL-EVR edge.
+SW2D_HD bool root_is_c(double b, double u, double c)
+{
+    return b == 1.0 && fabs(u) < 1.0e300 && ((c > 1.0e-140 && c < 1.0e150) || (c == 0.0 && !std::signbit(c)));
+}
+
+// x / d for a divisor whose correctly rounded reciprocal y = RN(1 / d) is known in advance: a first
+// quotient, one Newton correction that makes it faithful, and Markstein's final correction, which
+// then rounds it correctly (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  The residuals are taken as d q - x, so that a zero keeps its sign.
+// Needs x = +-0, or x, d, x / d and the residuals far from the ends of the exponent range (the
+// caller's business): then the result is the IEEE quotient.
+SW2D_HD double div_known(double x, double d, double y)
+{
+    using std::fma;
+    double q = x * y;
+    q = fma(-fma(d, q, -x), y, q);
+    return fma(-fma(d, q, -x), y, q);
+}
+
+// |x| in [2^-498, 2^498), or x = +-0: a difference of levels that div_known's slope terms take
+// (with lengths in slope_length_ok's range)
+SW2D_HD bool div_range_ok(double x)
+{
+#if defined(__CUDA_ARCH__)
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+#else
+    const unsigned hi = (unsigned)(sw2d_pm_bits(x) >> 32) & 0x7fffffffu;
+#endif
+    return hi - (525u << 20) < (996u << 20) || x == 0.0;
+}
+
+// lengths between centroids, and their components (which may be 0), for which every quotient and
+// residual of the slope terms stays normal when div_range_ok holds for the level difference
+SW2D_HD bool slope_length_ok(double v) { return fabs(v) >= 1.0e-30 && fabs(v) <= 1.0e30; }
+SW2D_HD bool slope_component_ok(double v) { return v == 0.0 || (fabs(v) >= 1.0e-60 && fabs(v) <= 1.0e30); }
+
 // First-order rotated state of a cell on an edge (swSpHypGodunov.cpp:17-35 and 44-76; the
 // boundary loop of swSpHypMusclEvr.cpp:142-159 is the same expression).
 SW2D_HD SideState godunov_side(double h, double q, double r, double zb, double b, double nx, double ny)
@@ -109,7 +150,7 @@ SW2D_HD SideState godunov_side(double h, double q, double r, double zb, double b
         u = s.q / d;
         c = sqrt(kGravity * h);
     }
-    const double root = sqrt_z((b - 1.0) * b * u * u + c * c);
+    const double root = warp_all(root_is_c(b, u, c)) ? c : sqrt_z((b - 1.0) * b * u * u + c * c);
     s.lm = b * u - root;
     s.lp = b * u + root;
     return s;
@@ -137,7 +178,7 @@ SW2D_HD SideState evr_side(bool left, double h, double q, double r, double zb, d
         cl = sqrt(kGravity * hd);
         ul = ql / hd;
         vl = rl / hd;
-        root1 = sqrt((b - 1.0) * b * ul * ul + cl * cl);
+        root1 = warp_all(root_is_c(b, ul, cl)) ? cl : sqrt((b - 1.0) * b * ul * ul + cl * cl);
     }
     const double lmv = b * ul - root1;
     const double lpv = b * ul + root1;
@@ -158,7 +199,7 @@ SW2D_HD SideState evr_side(bool left, double h, double q, double r, double zb, d
     s.r = hr * vl;
     const double u = div_z(s.q, smax(hr, kSmallReal));
     const double c = sqrt_z(kGravity * hr);
-    const double root = sqrt_z((b - 1.0) * b * u * u + c * c);
+    const double root = warp_all(root_is_c(b, u, c)) ? c : sqrt_z((b - 1.0) * b * u * u + c * c);
     s.lm = b * u - root;
     s.lp = b * u + root;
     return s;
@@ -239,9 +280,10 @@ SW2D_HD EdgeFlux hllc(bool blending, double bL, double bR, double phiL, double p
         double FL = spec_force(bL, phiL, hL, uL);
         double FR = spec_force(bR, phiR, hR, uR);
         f.f2 = (L2 * (FL + f.sl) - L1 * (FR - f.sr) + L1 * L2 * (phiR * R.q - phiL * L.q)) / den;
-        double vL = L.r / smax(hL, kSmallReal);
-        double vR = R.r / smax(hR, kSmallReal);
-        f.f3 = (f.f1 >= 0) ? bL * f.f1 * vL : bR * f.f1 * vR;
+        // the tangential velocity of the upwind side only: one division instead of two
+        const bool up = f.f1 >= 0;
+        const double vU = (up ? L.r : R.r) / smax(up ? hL : hR, kSmallReal);
+        f.f3 = (up ? bL : bR) * f.f1 * vU;
     } else if (rhs) {
         f.f1 = 0.;
         f.f2 = 0.;

@@ -131,6 +131,7 @@ struct DevMesh {
     const int2* eslot;       // {slot of (L, e), slot of (R, e)}
     const double2* nxy;
     const double2* mxy;
+    const double4* egeo;     // {dist of the centroids, 1 / dist, mx, my} (MUSCL slopes)
     const double4* emc;      // {mx - cx_L, my - cy_L, mx - cx_R, my - cy_R}
     const double* len;
     const double2* coef;     // {coefL, coefR}
@@ -177,6 +178,7 @@ struct DevMesh {
     double h_min, phi_min, cfl_max, dt_max, dt_map, v_max, fr_max;
     DryConsts dry;
     int neg_detect;
+    int geo_plain;   // the mesh's lengths allow div_known in the slopes (slope_length_ok)
     int rev_update;  // the cell update walks its blocks from the last cells to the first
     // dt reduction scratch
     double* part;
@@ -257,8 +259,8 @@ struct sw2d_handle {
     double4* bflux_buf = nullptr;
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
-    int edge_variant = 0;   // index into kVariants (sw2d_autotune)
-    int slope_variant = 2;
+    int edge_variant = 3;   // index into kVariants (sw2d_create's rule, sw2d_autotune)
+    int slope_variant = 4;
     sw2d::AdjointState* adj = nullptr;  // recorded trajectory, checkpoints and adjoint buffers
     int adj_flush_branch = 0;           // option "adjoint_flush_branch"
     int adj_keep_nonfinite = 0;         // option "adjoint_keep_nonfinite"

@@ -189,6 +189,24 @@ __global__ void k_edge_coefficients(DevMesh m, double2* coef, double4* bgeo)
     }
 }
 
+// statics of an internal edge: midpoint - centroid of L and R, the first difference of the MUSCL-EVR
+// reconstruction (swSpHypMusclEvr.cpp:197-207); with `geo`, the distance of its cells' centroids and
+// the slope weight 1 / dist (:31-38) beside the midpoint, `odd` set where the slopes may not divide
+// by that distance with div_known
+__global__ void k_edge_geometry(DevMesh m, double4* emc, double4* geo, unsigned* odd)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m.ni) return;
+    const int2 lr = m.lr[i];
+    const double2 a = m.cxy[lr.x], b = m.cxy[lr.y], mp = m.mxy[i];
+    emc[i] = make_double4(mp.x - a.x, mp.y - a.y, mp.x - b.x, mp.y - b.y);
+    if (!geo) return;
+    const double dx = b.x - a.x, dy = b.y - a.y;
+    const double dist = sqrt(dx * dx + dy * dy);
+    geo[i] = make_double4(dist, 1.0 / dist, mp.x, mp.y);
+    if (!(slope_length_ok(dist) && slope_component_ok(dx) && slope_component_ok(dy))) *odd = 1u;
+}
+
 // caller numbering <-> internal numbering
 __global__ void k_gather_state(const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
                                const int* __restrict__ perm, const double4* __restrict__ cst, double4* st, int n)
@@ -635,6 +653,11 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
     h->p = *params;
     h->model = dip ? kModelDip : ddp ? kModelDdp : kModelSp;
     h->dissipation = ((dip && dip->momentum_dissipation) || (ddp && ddp->momentum_dissipation)) ? 1 : 0;
+    // launch variants before any autotuning, measured at 1M and 4M cells: k_slopes 128 x 8 (41 us at
+    // 1M; 256 x 4: 41, 256 x 3: 48); k_edges 128 x 4 with the MUSCL-EVR scheme (80 us; 128 x 8: 83 with
+    // spills, 256 x 3: 82), 128 x 8 with Godunov, which needs fewer registers (56 us; 128 x 4: 58,
+    // 256 x 3: 62)
+    h->edge_variant = params->scheme == SW2D_SCHEME_GODUNOV ? 4 : 3;
     h->nc = mesh->cell_nb;
     h->ni = mesh->edge_int_nb;
     h->nb = mesh->edge_bnd_nb;
@@ -751,13 +774,6 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
         mxy[i] = make_double2(mesh->edge_int_mx[oe], mesh->edge_int_my[oe]);
         len[i] = mesh->edge_int_length[oe];
     }
-    // per internal edge, midpoint - centroid of L and R: the first difference of the MUSCL-EVR
-    // reconstruction (swSpHypMusclEvr.cpp:197-207), a static of the mesh computed once
-    std::vector<double4> emc(ni);
-    for (int64_t i = 0; i < ni; i++) {
-        const double2 a = cxy[lr[i].x], b = cxy[lr[i].y], mp = mxy[i];
-        emc[i] = make_double4(mp.x - a.x, mp.y - a.y, mp.x - b.x, mp.y - b.y);
-    }
     std::vector<int> bcell(nb), bbc(nb);
     std::vector<double4> bgeo(nb);
     for (int64_t i = 0; i < nb; i++) {
@@ -819,7 +835,6 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
     UP(lr, m.lr);
     UP(nxy, m.nxy);
     UP(mxy, m.mxy);
-    UP(emc, m.emc);
     UP(len, m.len);
     UP(bcell, m.bcell);
     UP(bbc, m.bbc);
@@ -860,6 +875,11 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
     double2* coef_d = nullptr;
     if ((rc = dev_alloc(h, ni, &coef_d))) return bail(rc);
     m.coef = coef_d;
+    double4 *emc_d = nullptr, *egeo_d = nullptr;
+    if ((rc = dev_alloc(h, ni, &emc_d))) return bail(rc);
+    m.emc = emc_d;
+    if (params->scheme == SW2D_SCHEME_MUSCL_EVR && (rc = dev_alloc(h, ni, &egeo_d))) return bail(rc);
+    m.egeo = egeo_d;
     // persistent balance slots start at zero, like the reference's resized flux vectors
     if ((rc = dev_alloc(h, nslot, &m.slot)) || (rc = dev_alloc(h, nslot, &m.slot_w)) ||
         (rc = dev_alloc(h, nc, &m.slope)) || (rc = dev_alloc(h, nc / 32 + grid_for(nc) + 2, &m.part)) ||
@@ -897,8 +917,16 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
     if (cudaMemcpyAsync(h->ctrl, h->ctrl_host, sizeof(Ctrl), cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
         return bail(fail(h, SW2D_E_CUDA, "ctrl upload"));
     k_edge_coefficients<<<grid_for(ni + nb), kBlock, 0, h->stream>>>(m, coef_d, bgeo_d);
+    unsigned odd = 1;  // set by an edge whose lengths div_known may not take (the staging array serves as the flag)
+    if (ni > 0) {
+        unsigned* flag = reinterpret_cast<unsigned*>(h->stage);
+        k_edge_geometry<<<grid_for(ni), kBlock, 0, h->stream>>>(m, emc_d, egeo_d, flag);
+        if (cudaMemcpyAsync(&odd, flag, sizeof(odd), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess)
+            return bail(fail(h, SW2D_E_CUDA, "edge geometry"));
+    }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess || cudaGetLastError() != cudaSuccess)
         return bail(fail(h, SW2D_E_CUDA, "initialisation kernels failed"));
+    m.geo_plain = odd ? 0 : 1;
     if ((rc = noalloc_prepare(h))) return bail(rc);
     if (!ddp) {
         // tables for the tiles of the fused step, which is an option ("fused_step"; the tiles
