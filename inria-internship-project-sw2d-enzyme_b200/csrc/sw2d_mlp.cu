@@ -4,17 +4,15 @@
 // stand-alone inference, and the DIP cell-update kernel with the network inside
 // (k_update_closure, further down) for the closure in a model's step.
 //
-// k_umma_gemm computes, for a tile of 128 rows per CTA, D = A * B^T with A [M x K] and B [N x K]
-// (bf16, row-major, K contiguous), K looped in chunks of 64 through shared memory (K-major
-// core-matrix layout of umma.cuh), N <= 256 in one MMA row, and an epilogue that reads D from
-// TMEM (each thread one row) and applies one of:
+// k_umma_gemm (stand-alone inference) computes, for a tile of 128 rows per CTA, D = A * B^T with
+// A [M x K] and B [N x K] (bf16, row-major, K contiguous), K looped in chunks of 64 through shared
+// memory (K-major core-matrix layout of umma.cuh), N <= 256 in one MMA row, and an epilogue that
+// reads D from TMEM (each thread one row) and applies one of:
 //   kEpiStore     out = D + bias                       (fp32)
 //   kEpiGelu      z = D + bias -> pre (fp32), gelu(z) -> act (bf16)      forward hidden layer
-//   kEpiGeluGrad  g = D * gelu'(pre) -> act (bf16)                       backward hidden layer
-// One layer's forward is one launch; the backward data gradients dH = dZ W are the same kernel
-// with the transposed weights; the weight gradients dW = dZ^T H are the same kernel with K = the
-// batch (operands transposed by k_transpose).  Every reduction runs in a fixed order: training
-// is deterministic.
+// Training is one kernel, k_mlp_train: forward, loss, backward and weight gradients of 128-row
+// tiles, with the pre-activations kept in TMEM and the activations in shared memory.  Every
+// reduction runs in a fixed order: training is deterministic.
 //
 // Every wait on the tensor core is bounded; a wait that runs out sets the status word, waits
 // once more (bounded) for the MMA in flight, frees the TMEM and returns.
@@ -40,7 +38,7 @@ constexpr int kMaxN = 128;
 constexpr long long kWaitPolls = 1LL << 26;  // ~ seconds of polling: far beyond any MMA here
 constexpr unsigned kStatusTimeout = 1u;
 
-enum { kEpiStore = 0, kEpiGelu = 1, kEpiGeluGrad = 2 };
+enum { kEpiStore = 0, kEpiGelu = 1 };
 
 struct GemmArgs {
     const __nv_bfloat16* A;
@@ -48,8 +46,7 @@ struct GemmArgs {
     int M, N, K, lda, ldb;
     const float* bias;       // [N] or null
     float* out;              // fp32 [M x ldo] (kEpiStore: D + bias; kEpiGelu: pre-activation)
-    __nv_bfloat16* act;      // bf16 [M x lda_out] (kEpiGelu, kEpiGeluGrad)
-    const float* pre;        // kEpiGeluGrad: pre-activation [M x ldo]
+    __nv_bfloat16* act;      // bf16 [M x lda_out] (kEpiGelu)
     int ldo, ldact;
     int n_valid;             // columns written (<= N)
     uint32_t tmem_cols;      // power of two >= max(32, N)
@@ -200,12 +197,10 @@ __global__ void __launch_bounds__(128) k_umma_gemm(GemmArgs g)
             const float d = __uint_as_float(v[j]);
             if (kMode == kEpiStore) {
                 g.out[(size_t)r * g.ldo + n] = d + (g.bias ? g.bias[n] : 0.0f);
-            } else if (kMode == kEpiGelu) {
+            } else {
                 const float z = d + (g.bias ? g.bias[n] : 0.0f);
                 g.out[(size_t)r * g.ldo + n] = z;
                 g.act[(size_t)r * g.ldact + n] = __float2bfloat16_rn(gelu(z));
-            } else {
-                g.act[(size_t)r * g.ldact + n] = __float2bfloat16_rn(d * gelu_grad(g.pre[(size_t)r * g.ldo + n]));
             }
         }
     }
@@ -213,23 +208,6 @@ __global__ void __launch_bounds__(128) k_umma_gemm(GemmArgs g)
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, g.tmem_cols);
     if (!ok && tid == 0) atomicOr(g.status, kStatusTimeout);
-}
-
-// out[c * ldo + r] = in[r * ldi + c] for r < rows, c < cols (bf16)
-__global__ void k_transpose(const __nv_bfloat16* __restrict__ in, int ldi, int rows, int cols, __nv_bfloat16* out,
-                            int ldo)
-{
-    __shared__ __nv_bfloat16 t[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int r = by + j, c = bx + threadIdx.x;
-        t[j][threadIdx.x] = (r < rows && c < cols) ? in[(size_t)r * ldi + c] : __float2bfloat16_rn(0.0f);
-    }
-    __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int c = bx + j, r = by + threadIdx.x;
-        if (c < cols && r < rows) out[(size_t)c * ldo + r] = t[threadIdx.x][j];
-    }
 }
 
 uint32_t tmem_cols_for(int n)
@@ -250,6 +228,7 @@ constexpr int kIn = 10, kInPad = 16, kHid = 64, kOut = 2, kOutPad = 16;
 // parameter vector: W1 [64 x 10], b1 [64], W2 [64 x 64], b2 [64], W3 [2 x 64], b3 [2]
 constexpr int kNW1 = kHid * kIn, kNB1 = kHid, kNW2 = kHid * kHid, kNB2 = kHid, kNW3 = kOut * kHid, kNB3 = kOut;
 constexpr int kNParams = kNW1 + kNB1 + kNW2 + kNB2 + kNW3 + kNB3;
+constexpr int kPartStride = (kNParams + 31) / 32 * 32;  // floats of one CTA's partial gradient
 
 }  // namespace sw2d
 
@@ -260,21 +239,24 @@ struct sw2d_mlp {
     std::string err;
     unsigned* status = nullptr;
     long long first_wait = kWaitPolls;  // sw2d_mlp_set_wait_polls
-    // fp32 master parameters, Adam moments, gradients
-    float *p = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr;
+    int sms = 0;
+    // fp32 master parameters, Adam moments; the gradient (result buffer of sw2d_mlp_loss_grad:
+    // gradient, loss partials, status word) and its pinned host copy
+    float *p = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *host = nullptr;
+    float* part = nullptr;  // per-CTA partial gradients [parts x kPartStride]
+    int64_t parts = 0;
     // bf16 operand copies: W1 [64 x 16] (inputs padded), W2 [64 x 64], W3 [16 x 64] (outputs padded),
     // and the transposed W2t [64 x 64], W3t [64 x 16] for the backward data gradients
     __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr, *w2t = nullptr, *w3t = nullptr;
     float *b1 = nullptr, *b2 = nullptr, *b3 = nullptr;  // fp32 biases (b3 padded to 16)
     // feature normalisation (x - mean) / std, target scale y * ystd + ymean
     float xmean[sw2d::kIn], xstd[sw2d::kIn], ymean[sw2d::kOut], ystd[sw2d::kOut];
-    // work buffers for a batch of up to cap rows
-    int64_t cap = 0;
-    __nv_bfloat16 *x = nullptr, *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
-    __nv_bfloat16 *tA = nullptr, *tB = nullptr;
-    float *z1 = nullptr, *z2 = nullptr, *y = nullptr, *t = nullptr, *loss = nullptr;
-    float *raw = nullptr;  // raw features [cap x 10]
-    float *gw1 = nullptr, *gw2 = nullptr, *gw3 = nullptr, *gb = nullptr;  // weight and bias gradients
+    // work buffers for inference on up to cap rows and training on up to tcap rows
+    int64_t cap = 0, tcap = 0;
+    __nv_bfloat16 *x = nullptr, *h1 = nullptr, *h2 = nullptr;
+    float *z1 = nullptr, *z2 = nullptr, *y = nullptr;
+    float *raw = nullptr;                                          // raw features [cap x 10]
+    float *traw = nullptr, *t = nullptr, *se = nullptr;  // training: features, targets, squared errors
     int64_t step = 0;
 };
 
@@ -354,84 +336,353 @@ __global__ void k_features(const float* __restrict__ raw, int64_t n, int64_t npa
     }
 }
 
-// normalised targets [n x 16 padded]; loss gradient dY = 2 (y - t) / (n * 2) and per-block
-// squared-error partial sums (deterministic reduction on the host)
-__global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t, int64_t n, int64_t npad,
-                       __nv_bfloat16* dy, float* partial)
+// ------------------------------------------------------------------------------------------
+// k_mlp_train: loss and parameter gradient of a batch, persistent over tiles of 128 rows (thread i
+// of the CTA owns row i of the tile, which is TMEM lane i).  Per tile, on the tensor core:
+//   Z1 = X W1^T, Z2 = H1 W2^T, Y = H2 W3^T           forward; H = bf16(gelu(Z + b)) by the epilogues
+//   dH2 = dY W3, dH1 = dZ2 W2                        backward; dZ = bf16(dH gelu'(Z + b))
+//   Ga += [dZ2 dZ1]^T [H1 X 1],  Gb += [H2 1]^T dY   weight and bias gradients, K = the tile's rows
+// Z1, Z2 stay in TMEM for the backward epilogues, and Ga, Gb accumulate there over the CTA's tiles;
+// the activations stay in shared memory, row-major for the next layer and transposed (K = rows) for
+// the gradients.  Column 10 of the transposed X, a padding column of the forward operand, holds the
+// ones that make the bias gradients.  Each CTA leaves one partial gradient; k_mlp_reduce adds them
+// in CTA order.  The kernel is bound by the latency of one tile's chain of seven MMA rounds and
+// their epilogues.  A training step of 4,096 rows through the C ABI (copies, Adam and the parameters
+// read back included) takes 100 us; with one GEMM launch per layer and direction, transposes, weight
+// gradients on one CTA (3 x 221 us) and column sums on one thread per column (3 x 201 us) it took 1,041.
+// ------------------------------------------------------------------------------------------
+struct TrainArgs {
+    const float* raw;    // [n x 10]
+    const float* t;      // [n x 2]
+    int64_t n;
+    int ntiles;
+    Norm nm;
+    const __nv_bfloat16 *w1, *w2, *w3, *w2t, *w3t;
+    const float *b1, *b2, *b3;
+    float* se;           // [n] squared error of each row
+    float* part;         // [gridDim.x x kPartStride]
+    unsigned* status;
+    long long first_wait;
+};
+
+// shared-memory plan of k_mlp_train (byte offsets, every operand 1 KB aligned)
+constexpr uint32_t kTX = 0, kTH1 = kTX + 4096, kTH2 = kTH1 + 16384, kTDY = kTH2 + 16384, kTDZ2 = kTDY + 4096,
+                   kTA = kTDZ2 + 16384, kTB = kTA + 32768, kTC = kTB + 20480, kTD = kTC + 32768, kTW1 = kTD + 4096,
+                   kTW2 = kTW1 + 2048, kTW3 = kTW2 + 8192, kTW2t = kTW3 + 2048, kTW3t = kTW2t + 8192,
+                   kTBias = kTW3t + 2048, kTBar = kTBias + 1024, kTrainSmem = kTBar + 64;
+// TMEM columns: Z1, Z2, Y, dH, Ga (80 columns), Gb
+constexpr uint32_t kCZ1 = 0, kCZ2 = 64, kCY = 128, kCD = 192, kCGa = 256, kCGb = 384, kTrainCols = 512;
+
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b)
+{
+    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&p);
+}
+
+// columns j, j + 1 (j even) of this thread's row r into the transposed tile at `base`: lanes r and
+// r ^ 1 exchange halves, so that each stores one 4-byte pair of rows
+__device__ __forceinline__ void put_transposed(char* base, int j, int r, uint32_t pair)
+{
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, pair, 1);
+    const int odd = r & 1;
+    const uint32_t v = odd ? __byte_perm(other, pair, 0x7632) : __byte_perm(pair, other, 0x5410);
+    *reinterpret_cast<uint32_t*>(base + core_offset(j + odd, r & ~1, kTileM)) = v;
+}
+
+// copies a row-major [rows x cols] bf16 matrix into its core-matrix layout
+__device__ __forceinline__ void stage_weights(char* dst, const __nv_bfloat16* src, int rows, int cols, int tid)
+{
+    const int nv = cols / 8;
+    for (int i = tid; i < rows * nv; i += kTileM) {
+        const int n = i / nv, c = (i - n * nv) * 8;
+        *reinterpret_cast<uint4*>(dst + core_offset(n, c, cols)) = *reinterpret_cast<const uint4*>(src + n * cols + c);
+    }
+}
+
+__global__ void __launch_bounds__(kTileM) k_mlp_train(TrainArgs a)
 {
     using namespace sw2d;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    float se = 0.0f;
-    if (i < npad) {
-        for (int k = 0; k < kOutPad; k++) {
-            float g = 0.0f;
-            if (i < n && k < kOut) {
-                const float d = y[i * kOutPad + k] - t[i * kOut + k];
-                se += d * d;
-                g = 2.0f * d / (float)(n * kOut);
+    extern __shared__ __align__(1024) char sm[];
+    __shared__ uint32_t tmem_holder;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kTBar);
+    float* sb = reinterpret_cast<float*>(sm + kTBias);  // b1 [64], b2 [64], b3 [16]
+    if (warp == 0) {
+        tmem_alloc(&tmem_holder, kTrainCols);
+        tmem_relinquish();
+    }
+    if (tid == 0) mbar_init(bar, 1);
+    stage_weights(sm + kTW1, a.w1, kHid, kInPad, tid);
+    stage_weights(sm + kTW2, a.w2, kHid, kHid, tid);
+    stage_weights(sm + kTW3, a.w3, kOutPad, kHid, tid);
+    stage_weights(sm + kTW2t, a.w2t, kHid, kHid, tid);
+    stage_weights(sm + kTW3t, a.w3t, kHid, kOutPad, tid);
+    if (tid < kHid) {
+        sb[tid] = a.b1[tid];
+        sb[kHid + tid] = a.b2[tid];
+    }
+    if (tid < kOutPad) sb[2 * kHid + tid] = a.b3[tid];
+    // rows 64 .. 127 of [H2 1]^T: a row of ones, then zeros
+    const uint32_t ones = pack_bf16(1.0f, 1.0f);
+    for (int j = kHid; j < kTileM; j += 2)
+        *reinterpret_cast<uint32_t*>(sm + kTC + core_offset(j + (tid & 1), tid & ~1, kTileM)) =
+            (j == kHid && !(tid & 1)) ? ones : 0u;
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = tmem_holder;
+    const uint32_t lane_base = tmem + ((uint32_t)(32 * warp) << 16);
+    const uint32_t s0 = smem_u32(sm);
+    uint32_t phase = 0;
+    bool ok = true;
+    // one round: every thread's operand writes visible, thread 0 issues, all wait; false ends the tile
+    auto round = [&](auto&& issue) -> bool {
+        fence_before_sync();
+        fence_proxy_async();
+        if (!__syncthreads_and(ok)) return false;
+        if (tid == 0) {
+            fence_after_sync();
+            issue();
+            mma_commit(bar);
+        }
+        if (!mbar_wait(bar, phase, a.first_wait)) {
+            ok = false;
+            mbar_wait(bar, phase, kWaitPolls);  // the MMA still in flight: give it time once more
+        }
+        phase ^= 1u;
+        fence_after_sync();
+        return true;
+    };
+    // D (+)= A B^T over K in steps of 16
+    auto gemm_k = [&](uint32_t col, uint32_t A, uint32_t B, int K, int N, bool acc) {
+        const uint32_t id = idesc_bf16_f32(kTileM, N);
+        for (int k = 0; k < K / 16; k++)
+            mma_bf16(tmem + col, smem_desc(s0 + A + 256u * k, K), smem_desc(s0 + B + 256u * k, K), id,
+                     (acc || k > 0) ? 1u : 0u);
+    };
+    bool first = true;
+    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+        const int64_t row = (int64_t)tile * kTileM + tid;
+        const bool valid = row < a.n;
+        {   // normalised features: the first layer's operand, and its transpose with the column of ones
+            float xv[kInPad];
+#pragma unroll
+            for (int k = 0; k < kInPad; k++)
+                xv[k] = (k < kIn && valid) ? (a.raw[row * kIn + k] - a.nm.xmean[k < kIn ? k : 0]) / a.nm.xstd[k < kIn ? k : 0] : 0.0f;
+#pragma unroll
+            for (int c = 0; c < kInPad; c += 8)
+                *reinterpret_cast<uint4*>(sm + kTX + core_offset(tid, c, kInPad)) =
+                    make_uint4(pack_bf16(xv[c], xv[c + 1]), pack_bf16(xv[c + 2], xv[c + 3]),
+                               pack_bf16(xv[c + 4], xv[c + 5]), pack_bf16(xv[c + 6], xv[c + 7]));
+            xv[kIn] = 1.0f;
+#pragma unroll
+            for (int c = 0; c < kInPad; c += 2) put_transposed(sm + kTB, kHid + c, tid, pack_bf16(xv[c], xv[c + 1]));
+        }
+        if (!round([&] { gemm_k(kCZ1, kTX, kTW1, kInPad, kHid, false); })) break;
+        // hidden layers: H = bf16(gelu(Z + b)), row-major and transposed
+#pragma unroll 1
+        for (int layer = 0; layer < 2; layer++) {
+            const float* b = sb + layer * kHid;
+            const uint32_t zc = layer == 0 ? kCZ1 : kCZ2, hs = layer == 0 ? kTH1 : kTH2, ht = layer == 0 ? kTB : kTC;
+#pragma unroll 1
+            for (int c0 = 0; c0 < kHid; c0 += 16) {
+                uint32_t v[16], hv[8];
+                tmem_ld16(lane_base + zc + (uint32_t)c0, v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    float g0, g1;
+                    gelu_bias2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]), b[c0 + 2 * j], b[c0 + 2 * j + 1],
+                               g0, g1);
+                    hv[j] = pack_bf16(g0, g1);
+                    put_transposed(sm + ht, c0 + 2 * j, tid, hv[j]);
+                }
+                *reinterpret_cast<uint4*>(sm + hs + core_offset(tid, c0, kHid)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                *reinterpret_cast<uint4*>(sm + hs + core_offset(tid, c0 + 8, kHid)) = make_uint4(hv[4], hv[5], hv[6], hv[7]);
             }
-            dy[i * kOutPad + k] = __float2bfloat16_rn(g);
+            if (layer == 0) {
+                if (!round([&] { gemm_k(kCZ2, kTH1, kTW2, kHid, kHid, false); })) break;
+            } else {
+                if (!round([&] { gemm_k(kCY, kTH2, kTW3, kHid, kOutPad, false); })) break;
+            }
+        }
+        {   // loss of the row and dY = 2 (y - t) / (2 n)
+            uint32_t v[16];
+            tmem_ld16(lane_base + kCY, v);
+            tmem_wait_ld();
+            float g[kOut] = {0.0f, 0.0f}, se = 0.0f;
+            if (valid) {
+#pragma unroll
+                for (int k = 0; k < kOut; k++) {
+                    const float tn = (a.t[row * kOut + k] - a.nm.ymean[k]) / a.nm.ystd[k];
+                    const float d = (__uint_as_float(v[k]) + sb[2 * kHid + k]) - tn;
+                    se += d * d;
+                    g[k] = 2.0f * d / (float)(a.n * kOut);
+                }
+                a.se[row] = se;
+            }
+            const uint32_t pair = pack_bf16(g[0], g[1]);
+            *reinterpret_cast<uint4*>(sm + kTDY + core_offset(tid, 0, kOutPad)) = make_uint4(pair, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(sm + kTDY + core_offset(tid, 8, kOutPad)) = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int j = 0; j < kOutPad; j += 2) put_transposed(sm + kTD, j, tid, j == 0 ? pair : 0u);
+        }
+        if (!round([&] { gemm_k(kCD, kTDY, kTW3t, kOutPad, kHid, false); })) break;
+        // dZ2 then dZ1 = bf16(dH gelu'(Z + b)); dZ2 is also the operand of the next data gradient
+#pragma unroll 1
+        for (int layer = 1; layer >= 0; layer--) {
+            const float* b = sb + layer * kHid;
+            const uint32_t zc = layer == 0 ? kCZ1 : kCZ2;
+#pragma unroll 1
+            for (int c0 = 0; c0 < kHid; c0 += 16) {
+                uint32_t d[16], z[16], hv[8];
+                tmem_ld16(lane_base + kCD + (uint32_t)c0, d);
+                tmem_ld16(lane_base + zc + (uint32_t)c0, z);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int c = 2 * j;
+                    hv[j] = pack_bf16(__uint_as_float(d[c]) * gelu_grad(__uint_as_float(z[c]) + b[c0 + c]),
+                                      __uint_as_float(d[c + 1]) * gelu_grad(__uint_as_float(z[c + 1]) + b[c0 + c + 1]));
+                    put_transposed(sm + kTA, (layer == 0 ? kHid : 0) + c0 + c, tid, hv[j]);
+                }
+                if (layer == 1) {
+                    *reinterpret_cast<uint4*>(sm + kTDZ2 + core_offset(tid, c0, kHid)) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
+                    *reinterpret_cast<uint4*>(sm + kTDZ2 + core_offset(tid, c0 + 8, kHid)) =
+                        make_uint4(hv[4], hv[5], hv[6], hv[7]);
+                }
+            }
+            if (layer == 1 && !round([&] { gemm_k(kCD, kTDZ2, kTW2t, kHid, kHid, false); })) break;
+        }
+        if (!round([&] {
+                gemm_k(kCGa, kTA, kTB, kTileM, kHid + kInPad, !first);
+                gemm_k(kCGb, kTC, kTD, kTileM, kOutPad, !first);
+            }))
+            break;
+        first = false;
+    }
+    ok = __syncthreads_and(ok);
+    if (ok) {
+        // lane i: Ga row i ([dZ2]_i . [H1 X 1] or [dZ1]_{i-64} . ...), Gb row i ([H2]_i . dY, row 64: sum dY)
+        float* out = a.part + (size_t)blockIdx.x * kPartStride;
+        const int o = tid & (kHid - 1);
+        const bool two = tid < kHid;
+        uint32_t v[16];
+#pragma unroll 1
+        for (int c0 = 0; c0 < kHid; c0 += 16) {
+            tmem_ld16(lane_base + kCGa + (uint32_t)c0, v);
+            tmem_wait_ld();
+            if (two) {
+                float4* w = reinterpret_cast<float4*>(out + kNW1 + kNB1 + o * kHid + c0);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    w[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+            }
+        }
+        tmem_ld16(lane_base + kCGa + kHid, v);
+        tmem_wait_ld();
+        if (two) {
+            out[kNW1 + kNB1 + kNW2 + o] = __uint_as_float(v[kIn]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kIn; k++) out[o * kIn + k] = __uint_as_float(v[k]);
+            out[kNW1 + o] = __uint_as_float(v[kIn]);
+        }
+        tmem_ld16(lane_base + kCGb, v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int k = 0; k < kOut; k++) {
+            if (two) out[kNW1 + kNB1 + kNW2 + kNB2 + k * kHid + o] = __uint_as_float(v[k]);
+            else if (tid == kHid) out[kNParams - kNB3 + k] = __uint_as_float(v[k]);
         }
     }
-    __shared__ float s[256];
-    s[threadIdx.x] = se;
+    fence_before_sync();
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if (warp == 0) tmem_dealloc(tmem, kTrainCols);
+    if (!ok && tid == 0) atomicOr(a.status, kStatusTimeout);
+}
+
+// Gradient = the partials in CTA order, four interleaved chains per parameter; the blocks after
+// `nb_param` reduce the rows' squared errors, 256 rows each (the host adds those); the status word
+// goes behind them.
+__global__ void __launch_bounds__(256) k_mlp_reduce(const float* __restrict__ part, int nparts, int nb_param,
+                                                    const float* __restrict__ se, int64_t n, float* out,
+                                                    const unsigned* status, int nb_loss)
+{
+    using namespace sw2d;
+    if ((int)blockIdx.x < nb_param) {
+        const int i = blockIdx.x * 256 + threadIdx.x;
+        if (i < kNParams) {
+            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            int c = 0;
+            for (; c + 4 <= nparts; c += 4)
+#pragma unroll
+                for (int k = 0; k < 4; k++) s[k] += part[(size_t)(c + k) * kPartStride + i];
+            for (int k = 0; c + k < nparts; k++) s[k] += part[(size_t)(c + k) * kPartStride + i];
+            out[i] = (s[0] + s[1]) + (s[2] + s[3]);
+        }
+        return;
+    }
+    const int b = (int)blockIdx.x - nb_param;
+    const int64_t r = (int64_t)b * 256 + threadIdx.x;
+    __shared__ float s[256];
+    s[threadIdx.x] = r < n ? se[r] : 0.0f;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) s[threadIdx.x] += s[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
+    if (threadIdx.x == 0) {
+        out[kNParams + b] = s[0];
+        if (b == 0) out[kNParams + nb_loss] = __uint_as_float(*status);
+    }
 }
 
-// column sums of a bf16 [n x ld] array (bias gradients), one thread per column, fixed order
-__global__ void k_colsum(const __nv_bfloat16* __restrict__ a, int64_t n, int ld, int cols, float* out)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.0f;
-    for (int64_t i = 0; i < n; i++) s += __bfloat162float(a[i * ld + c]);
-    out[c] = s;
-}
-
-// gradient vector from the weight-gradient GEMM outputs (fp32 [rows x cols] with padding)
-__global__ void k_pack_grad(const float* __restrict__ gw1, const float* __restrict__ gw2,
-                            const float* __restrict__ gw3, const float* __restrict__ gb, float* grad)
+// Adam on one parameter per thread, and the refresh of its bf16 operand copies (the padding of the
+// copies is zero from their creation and stays so)
+__global__ void k_adam(float* p, float* m1, float* m2, const float* __restrict__ g, float lr, float b1, float b2, float eps,
+                       float c1, float c2, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3, __nv_bfloat16* w2t,
+                       __nv_bfloat16* w3t, float* sb1, float* sb2, float* sb3)
 {
     using namespace sw2d;
-    for (int i = threadIdx.x; i < kNW1; i += blockDim.x) grad[i] = gw1[(i / kIn) * kInPad + (i % kIn)];
-    for (int i = threadIdx.x; i < kNB1; i += blockDim.x) grad[kNW1 + i] = gb[i];
-    for (int i = threadIdx.x; i < kNW2; i += blockDim.x) grad[kNW1 + kNB1 + i] = gw2[i];
-    for (int i = threadIdx.x; i < kNB2; i += blockDim.x) grad[kNW1 + kNB1 + kNW2 + i] = gb[kHid + i];
-    for (int i = threadIdx.x; i < kNW3; i += blockDim.x) grad[kNW1 + kNB1 + kNW2 + kNB2 + i] = gw3[i];
-    for (int i = threadIdx.x; i < kNB3; i += blockDim.x) grad[kNParams - kNB3 + i] = gb[2 * kHid + i];
-}
-
-__global__ void k_adam(float* p, float* m1, float* m2, const float* __restrict__ g, int n, float lr, float b1,
-                       float b2, float eps, float c1, float c2)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kNParams) return;
     const float gi = g[i];
     const float a = b1 * m1[i] + (1.0f - b1) * gi;
     const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
     m1[i] = a;
     m2[i] = b;
-    p[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+    const float v = p[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+    p[i] = v;
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    if (i < kNW1) {
+        w1[(i / kIn) * kInPad + i % kIn] = h;
+    } else if ((i -= kNW1) < kNB1) {
+        sb1[i] = v;
+    } else if ((i -= kNB1) < kNW2) {
+        w2[i] = h;
+        w2t[(i % kHid) * kHid + i / kHid] = h;
+    } else if ((i -= kNW2) < kNB2) {
+        sb2[i] = v;
+    } else if ((i -= kNB2) < kNW3) {
+        w3[i] = h;
+        w3t[(i % kHid) * kOutPad + i / kHid] = h;
+    } else {
+        sb3[i - kNW3] = v;
+    }
 }
 
 int gemm(sw2d_mlp* m, int mode, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N, int K,
-         const float* bias, float* out, int ldo, __nv_bfloat16* act, int ldact, const float* pre, int n_valid,
-         cudaStream_t stream = nullptr)
+         const float* bias, float* out, int ldo, __nv_bfloat16* act, int ldact, int n_valid)
 {
-    if (!stream) stream = m->stream;
     if (N % 16 || N > kMaxN || K % 16 || K <= 0 || M <= 0 || (lda % 8) || (ldb % 8))
         return mlp_fail(m, SW2D_E_ARG, "gemm: shape outside the kernel's contract");
-    GemmArgs g{A, B, M, N, K, lda, ldb, bias, out, act, pre, ldo, ldact, n_valid, tmem_cols_for(N), m->status,
+    GemmArgs g{A, B, M, N, K, lda, ldb, bias, out, act, ldo, ldact, n_valid, tmem_cols_for(N), m->status,
                m->first_wait};
     const unsigned grid = (unsigned)((M + kTileM - 1) / kTileM);
-    if (mode == kEpiStore) k_umma_gemm<kEpiStore><<<grid, 128, 0, stream>>>(g);
-    else if (mode == kEpiGelu) k_umma_gemm<kEpiGelu><<<grid, 128, 0, stream>>>(g);
-    else k_umma_gemm<kEpiGeluGrad><<<grid, 128, 0, stream>>>(g);
+    if (mode == kEpiStore) k_umma_gemm<kEpiStore><<<grid, 128, 0, m->stream>>>(g);
+    else k_umma_gemm<kEpiGelu><<<grid, 128, 0, m->stream>>>(g);
     MCK(cudaGetLastError());
     return SW2D_OK;
 }
@@ -443,14 +694,37 @@ int ensure_cap(sw2d_mlp* m, int64_t n)
     if (npad <= m->cap) return SW2D_OK;
     int rc;
     if ((rc = malloc_dev(m, npad * kInPad, &m->x)) || (rc = malloc_dev(m, npad * kHid, &m->h1)) ||
-        (rc = malloc_dev(m, npad * kHid, &m->h2)) || (rc = malloc_dev(m, npad * kOutPad, &m->dy)) ||
-        (rc = malloc_dev(m, npad * kHid, &m->dz2)) || (rc = malloc_dev(m, npad * kHid, &m->dz1)) ||
-        (rc = malloc_dev(m, npad * kHid, &m->tA)) || (rc = malloc_dev(m, npad * kHid, &m->tB)) ||
-        (rc = malloc_dev(m, npad * kHid, &m->z1)) || (rc = malloc_dev(m, npad * kHid, &m->z2)) ||
-        (rc = malloc_dev(m, npad * kOutPad, &m->y)) || (rc = malloc_dev(m, npad * kOut, &m->t)) ||
-        (rc = malloc_dev(m, npad / 256 + 2, &m->loss)) || (rc = malloc_dev(m, npad * kIn, &m->raw)))
+        (rc = malloc_dev(m, npad * kHid, &m->h2)) || (rc = malloc_dev(m, npad * kHid, &m->z1)) ||
+        (rc = malloc_dev(m, npad * kHid, &m->z2)) || (rc = malloc_dev(m, npad * kOutPad, &m->y)) ||
+        (rc = malloc_dev(m, npad * kIn, &m->raw)))
         return rc;
     m->cap = npad;
+    return SW2D_OK;
+}
+
+// floats of the result buffer of a batch of n rows: gradient, loss partials (256 rows each), status
+size_t result_floats(int64_t n) { return (size_t)sw2d::kNParams + (size_t)((n + 255) / 256) + 1; }
+
+// training buffers for n rows (the pinned copy is replaced together with the device buffer)
+int ensure_train(sw2d_mlp* m, int64_t n)
+{
+    using namespace sw2d;
+    if (n <= m->tcap) return SW2D_OK;
+    int rc;
+    if (m->host) MCK(cudaFreeHost(m->host));
+    m->host = nullptr;
+    MCK(cudaMallocHost(&m->host, result_floats(n) * sizeof(float)));
+    float* grad = nullptr;
+    const int64_t parts = std::min<int64_t>((n + kTileM - 1) / kTileM, m->sms);  // one per CTA
+    if (parts > m->parts) {
+        if ((rc = malloc_dev(m, parts * kPartStride, &m->part))) return rc;
+        m->parts = parts;
+    }
+    if ((rc = malloc_dev(m, n * kIn, &m->traw)) || (rc = malloc_dev(m, n * kOut, &m->t)) ||
+        (rc = malloc_dev(m, n, &m->se)) || (rc = malloc_dev(m, result_floats(n), &grad)))
+        return rc;
+    m->grad = grad;
+    m->tcap = n;
     return SW2D_OK;
 }
 
@@ -470,13 +744,13 @@ int forward(sw2d_mlp* m, int64_t npad)
     using namespace sw2d;
     int rc;
     if ((rc = gemm(m, kEpiGelu, m->x, kInPad, m->w1, kInPad, (int)npad, kHid, kInPad, m->b1, m->z1, kHid, m->h1, kHid,
-                   nullptr, kHid)))
+                   kHid)))
         return rc;
     if ((rc = gemm(m, kEpiGelu, m->h1, kHid, m->w2, kHid, (int)npad, kHid, kHid, m->b2, m->z2, kHid, m->h2, kHid,
-                   nullptr, kHid)))
+                   kHid)))
         return rc;
     return gemm(m, kEpiStore, m->h2, kHid, m->w3, kHid, (int)npad, kOutPad, kHid, m->b3, m->y, kOutPad, nullptr, 0,
-                nullptr, kOutPad);
+                kOutPad);
 }
 
 }  // namespace
@@ -498,6 +772,9 @@ int sw2d_mlp_create(int device, const float* params, const float* norm, sw2d_mlp
     };
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(SW2D_E_CUDA);
+    if (cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem) != cudaSuccess)
+        return bail(SW2D_E_CUDA);
     for (int k = 0; k < kIn; k++) {
         m->xmean[k] = norm[k];
         m->xstd[k] = norm[kIn + k];
@@ -515,9 +792,7 @@ int sw2d_mlp_create(int device, const float* params, const float* norm, sw2d_mlp
         (rc = malloc_dev(m, kOutPad * kHid, &m->w3)) || (rc = malloc_dev(m, kHid * kHid, &m->w2t)) ||
         (rc = malloc_dev(m, kHid * kOutPad, &m->w3t)) || (rc = malloc_dev(m, kHid, &m->b1)) ||
         (rc = malloc_dev(m, kHid, &m->b2)) || (rc = malloc_dev(m, kOutPad, &m->b3)) ||
-        (rc = malloc_dev(m, 1, &m->status)) || (rc = malloc_dev(m, kHid * kInPad, &m->gw1)) ||
-        (rc = malloc_dev(m, kHid * kHid, &m->gw2)) || (rc = malloc_dev(m, kOutPad * kHid, &m->gw3)) ||
-        (rc = malloc_dev(m, 2 * kHid + kOutPad, &m->gb)))
+        (rc = malloc_dev(m, 1, &m->status)))
         return bail(rc);
     if (cudaMemcpyAsync(m->p, params, kNParams * sizeof(float), cudaMemcpyHostToDevice, m->stream) != cudaSuccess)
         return bail(SW2D_E_CUDA);
@@ -533,6 +808,7 @@ int sw2d_mlp_destroy(sw2d_mlp* m)
     cudaSetDevice(m->device);
     if (m->stream) cudaStreamSynchronize(m->stream);
     for (void* p : m->allocs) cudaFree(p);
+    if (m->host) cudaFreeHost(m->host);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return SW2D_OK;
@@ -605,64 +881,45 @@ int sw2d_mlp_loss_grad(sw2d_mlp* m, const float* features, const float* targets,
     using namespace sw2d;
     if (!m || !features || !targets || n <= 0) return SW2D_E_ARG;
     MCK(cudaSetDevice(m->device));
-    int rc = ensure_cap(m, n);
+    int rc = ensure_train(m, n);
     if (rc) return rc;
-    const int64_t npad = (n + kTileM - 1) / kTileM * kTileM;
-    std::vector<float> tn((size_t)n * kOut);
-    for (int64_t i = 0; i < n; i++)
-        for (int k = 0; k < kOut; k++) tn[i * kOut + k] = (targets[i * kOut + k] - m->ymean[k]) / m->ystd[k];
-    MCK(cudaMemcpyAsync(m->raw, features, n * kIn * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    MCK(cudaMemcpyAsync(m->t, tn.data(), n * kOut * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    k_features<<<(unsigned)((npad + 255) / 256), 256, 0, m->stream>>>(m->raw, n, npad, norm_of(m), m->x);
-    if ((rc = forward(m, npad))) return rc;
-    const unsigned lb = (unsigned)((npad + 255) / 256);
-    k_loss<<<lb, 256, 0, m->stream>>>(m->y, m->t, n, npad, m->dy, m->loss);
-    // backward data gradients on the tensor cores: dZ2 = (dY W3) * gelu'(Z2), dZ1 = (dZ2 W2) * gelu'(Z1)
-    if ((rc = gemm(m, kEpiGeluGrad, m->dy, kOutPad, m->w3t, kOutPad, (int)npad, kHid, kOutPad, nullptr, nullptr, kHid,
-                   m->dz2, kHid, m->z2, kHid)))
-        return rc;
-    if ((rc = gemm(m, kEpiGeluGrad, m->dz2, kHid, m->w2t, kHid, (int)npad, kHid, kHid, nullptr, nullptr, kHid, m->dz1,
-                   kHid, m->z1, kHid)))
-        return rc;
-    // weight gradients on the tensor cores with K = the batch: dW = dZ^T H
-    float *gw1 = m->gw1, *gw2 = m->gw2, *gw3 = m->gw3, *gb = m->gb;
-    const int K = (int)npad;
-    dim3 tb(32, 8);
-    auto transpose = [&](const __nv_bfloat16* a, int cols, __nv_bfloat16* o) {
-        dim3 gr((unsigned)((cols + 31) / 32), (unsigned)((npad + 31) / 32));
-        k_transpose<<<gr, tb, 0, m->stream>>>(a, cols, (int)npad, cols, o, (int)npad);
-    };
-    transpose(m->dy, kOutPad, m->tA);
-    transpose(m->h2, kHid, m->tB);
-    if ((rc = gemm(m, kEpiStore, m->tA, K, m->tB, K, kOutPad, kHid, K, nullptr, gw3, kHid, nullptr, 0, nullptr, kHid)))
-        return rc;
-    transpose(m->dz2, kHid, m->tA);
-    transpose(m->h1, kHid, m->tB);
-    if ((rc = gemm(m, kEpiStore, m->tA, K, m->tB, K, kHid, kHid, K, nullptr, gw2, kHid, nullptr, 0, nullptr, kHid)))
-        return rc;
-    transpose(m->dz1, kHid, m->tA);
-    transpose(m->x, kInPad, m->tB);
-    if ((rc = gemm(m, kEpiStore, m->tA, K, m->tB, K, kHid, kInPad, K, nullptr, gw1, kInPad, nullptr, 0, nullptr,
-                   kInPad)))
-        return rc;
-    k_colsum<<<1, 64, 0, m->stream>>>(m->dz1, npad, kHid, kHid, gb);
-    k_colsum<<<1, 64, 0, m->stream>>>(m->dz2, npad, kHid, kHid, gb + kHid);
-    k_colsum<<<1, 64, 0, m->stream>>>(m->dy, npad, kOutPad, kOutPad, gb + 2 * kHid);
-    k_pack_grad<<<1, 256, 0, m->stream>>>(gw1, gw2, gw3, gb, m->grad);
+    MCK(cudaMemcpyAsync(m->traw, features, n * kIn * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    MCK(cudaMemcpyAsync(m->t, targets, n * kOut * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    TrainArgs a;
+    a.raw = m->traw;
+    a.t = m->t;
+    a.n = n;
+    a.ntiles = (int)((n + kTileM - 1) / kTileM);
+    a.nm = norm_of(m);
+    a.w1 = m->w1;
+    a.w2 = m->w2;
+    a.w3 = m->w3;
+    a.w2t = m->w2t;
+    a.w3t = m->w3t;
+    a.b1 = m->b1;
+    a.b2 = m->b2;
+    a.b3 = m->b3;
+    a.se = m->se;
+    a.part = m->part;
+    a.status = m->status;
+    a.first_wait = m->first_wait;
+    const int grid = std::min(a.ntiles, m->sms);
+    k_mlp_train<<<grid, kTileM, kTrainSmem, m->stream>>>(a);
+    const int nbp = (kNParams + 255) / 256, nbl = (int)((n + 255) / 256);
+    k_mlp_reduce<<<nbp + nbl, 256, 0, m->stream>>>(m->part, grid, nbp, m->se, n, m->grad, m->status, nbl);
     MCK(cudaGetLastError());
-    std::vector<float> part(lb);
-    MCK(cudaMemcpyAsync(part.data(), m->loss, lb * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    if (grad_out) MCK(cudaMemcpyAsync(grad_out, m->grad, kNParams * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+    MCK(cudaMemcpyAsync(m->host, m->grad, result_floats(n) * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
     MCK(cudaStreamSynchronize(m->stream));
     unsigned st = 0;
-    MCK(cudaMemcpy(&st, m->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    std::memcpy(&st, m->host + kNParams + nbl, sizeof(st));
     if (st) {
         // reported once: the kernel that ran out freed its TMEM, and the object stays usable
         MCK(cudaMemset(m->status, 0, sizeof(unsigned)));
         return mlp_fail(m, SW2D_E_CUDA, "tensor-core wait ran out");
     }
+    if (grad_out) std::memcpy(grad_out, m->host, kNParams * sizeof(float));
     double s = 0.0;
-    for (float v : part) s += v;
+    for (int i = 0; i < nbl; i++) s += m->host[kNParams + i];
     if (loss) *loss = s / (double)(n * kOut);
     return SW2D_OK;
 }
@@ -677,9 +934,8 @@ int sw2d_mlp_adam_step(sw2d_mlp* m, float lr)
     m->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, (float)m->step), c2 = 1.0f - std::pow(b2, (float)m->step);
-    k_adam<<<(kNParams + 255) / 256, 256, 0, m->stream>>>(m->p, m->m1, m->m2, m->grad, kNParams, lr, b1, b2, 1e-8f,
-                                                           c1, c2);
-    k_refresh_weights<<<1, 256, 0, m->stream>>>(m->p, m->w1, m->w2, m->w3, m->w2t, m->w3t, m->b1, m->b2, m->b3);
+    k_adam<<<(kNParams + 63) / 64, 64, 0, m->stream>>>(m->p, m->m1, m->m2, m->grad, lr, b1, b2, 1e-8f, c1, c2, m->w1, m->w2,
+                                                       m->w3, m->w2t, m->w3t, m->b1, m->b2, m->b3);
     MCK(cudaGetLastError());
     MCK(cudaStreamSynchronize(m->stream));
     return SW2D_OK;
