@@ -42,7 +42,7 @@ struct sw2d_batch {
     // work-queue form
     sw2d::QueueState* queue = nullptr;
     int mode = 0;  // SW2D_BATCH_BRANCHES or SW2D_BATCH_QUEUE
-    int q_variant = 3, q_cells = 4096, q_edges = 4096;  // 128 threads x 6 CTAs per SM, the C4 ensemble's best
+    int q_variant = 3, q_cells = 4096, q_edges = 4096;  // 128 threads x 6 CTAs per SM; tiles by queue_tile_rule
     cudaGraphExec_t qgraph = nullptr;
     int qgraph_steps = 0;
     std::string err;
@@ -185,6 +185,9 @@ int sw2d_batch_create(sw2d_handle* const* members, int n_members, sw2d_batch** o
             return bail(bfail(b, SW2D_E_CUDA, "member stream synchronisation failed"));
     std::string why;
     if (queue_eligible(members, n_members, why)) {
+        int64_t cells = 0;
+        for (sw2d_handle* h : b->members) cells += h->nc;
+        b->q_cells = b->q_edges = queue_tile_rule(cells);
         if (queue_build(b->queue, members, n_members, b->q_variant, b->q_cells, b->q_edges, why) == SW2D_OK) b->mode = 1;
         else return bail(bfail(b, SW2D_E_CUDA, why));
     }

@@ -384,6 +384,19 @@ int queue_build(QueueState*& q, sw2d_handle* const* members, int n, int variant,
     return SW2D_OK;
 }
 
+// Cells (edges) per tile for an ensemble of `cells` cells in all: a power of two near one tile per
+// resident CTA and phase, 128 .. 4096.  Smaller tiles pay a CTA's item overhead too often, larger ones
+// make each phase of a member a serial chain: 424k cells in 24 members, us per step with tiles of
+// 128 / 256 / 512 / 1024 / 4096: 137 / 111 / 105 / 161 / 457; 21k cells in 6 members: 30 / 40 / 60 / 99 /
+// 323; 1.7M cells in 100 members: 559 / 446 / 395 / 369 / 598; 12.2M cells in 256 members: 4096.
+int queue_tile_rule(int64_t cells)
+{
+    const int64_t ctas = 148 * 6;
+    int tile = 128;
+    while (tile < 4096 && (int64_t)tile * ctas * 3 < cells * 2) tile *= 2;
+    return tile;
+}
+
 // Enqueues on `stream` the launch that advances every member by `steps` steps: the members'
 // counters and the ticket counter are zeroed first (both captured in a graph by the caller).
 int queue_launch(QueueState* q, int steps, cudaStream_t stream)

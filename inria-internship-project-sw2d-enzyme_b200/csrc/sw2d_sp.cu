@@ -316,6 +316,19 @@ struct Variant {
 constexpr Variant kVariants[] = {{256, 3}, {256, 2}, {256, 4}, {128, 4}, {128, 8}, {512, 1}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
+// The variant of k_edges before any autotuning, where the lines between the measured ones lie (us per
+// launch, Gaussian bumps and channel): MUSCL-EVR SP 128 x 4 at every size (1.5M cells: 116; 256 x 3: 117,
+// lake 127 against 133); Godunov SP needs fewer registers, 128 x 8 (1.5M: 78; 256 x 3: 88), with too few
+// blocks to use them below 100k cells (50k: 9.4; 256 x 3: 8.4); DIP carries more per edge, MUSCL-EVR
+// 128 x 4 (300k: 38; 256 x 3: 39) until the grid is many waves deep (500k: 64 against 60, 3M: 322
+// against 298), Godunov 128 x 4 (3M: 191; 256 x 3: 193, 128 x 8: 199).  The DDP set-up sets its own.
+int default_edge_variant(int model, int scheme, int64_t cells)
+{
+    const bool godunov = scheme == SW2D_SCHEME_GODUNOV;
+    if (model == kModelDip) return godunov || cells < 400000 ? 3 : 0;
+    return !godunov ? 3 : cells < 100000 ? 0 : 4;
+}
+
 template <int kScheme, bool kBlending, int kModel, int V>
 void launch_edges_v(sw2d_handle* h, const DevMesh& m, unsigned n)
 {
@@ -653,11 +666,7 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
     h->p = *params;
     h->model = dip ? kModelDip : ddp ? kModelDdp : kModelSp;
     h->dissipation = ((dip && dip->momentum_dissipation) || (ddp && ddp->momentum_dissipation)) ? 1 : 0;
-    // launch variants before any autotuning, measured at 1M and 4M cells: k_slopes 128 x 8 (41 us at
-    // 1M; 256 x 4: 41, 256 x 3: 48); k_edges 128 x 4 with the MUSCL-EVR scheme (80 us; 128 x 8: 83 with
-    // spills, 256 x 3: 82), 128 x 8 with Godunov, which needs fewer registers (56 us; 128 x 4: 58,
-    // 256 x 3: 62)
-    h->edge_variant = params->scheme == SW2D_SCHEME_GODUNOV ? 4 : 3;
+    h->edge_variant = default_edge_variant(h->model, params->scheme, mesh->cell_nb);
     h->nc = mesh->cell_nb;
     h->ni = mesh->edge_int_nb;
     h->nb = mesh->edge_bnd_nb;
