@@ -27,6 +27,7 @@
 #ifndef SW2D_PORTABLE_MATH_H
 #define SW2D_PORTABLE_MATH_H
 
+#include <math.h>
 #include <stdint.h>
 
 #if defined(__CUDACC__)
@@ -55,6 +56,33 @@ SW2D_PM_FN double sw2d_pm_from_bits(uint64_t b)
     double x;
     memcpy(&x, &b, sizeof x);
     return x;
+#endif
+}
+
+/* x / d for d > 0, with the same bits.  A zero numerator leaves the inline sequence of the CUDA
+ * division for its general routine, some 500 cycles away, and zeros are everywhere in a flow at rest
+ * and at its limiters: they divide d by d instead and the result is x itself (+-0, or x / d unchanged
+ * where d is not positive). */
+SW2D_PM_FN double sw2d_div(double x, double d)
+{
+#if defined(__CUDA_ARCH__)
+    const bool z = x == 0.0 && d > 0.0;
+    const double q = (z ? d : x) / d;
+    return z ? x : q;
+#else
+    return x / d;
+#endif
+}
+
+/* the square root, zeros likewise kept off the general routine */
+SW2D_PM_FN double sw2d_sqrt(double x)
+{
+#if defined(__CUDA_ARCH__)
+    const bool z = x == 0.0;
+    const double r = sqrt(z ? 1.0 : x);
+    return z ? x : r;
+#else
+    return sqrt(x);
 #endif
 }
 
@@ -165,7 +193,7 @@ SW2D_PM_FN double sw2d_cbrt(double x)
     }
     const double t = (j == 0) ? m : ((j == 1) ? m * 2.0 : m * 4.0);
     double y = (0.75 + 0.25 * m) * ((j == 0) ? 1.0 : ((j == 1) ? 1.26 : 1.5874));
-    for (int it = 0; it < 5; it++) y = y - (y * y * y - t) / (3.0 * (y * y));
+    for (int it = 0; it < 5; it++) y = y - sw2d_div(y * y * y - t, 3.0 * (y * y));
     const double r = y * sw2d_pm_pow2(k);
     return sw2d_pm_from_bits(sw2d_pm_bits(r) | sign);
 }

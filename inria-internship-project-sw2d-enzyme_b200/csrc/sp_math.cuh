@@ -37,6 +37,7 @@ constexpr unsigned kStatusHllcConfig = 2u;
 constexpr unsigned kStatusNegDepth = 4u;
 constexpr unsigned kStatusBcType = 8u;
 constexpr unsigned kStatusBcFr = 16u;
+constexpr unsigned kStatusRunWait = 1u << 16;  // a wait of the run kernel ran out (sw2d_run.cu)
 constexpr unsigned kStatusUnsupported = 32u;  // a case the reverse kernels do not handle
 
 SW2D_HD double smax(double a, double b) { return (a < b) ? b : a; }
@@ -88,9 +89,34 @@ SW2D_HD bool warp_all(bool p)
 #endif
 }
 
-SW2D_HD double sqrt_z(double x) { return warp_all(x == 0.0) ? x : sqrt(x); }
+// How the edge routines divide and take roots where a zero numerator or argument is possible; the
+// bits are the same.  DivPlain: the plain operations, for kernels with many warps per SM, which hide
+// the detour a zero takes on the GPU (sw2d_div says which) better than they issue the instructions to
+// avoid it (k_edges, Godunov, 1M cells: 57 us plain, 61 with DivZero).  DivZero: for kernels bound by
+// the latency of one warp's chain (a division 125 cycles, 425 with a zero in the warp, 160 with
+// sw2d_div).
+struct DivPlain {
+    static constexpr bool kVote = true;  // whole warps at rest skip their divisions
+    static SW2D_HD double div(double x, double d) { return x / d; }
+    static SW2D_HD double root(double x) { return sqrt(x); }
+};
+struct DivZero {
+    static constexpr bool kVote = false;
+    static SW2D_HD double div(double x, double d) { return sw2d_div(x, d); }
+    static SW2D_HD double root(double x) { return sw2d_sqrt(x); }
+};
 
-SW2D_HD double div_z(double x, double d) { return warp_all(x == 0.0) ? x : x / d; }  // d > 0
+template <class D>
+SW2D_HD double sqrt_z(double x)
+{
+    return D::kVote && warp_all(x == 0.0) ? x : D::root(x);
+}
+
+template <class D>
+SW2D_HD double div_z(double x, double d)  // d > 0
+{
+    return D::kVote && warp_all(x == 0.0) ? x : D::div(x, d);
+}
 
 // sqrt((b - 1) b u u + c c) is c itself for b == 1 (the first term is then +-0 for a finite u) and
 // c = +0 or c c normal: in radix 2 the correctly rounded square root of the rounded square of c
@@ -135,6 +161,7 @@ SW2D_HD bool slope_component_ok(double v) { return v == 0.0 || (fabs(v) >= 1.0e-
 
 // First-order rotated state of a cell on an edge (swSpHypGodunov.cpp:17-35 and 44-76; the
 // boundary loop of swSpHypMusclEvr.cpp:142-159 is the same expression).
+template <class D = DivPlain>
 SW2D_HD SideState godunov_side(double h, double q, double r, double zb, double b, double nx, double ny)
 {
     SideState s;
@@ -143,14 +170,14 @@ SW2D_HD SideState godunov_side(double h, double q, double r, double zb, double b
     s.r = -q * ny + r * nx;
     const double d = smax(h, kSmallReal);
     double u, c;
-    if (warp_all(h == 0.0 && s.q == 0.0)) {  // d == 1e-16 > 0; sqrt(g * +-0) == g * +-0
+    if (D::kVote && warp_all(h == 0.0 && s.q == 0.0)) {  // d == 1e-16 > 0; sqrt(g * +-0) == g * +-0
         u = s.q;
         c = kGravity * h;
     } else {
-        u = s.q / d;
-        c = sqrt(kGravity * h);
+        u = div_z<D>(s.q, d);
+        c = D::root(kGravity * h);
     }
-    const double root = warp_all(root_is_c(b, u, c)) ? c : sqrt_z((b - 1.0) * b * u * u + c * c);
+    const double root = warp_all(root_is_c(b, u, c)) ? c : sqrt_z<D>((b - 1.0) * b * u * u + c * c);
     s.lm = b * u - root;
     s.lp = b * u + root;
     return s;
@@ -161,6 +188,7 @@ SW2D_HD SideState godunov_side(double h, double q, double r, double zb, double b
 // cell.  `left` selects max(0,.) (L side) or min(0,.) (R side) for the wave speeds; dt is the
 // previous step's time step; (dmx, dmy) = edge midpoint - cell centroid, the first difference the
 // reference evaluates in `mx - cx - 0.5 * l * dt * nx` (a static of the mesh).
+template <class D = DivPlain>
 SW2D_HD SideState evr_side(bool left, double h, double q, double r, double zb, double b, double zc,
                                               double sx, double sy, double dmx, double dmy,
                                               double nx, double ny, double dt, const DryConsts& k)
@@ -168,7 +196,7 @@ SW2D_HD SideState evr_side(bool left, double h, double q, double r, double zb, d
     const double ql = q * nx + r * ny;
     const double rl = r * nx - q * ny;
     double cl, ul, vl, root1;
-    if (warp_all(!(kSmallReal < h) && ql == 0.0 && rl == 0.0 && b < 1.0e308)) {  // b >= 1 and finite
+    if (D::kVote && warp_all(!(kSmallReal < h) && ql == 0.0 && rl == 0.0 && b < 1.0e308)) {  // b >= 1 and finite
         cl = k.c0;
         ul = ql;
         vl = rl;
@@ -176,8 +204,13 @@ SW2D_HD SideState evr_side(bool left, double h, double q, double r, double zb, d
     } else {
         const double hd = smax(kSmallReal, h);
         cl = sqrt(kGravity * hd);
-        ul = ql / hd;
-        vl = rl / hd;
+        if (D::kVote && warp_all(ql == 0.0 && rl == 0.0)) {  // water at rest
+            ul = ql;
+            vl = rl;
+        } else {
+            ul = D::div(ql, hd);
+            vl = D::div(rl, hd);
+        }
         root1 = warp_all(root_is_c(b, ul, cl)) ? cl : sqrt((b - 1.0) * b * ul * ul + cl * cl);
     }
     const double lmv = b * ul - root1;
@@ -197,9 +230,9 @@ SW2D_HD SideState evr_side(bool left, double h, double q, double r, double zb, d
     s.z = hr + zb;
     s.q = hr * ul;
     s.r = hr * vl;
-    const double u = div_z(s.q, smax(hr, kSmallReal));
-    const double c = sqrt_z(kGravity * hr);
-    const double root = warp_all(root_is_c(b, u, c)) ? c : sqrt_z((b - 1.0) * b * u * u + c * c);
+    const double u = div_z<D>(s.q, smax(hr, kSmallReal));
+    const double c = sqrt_z<D>(kGravity * hr);
+    const double root = warp_all(root_is_c(b, u, c)) ? c : sqrt_z<D>((b - 1.0) * b * u * u + c * c);
     s.lm = b * u - root;
     s.lp = b * u + root;
     return s;
@@ -212,6 +245,7 @@ struct EdgeFlux {
 
 // swSp::hypHllc (swSpHyp.cpp:664-821) and swSp::hypHllcBlending (swSpHyp.cpp:824-998).
 // Flags kStatusHllcConfig for the configuration the reference rejects (:728-739).
+template <class D = DivPlain>
 SW2D_HD EdgeFlux hllc(bool blending, double bL, double bR, double phiL, double phiR, double zbL,
                                          double zbR, const SideState& L, const SideState& R, double h_min,
                                          double phi_min)
@@ -247,12 +281,16 @@ SW2D_HD EdgeFlux hllc(bool blending, double bL, double bR, double phiL, double p
     }
     if (both) {
         double uL, uR;
-        if (blending) {
-            uL = L.q / smax(hL, kSmallReal);
-            uR = R.q / smax(hR, kSmallReal);
+        const bool rest = D::kVote && warp_all(L.q == 0.0 && R.q == 0.0 && L.r == 0.0 && R.r == 0.0);
+        if (rest) {
+            uL = L.q;
+            uR = R.q;
+        } else if (blending) {
+            uL = D::div(L.q, smax(hL, kSmallReal));
+            uR = D::div(R.q, smax(hR, kSmallReal));
         } else {
-            uL = L.q / smax(kSmallReal, hL);
-            uR = R.q / smax(kSmallReal, hR);
+            uL = D::div(L.q, smax(kSmallReal, hL));
+            uR = D::div(R.q, smax(kSmallReal, hR));
         }
         double L1 = smin(L.lm, smin(R.lm, 0.));
         double L2 = smax(L.lp, smax(R.lp, 0.));
@@ -262,27 +300,28 @@ SW2D_HD EdgeFlux hllc(bool blending, double bL, double bR, double phiL, double p
         if (blending) {
             double alpha_h = 0.0;
             if (fabs(zbL - zbR) > kSmallReal) alpha_h = smax(0.0, smin(1.0, (L.z - R.z) / (zbL - zbR)));
-            double F1h = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (hR - hL)) / den;
-            double F1z = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)) / den;
+            double F1h = D::div(phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (hR - hL)), den);
+            double F1z = D::div(phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)), den);
             f.f1 = alpha_h * F1h + (1.0 - alpha_h) * F1z;
             double fact = 0.5 * smin(phiL, phiR) * (hL + hR);
             double s2z = (phiR * hR * hR - phiL * hL * hL) * 0.5 + fact * (L.z - R.z);
             double s2h = (zbL > zbR) ? phiR * hR * (zbL - zbR) : phiL * hL * (zbL - zbR);
             s2 = alpha_h * s2h + (1.0 - alpha_h) * s2z;
         } else {
-            f.f1 = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)) / den;
+            f.f1 = sw2d_div(phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)), den);
             double fact = 0.5 * smin(phiL, phiR) * (hL + hR);
             s2 = (phiR * hR * hR - phiL * hL * hL) * 0.5 + fact * (L.z - R.z);
         }
-        s2 = s2 * kGravity / den;
+        s2 = D::div(s2 * kGravity, den);
         f.sl = -L1 * s2;
         f.sr = L2 * s2;
         double FL = spec_force(bL, phiL, hL, uL);
         double FR = spec_force(bR, phiR, hR, uR);
-        f.f2 = (L2 * (FL + f.sl) - L1 * (FR - f.sr) + L1 * L2 * (phiR * R.q - phiL * L.q)) / den;
+        f.f2 = D::div(L2 * (FL + f.sl) - L1 * (FR - f.sr) + L1 * L2 * (phiR * R.q - phiL * L.q), den);
         // the tangential velocity of the upwind side only: one division instead of two
         const bool up = f.f1 >= 0;
-        const double vU = (up ? L.r : R.r) / smax(up ? hL : hR, kSmallReal);
+        const double rU = up ? L.r : R.r;
+        const double vU = rest ? rU : D::div(rU, smax(up ? hL : hR, kSmallReal));
         f.f3 = (up ? bL : bR) * f.f1 * vU;
     } else if (rhs) {
         f.f1 = 0.;
@@ -335,7 +374,7 @@ SW2D_HD double bc_value(const double* tv, const double* vv, int64_t n, double ti
 // swSp::hypHCritical (swSpHyp.cpp:651-661)
 SW2D_HD double h_critical(double phi, double q)
 {
-    return sw2d_exp((1. / 3.) * sw2d_log((q / smax(phi, kSmallReal)) / kGravity));
+    return sw2d_exp((1. / 3.) * sw2d_log(sw2d_div(sw2d_div(q, smax(phi, kSmallReal)), kGravity)));
 }
 
 // swSp::hypBoundaryFlux (swSpHyp.cpp:13-135); the boundary geometric source stays 0.  Returns
@@ -352,7 +391,7 @@ SW2D_HD unsigned boundary_flux(double bR, double phiR, double zbR, const SideSta
         hR = 0.;
     }
     double cR = sqrt(kGravity * smax(hR, kSmallReal));
-    double uR = q1 / smax(hR, kSmallReal);
+    double uR = sw2d_div(q1, smax(hR, kSmallReal));
     double L1 = smax(0.0, S.lp);
     double flux2R = spec_force(bR, phiR, hR, uR);
     double flux1 = 0.0, flux2 = 0.0;
@@ -386,7 +425,7 @@ SW2D_HD unsigned boundary_flux(double bR, double phiR, double zbR, const SideSta
     if (flux1 > 0) {
         flux3 = 0;
     } else {
-        double vR = r1 / smax(hR, kSmallReal);
+        double vR = sw2d_div(r1, smax(hR, kSmallReal));
         flux3 = flux1 * vR;
     }
     *f1o = flux1;

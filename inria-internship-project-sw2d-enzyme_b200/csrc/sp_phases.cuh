@@ -165,8 +165,10 @@ __device__ __forceinline__ void slopes_cell(const DevMesh& m, int c)
                         sy += div_known(div_known(dz * (xj[i].y - xy.y), dist, w), dist, w) * w;
                         wsum += w;
                     }
-                sx /= wsum;
-                sy /= wsum;
+                if (!warp_all(sx == 0.0 && sy == 0.0)) {  // wsum > 0: a zero sum (a level surface) stays
+                    sx /= wsum;
+                    sy /= wsum;
+                }
             } else {
                 const double2 g = slope_gradient<L>(m.st, m.cxy, m.cint, k0, k1, zc, xy);
                 sx = g.x;
@@ -349,31 +351,38 @@ __device__ __forceinline__ double cfl_cell(const DevMesh& m, int c)
 // minimum that keeps a when b is not smaller (a NaN candidate b never wins)
 __device__ __forceinline__ double min_keep(double a, double b) { return (b < a) ? b : a; }
 
-// dt_finalize: the grid minimum dt (at most dt_max), snapped to the next storage time
-// (swSpHyp.cpp:496-504) and clipped at t_max; sets the control block's dt, go and store_map.
+// dt_snap: the grid minimum dt (at most dt_max), snapped to the next storage time
+// (swSpHyp.cpp:496-504) and clipped at t_max; `store` tells whether the step ends on a storage time.
 // kDdpSnap: the DDP model's form of the snap, which truncates t and t + dt to integers before
 // dividing by dt_map (swDdpHyp.cpp:588-600: `(int)t / dt_map`).
-template <bool kDdpSnap, class L = LdNc>
-__device__ __forceinline__ void dt_finalize(const DevMesh& m, Ctrl* ctrl, double dt)
+template <bool kDdpSnap>
+__device__ __forceinline__ double dt_snap(double dt_map, double t, double t_max, double dt, int& store)
 {
-    const double t = L::ctl(&ctrl->t);
-    const double t_max = L::ctl(&ctrl->t_max);
-    int store = m.dt_map <= -kSmallReal ? 1 : 0;
-    if (m.dt_map > kSmallReal) {
+    store = dt_map <= -kSmallReal ? 1 : 0;
+    if (dt_map > kSmallReal) {
         int now, later;
         if (kDdpSnap) {
-            now = (int)((double)(int)t / m.dt_map);
-            later = (int)((double)(int)(t + dt) / m.dt_map);
+            now = (int)((double)(int)t / dt_map);
+            later = (int)((double)(int)(t + dt) / dt_map);
         } else {
-            now = (int)(t / m.dt_map);
-            later = (int)((t + dt) / m.dt_map);
+            now = (int)(t / dt_map);
+            later = (int)((t + dt) / dt_map);
         }
         if (later > now) {
-            dt = later * m.dt_map - t;
+            dt = later * dt_map - t;
             store = 1;
         }
     }
     if ((t + dt) > t_max) dt = t_max - t;
+    return dt;
+}
+
+// dt_finalize: dt_snap of the grid minimum into the control block's dt, go and store_map
+template <bool kDdpSnap, class L = LdNc>
+__device__ __forceinline__ void dt_finalize(const DevMesh& m, Ctrl* ctrl, double dt)
+{
+    int store;
+    dt = dt_snap<kDdpSnap>(m.dt_map, L::ctl(&ctrl->t), L::ctl(&ctrl->t_max), dt, store);
     ctrl->store_map = store;
     ctrl->dt = dt;
     ctrl->go = 1;

@@ -233,6 +233,7 @@ struct AdjointState;  // sw2d_adjoint.cu
 struct AssimState;    // sw2d_assim.cu
 struct DdpState;      // sw2d_ddp.cu
 struct ClosureState;  // sw2d_mlp.cu
+struct RunState;      // sw2d_run.cu
 
 }  // namespace sw2d
 
@@ -282,6 +283,9 @@ struct sw2d_handle {
     int fused = 0;                      // step as the two kernels k_flux + k_update (option "fused_step")
     int fused_slopes = 0;               // MUSCL-EVR: slopes inside k_flux (1) or by k_slopes first (0)
     int flux_variant = 0;               // launch variant of k_flux (sw2d_autotune)
+    sw2d::RunState* run = nullptr;      // run kernel of small meshes
+    int run_kernel = 1;                 // option "run_kernel"
+    int64_t run_polls = -1;             // option "run_wait_polls" (< 0: the default)
     std::string err;
 };
 
@@ -355,6 +359,17 @@ int flux_variants();
 std::string flux_variant_label(int v);
 int tiles_build(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<int2>& cint,
                 const std::vector<int2>& lr, const std::vector<int>& bcell, int tile_cells, std::string& why);
+// Tiles of `tile_cells` cells (at least `least`) into `tm` and `allocs`, with the rings and lists of
+// the slopes when own_slopes.
+int tiles_make(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<int2>& cint, const std::vector<int2>& lr,
+               const std::vector<int>& bcell, int tile_cells, bool own_slopes, int least, TileMesh& tm,
+               std::vector<void*>& allocs, std::string& why);
+
+// The run kernel of small meshes (sw2d_run.cu): whether the handle's next steps may take it (its
+// tiles are built the first time), the launches of n steps, the release.
+int run_ready(sw2d_handle* h, bool* ready);
+int run_steps(sw2d_handle* h, int64_t n);
+void run_release(sw2d_handle* h);
 
 // The CFL kernel with the DDP model's map-storage snap (swDdpHyp.cpp:588-600).
 void launch_cfl_ddp_on(sw2d_handle* h, const DevMesh& m);
@@ -372,12 +387,12 @@ __device__ __forceinline__ void cell_sources(const DevMesh& m, int c, double dt,
     if (kFriction != SW2D_FRICTION_NONE) {
         if (hh > hthr) {
             const double4 fr = fr_pre ? *fr_pre : ld(&m.fric[c]);
-            double u = qq / hh;
-            double v = rr / hh;
+            double u = sw2d_div(qq, hh);
+            double v = sw2d_div(rr, hh);
             double ca = fr.z, sa = fr.w;
             double ul = u * ca + v * sa;
             double vl = -u * sa + v * ca;
-            double un = sqrt(u * u + v * v);
+            double un = sw2d_sqrt(u * u + v * v);
             // h^(-4/3) once per cell; isotropic friction (equal coefficients): the same factor,
             // computed once
             const double P = (kFriction != SW2D_FRICTION_CHEZY && hh > kSmallReal) ? friction_power(hh) : 0.0;
@@ -403,8 +418,9 @@ __device__ __forceinline__ void cell_sources(const DevMesh& m, int c, double dt,
             const double4 hl = ld(&m.hla[c]);
             double ax = 0, ay = 0;
             if (hh > hl.x) {
-                ax = sqrt(qx * qx + qy * qy) * hl.y / hh;
-                ay = sqrt(qx * qx + qy * qy) * hl.z / hh;
+                const double qn = sw2d_sqrt(qx * qx + qy * qy);
+                ax = sw2d_div(qn * hl.y, hh);
+                ay = sw2d_div(qn * hl.z, hh);
             }
             qx = qx * sw2d_exp(-ax * dt);
             qy = qy * sw2d_exp(-ay * dt);
@@ -415,8 +431,13 @@ __device__ __forceinline__ void cell_sources(const DevMesh& m, int c, double dt,
         qq = qx * ca - qy * sa;
         rr = qx * sa + qy * ca;
     }
-    // swSp::correctVelocity (swSp.cpp:447-479)
-    if (hh > m.h_min) {
+    // swSp::correctVelocity (swSp.cpp:447-479).  A cell whose squared discharge is well below both
+    // squared bounds (2 % of margin over the roundings of the reference's expression) cannot be capped
+    // and takes no root and no division; a bound that under- or overflows or is NaN fails the test.
+    const double q2 = qq * qq + rr * rr, hv = hh * m.v_max;
+    const bool slow_flow = m.v_max > 0.0 && m.fr_max > 0.0 && q2 < 0.98 * (hv * hv) &&
+                           q2 < 0.98 * ((kGravity * hh) * (hh * hh) * (m.fr_max * m.fr_max));
+    if (hh > m.h_min && !slow_flow) {
         double qn = sqrt(qq * qq + rr * rr);
         double cc = sqrt(kGravity * hh);
         double Fr = qn / cc / hh;
