@@ -297,6 +297,8 @@ int status_to_code(sw2d_handle* h, unsigned st)
     if (st & kStatusPhiG) return fail(h, SW2D_E_PHIG, "specificForce : phiG is < small");
     if (st & kStatusTable)
         return fail(h, SW2D_E_DDP_TABLE, "DDP - NaN elevation or volume in a porosity-table lookup");
+    if (st & kStatusRunWait)
+        return fail(h, SW2D_E_CUDA, "a wait between the tiles of the run kernel ran out; the state is undefined");
     if (st & kStatusUnsupported)
         return fail(h, SW2D_E_UNSUPPORTED, "cell with more neighbours than the adjoint's slope reverse handles");
     return SW2D_OK;
@@ -915,7 +917,7 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
     }
     if (cudaMalloc(&h->ctrl, sizeof(Ctrl)) != cudaSuccess) return bail(fail(h, SW2D_E_CUDA, "cudaMalloc ctrl"));
     h->allocs.push_back(h->ctrl);
-    if (cudaMallocHost(&h->ctrl_host, sizeof(Ctrl)) != cudaSuccess) return bail(fail(h, SW2D_E_CUDA, "cudaMallocHost"));
+    if (cudaMallocHost(&h->ctrl_host, 2 * sizeof(Ctrl)) != cudaSuccess) return bail(fail(h, SW2D_E_CUDA, "cudaMallocHost"));
     m.ctrl = h->ctrl;
     Ctrl c0{};
     c0.t = params->t_0;
@@ -971,6 +973,17 @@ int sw2d_step_n(sw2d_handle* h, int64_t n_steps, int64_t* steps_done)
 {
     if (!h || n_steps < 0) return fail(h, SW2D_E_ARG, "invalid arguments");
     CK(cudaSetDevice(h->device));
+    bool run = false;
+    if (const int rc = run_ready(h, &run)) return rc;
+    if (run) {  // a small mesh: all steps in one launch, the control block copied out before and after it
+        Ctrl* host = h->ctrl_host;
+        CK(cudaMemcpyAsync(host + 1, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
+        if (const int rc = run_steps(h, n_steps)) return rc;
+        CK(cudaMemcpyAsync(host, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        if (steps_done) *steps_done = host[0].steps - host[1].steps;
+        return status_to_code(h, host[0].status);
+    }
     CK(cudaMemcpyAsync(h->ctrl_host, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     const long long before = h->ctrl_host->steps;
@@ -1023,7 +1036,9 @@ int sw2d_prepare_steps(sw2d_handle* h)
 {
     if (!h) return fail(h, SW2D_E_ARG, "invalid handle");
     CK(cudaSetDevice(h->device));
-    const int rc = ensure_graph(h, h->result ? result_chunk(h) : kGraphSteps);
+    bool run = false;
+    int rc = run_ready(h, &run);
+    if (!rc && !run) rc = ensure_graph(h, h->result ? result_chunk(h) : kGraphSteps);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->stream));
     return SW2D_OK;
@@ -1485,6 +1500,14 @@ int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value)
     } else if (std::strcmp(name, "update_reverse") == 0) {
         // block order of the cell update: 1 from the last cells to the first (the same results)
         h->m.rev_update = value ? 1 : 0;
+    } else if (std::strcmp(name, "run_kernel") == 0) {
+        // 1 (default): sw2d_step_n and sw2d_execute take the steps of a small SP or DIP mesh in one
+        // launch (sw2d_run.cu); 0: by the step's kernels (the same results)
+        h->run_kernel = value ? 1 : 0;
+    } else if (std::strcmp(name, "run_wait_polls") == 0) {
+        // poll limit of the run kernel's waits (< 0: the default)
+        h->run_polls = value;
+        return SW2D_OK;
     } else if (std::strcmp(name, "flux_variant") == 0) {
         if (value < 0 || value >= flux_variants()) return fail(h, SW2D_E_ARG, "flux_variant outside the variants");
         h->flux_variant = (int)value;
@@ -1508,6 +1531,7 @@ int sw2d_get_option(sw2d_handle* h, const char* name, int64_t* value)
     if (!h || !name || !value) return fail(h, SW2D_E_ARG, "invalid arguments");
     if (std::strcmp(name, "fused_step") == 0) *value = h->fused;
     else if (std::strcmp(name, "flux_variant") == 0) *value = h->flux_variant;
+    else if (std::strcmp(name, "run_kernel") == 0) *value = h->run_kernel;
     else if (std::strcmp(name, "update_reverse") == 0) *value = h->m.rev_update;
     else if (std::strcmp(name, "fused_slopes") == 0) *value = h->fused_slopes;
     else if (std::strcmp(name, "tile_cells") == 0) *value = h->tiles.tile_cells;
@@ -1870,6 +1894,7 @@ int sw2d_destroy(sw2d_handle* h)
     ddp_release(h);
     closure_release(h);
     result_release(h);
+    run_release(h);
     for (void* p : h->allocs) cudaFree(p);
     for (void* p : h->tile_allocs) cudaFree(p);
     if (h->saved_point) cudaFree(h->saved_point);

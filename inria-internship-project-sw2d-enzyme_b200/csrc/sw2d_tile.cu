@@ -43,27 +43,11 @@
 #include <vector>
 
 #include "sw2d_internal.cuh"
+#include "tile_phases.cuh"
 
 using namespace sw2d;
 
 namespace {
-
-// Asynchronous global -> shared copies (cp.async, sm_80+): every copy of a tile is issued before
-// the first is waited for, so the loads of a tile are in flight together.
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cpa16(void* s, const void* g)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(s)), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cpa8(void* s, const void* g)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(s)), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cpa4(void* s, const void* g)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr(s)), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cpa_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // A tile's stage in shared memory, in the global records' own layouts (byte offsets computed on
 // the host, TileMesh::o_*): per staged cell its state {h, q, r, z} and centroid {x, y}; per tile
@@ -296,75 +280,36 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_flux(DevMesh m, TileMesh tm
         const bool rec = m.flux != nullptr || m.lmax != nullptr;
         for (int j = threadIdx.x; j < nflux; j += kThreads) {
             const ushort2 ll = sv.ell[j];
-            const int a = ll.x, b = ll.y;
-            const double2 n = sv.en[j];
-            const double4 Sa = sv.st[a], Sb = sv.st[b];
-            const double4 Ka = sv.cst[a], Kb = sv.cst[b];
-            SideState SL, SR;
-            double phiG = 0.0, xL = 1.0, xR = 1.0;
-            if (kDip) {
-                phiG = sv.epg[j];
-                xL = dip_x(Ka.z, phiG);
-                xR = dip_x(Kb.z, phiG);
+            TileEdge E;
+            E.a = ll.x;
+            E.b = ll.y;
+            E.n = sv.en[j];
+            E.cf = sv.ecf[j];
+            E.len = sv.elen[j];
+            E.phig = kDip ? sv.epg[j] : 0.0;
+            if (kMuscl) {
+                const double2 mp = sv.em[j], ca = sv.xy[E.a], cb = sv.xy[E.b];
+                E.ga = sv.sl[E.a];
+                E.gb = sv.sl[E.b];
+                E.da = make_double2(mp.x - ca.x, mp.y - ca.y);
+                E.db = make_double2(mp.x - cb.x, mp.y - cb.y);
             }
-            if (!kMuscl) {
-                if (kDip) {
-                    SL = godunov_side_dip(Sa.x, Sa.y, Sa.z, Ka.x, Ka.y, xL, n.x, n.y);
-                    SR = godunov_side_dip(Sb.x, Sb.y, Sb.z, Kb.x, Kb.y, xR, n.x, n.y);
-                } else {
-                    SL = godunov_side(Sa.x, Sa.y, Sa.z, Ka.x, Ka.y, n.x, n.y);
-                    SR = godunov_side(Sb.x, Sb.y, Sb.z, Kb.x, Kb.y, n.x, n.y);
-                }
-            } else {
-                const double2 mp = sv.em[j];
-                const double2 ca = sv.xy[a], cb = sv.xy[b];
-                const double2 ga = sv.sl[a], gb = sv.sl[b];
-                const double dax = mp.x - ca.x, day = mp.y - ca.y;
-                const double dbx = mp.x - cb.x, dby = mp.y - cb.y;
-                if (kDip) {
-                    SL = evr_side_dip(true, Sa.x, Sa.y, Sa.z, Ka.x, Ka.y, xL, Sa.w, ga.x, ga.y, dax, day, n.x, n.y, dtp);
-                    SR = evr_side_dip(false, Sb.x, Sb.y, Sb.z, Kb.x, Kb.y, xR, Sb.w, gb.x, gb.y, dbx, dby, n.x, n.y, dtp);
-                } else {
-                    SL = evr_side(true, Sa.x, Sa.y, Sa.z, Ka.x, Ka.y, Sa.w, ga.x, ga.y, dax, day, n.x, n.y, dtp, m.dry);
-                    SR = evr_side(false, Sb.x, Sb.y, Sb.z, Kb.x, Kb.y, Sb.w, gb.x, gb.y, dbx, dby, n.x, n.y, dtp, m.dry);
-                }
-            }
-            const double lm = max4(fabs(SL.lm), fabs(SL.lp), fabs(SR.lm), fabs(SR.lp));
-            const int e = rec ? ((j < ne_own) ? TI(e0) + j : ld(&tm.xe[TI(xoff) + j - ne_own])) : 0;
-            if (m.lmax) m.lmax[e] = lm;
-            const double lw = lm * sv.elen[j];
-            const bool wetL = Sa.x > m.h_min, wetR = Sb.x > m.h_min;
             const int2 sl = sv.esl[j];
-            const bool ownL = a < nt, ownR = b < nt;
-            if (ownL) sv.lam[sl.x - s0] = wetL ? lw : 0.0;
-            if (ownR) sv.lam[sl.y - s0] = (wetL || wetR) ? lw : 0.0;
-            const double hL = SL.z - Ka.x, hR = SR.z - Kb.x;
-            if ((hL > m.h_min) || (hR > m.h_min)) {
-                EdgeFlux f = kDip ? hllc_dip(kBlending, Ka.y, Kb.y, phiG, Ka.z, Kb.z, Ka.x, Kb.x, SL, SR, m.h_min, m.phi_min)
-                                  : hllc(kBlending, Ka.y, Kb.y, Ka.z, Kb.z, Ka.x, Kb.x, SL, SR, m.h_min, m.phi_min);
-                bad |= f.bad;
-                if (isnan(f.f1)) bad |= kStatusNanFlux;
-                if (m.flux) {
+            double lm;
+            EdgeFlux f;
+            bool flux;
+            bad |= tile_edge<kScheme, kBlending, kModel, DivPlain>(
+                m, E, sv.st[E.a], sv.st[E.b], sv.cst[E.a], sv.cst[E.b], dtp, E.a < nt, E.b < nt, lm, f, flux,
+                [&](int side, double v) { sv.lam[(side ? sl.y : sl.x) - s0] = v; },
+                [&](int side, const Slot& v) { m.slot[side ? sl.y : sl.x] = v; });
+            if (rec) {
+                const int e = (j < ne_own) ? TI(e0) + j : ld(&tm.xe[TI(xoff) + j - ne_own]);
+                if (m.lmax) m.lmax[e] = lm;
+                if (m.flux && flux) {
                     double2* fp = m.flux + 3 * (size_t)e;
                     fp[0] = make_double2(f.f1, f.f2);
                     fp[1] = make_double2(f.f3, f.sl);
                     fp[2] = make_double2(f.sr, 0.0);
-                }
-                const double2 cf = sv.ecf[j];
-                const double nx = n.x, ny = n.y;
-                if (ownL) {
-                    const double c = cf.x;
-                    const double f1 = -c, f2F2 = -c * nx, f2F3 = +c * ny, f2S2 = +c * nx;
-                    const double f3F2 = -c * ny, f3F3 = -c * nx, f3S2 = +c * ny;
-                    m.slot[sl.x] = make_slot(f1 * f.f1, f2F2 * f.f2 + f2S2 * f.sl + f2F3 * f.f3,
-                                             f3F2 * f.f2 + f3S2 * f.sl + f3F3 * f.f3);
-                }
-                if (ownR) {
-                    const double c = cf.y;
-                    const double f1 = +c, f2F2 = +c * nx, f2F3 = -c * ny, f2S2 = +c * nx;
-                    const double f3F2 = +c * ny, f3F3 = +c * nx, f3S2 = +c * ny;
-                    m.slot[sl.y] = make_slot(f1 * f.f1, f2F2 * f.f2 + f2S2 * f.sr + f2F3 * f.f3,
-                                             f3F2 * f.f2 + f3S2 * f.sr + f3F3 * f.f3);
                 }
             }
         }
@@ -377,27 +322,14 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_flux(DevMesh m, TileMesh tm
         for (int j = threadIdx.x; j < nbe; j += kThreads) {
             const int e = b0 + j;
             const int l = ld(&m.bcell[e]) - c0;
-            const double4 g = ld(&m.bgeo[e]);
-            const double4 Sl = sv.st[l], Kl = sv.cst[l];
-            const double phiGb = kDip ? ld(&m.phigb[e]) : 0.0;
-            SideState S = kDip ? godunov_side_dip(Sl.x, Sl.y, Sl.z, Kl.x, Kl.y, dip_x(Kl.z, phiGb), g.x, g.y)
-                               : godunov_side(Sl.x, Sl.y, Sl.z, Kl.x, Kl.y, g.x, g.y);
-            const double lm = kMuscl ? smax(fabs(S.lm), fabs(S.lp)) : smax(fabs(S.lp), fabs(S.lm));
+            double lm, cfl, f1, f2, f3;
+            Slot v;
+            bad |= tile_boundary<kScheme, kModel, DivPlain>(m, e, sv.st[l], sv.cst[l], tnow, lm, cfl, f1, f2, f3, v);
             if (m.lmaxb) m.lmaxb[e] = lm;
             const int sbi = ld(&m.bslot[e]);
-            sv.lam[sbi - s0] = (Sl.x > m.h_min) ? lm * g.z : 0.0;
-            const int k = ld(&m.bbc[e]);
-            const long long o0 = ld(&m.bcoff[k]), o1 = ld(&m.bcoff[k + 1]);
-            const double v = bc_value(m.bctimes + o0, m.bcvals + o0, o1 - o0, tnow);
-            double f1, f2, f3;
-            bad |= kDip ? boundary_flux_dip(Kl.y, phiGb, Kl.z, Kl.x, S, ld(&m.bctype[k]), v, m.h_min, &f1, &f2, &f3)
-                        : boundary_flux(Kl.y, Kl.z, Kl.x, S, ld(&m.bctype[k]), v, m.h_min, &f1, &f2, &f3);
+            sv.lam[sbi - s0] = cfl;
             if (m.bflux) m.bflux[e] = make_double4(f1, f2, f3, 0.0);
-            const double cf = g.w, nx = g.x, ny = g.y;
-            const double fa = +cf, f2F2 = +cf * nx, f2F3 = -cf * ny, f2S2 = +cf * nx;
-            const double f3F2 = +cf * ny, f3F3 = +cf * nx, f3S2 = +cf * ny;
-            const double s2 = 0.0;  // boundary geometric source: never set by hypBoundaryFlux
-            m.slot[sbi] = make_slot(fa * f1, f2F2 * f2 + f2S2 * s2 + f2F3 * f3, f3F2 * f2 + f3S2 * s2 + f3F3 * f3);
+            m.slot[sbi] = v;
         }
     }
     if (bad) atomicOr(&ctrl->status, bad);
@@ -554,11 +486,18 @@ cudaError_t launch_flux(sw2d_handle* h, const DevMesh& m, int v, bool attr_only)
 int tiles_build(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<int2>& cint,
                 const std::vector<int2>& lr, const std::vector<int>& bcell, int tile_cells, std::string& why)
 {
-    // ring 2, the ring-1 slope edges and the neighbour lists serve the slopes k_flux computes
-    const bool muscl = h->p.scheme == SW2D_SCHEME_MUSCL_EVR && h->fused_slopes;
-    const bool slopes_read = h->p.scheme == SW2D_SCHEME_MUSCL_EVR && !h->fused_slopes;
+    return tiles_make(h, coff, cint, lr, bcell, tile_cells, h->fused_slopes != 0, 32, h->tiles, h->tile_allocs, why);
+}
+
+int tiles_make(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<int2>& cint, const std::vector<int2>& lr,
+               const std::vector<int>& bcell, int tile_cells, bool own_slopes, int least, TileMesh& tm,
+               std::vector<void*>& allocs, std::string& why)
+{
+    // ring 2, the ring-1 slope edges and the neighbour lists serve the slopes a tile computes itself
+    const bool muscl = h->p.scheme == SW2D_SCHEME_MUSCL_EVR && own_slopes;
+    const bool slopes_read = h->p.scheme == SW2D_SCHEME_MUSCL_EVR && !own_slopes;
     const int nc = (int)h->nc, ni = (int)h->ni, nb = (int)h->nb;
-    if (tile_cells < 32 || tile_cells > 8192) {
+    if (tile_cells < least || tile_cells > 8192) {
         why = "tile size outside 32..8192 cells";
         return SW2D_E_ARG;
     }
@@ -694,7 +633,6 @@ int tiles_build(sw2d_handle* h, const std::vector<int2>& coff, const std::vector
         na_max = std::max(na_max, nedges);
         nent_max = std::max(nent_max, ti.nent);
     }
-    TileMesh& tm = h->tiles;
     TileMesh probe;
     probe.nl_max = nl_max;
     probe.nf_max = nf_max;
@@ -710,8 +648,8 @@ int tiles_build(sw2d_handle* h, const std::vector<int2>& coff, const std::vector
         return SW2D_E_UNSUPPORTED;
     }
     // replace the previous tiles' arrays
-    for (void* p : h->tile_allocs) cudaFree(p);
-    h->tile_allocs.clear();
+    for (void* p : allocs) cudaFree(p);
+    allocs.clear();
     tm = probe;
     tm.ntiles = ntiles;
     tm.tile_cells = tile_cells;
@@ -720,7 +658,7 @@ int tiles_build(sw2d_handle* h, const std::vector<int2>& coff, const std::vector
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(1, vec.size()) * sizeof(T);
         if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(h, SW2D_E_CUDA, "cudaMalloc (tiles)");
-        h->tile_allocs.push_back(p);
+        allocs.push_back(p);
         if (!vec.empty() && cudaMemcpyAsync(p, vec.data(), vec.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream) !=
                                 cudaSuccess)
             return fail(h, SW2D_E_CUDA, "tile upload");
@@ -740,8 +678,8 @@ int tiles_build(sw2d_handle* h, const std::vector<int2>& coff, const std::vector
     if (!rc) rc = up(soffs, &d_soffs);
     if (!rc && cudaStreamSynchronize(h->stream) != cudaSuccess) rc = fail(h, SW2D_E_CUDA, "tile upload");
     if (rc) {
-        for (void* p : h->tile_allocs) cudaFree(p);
-        h->tile_allocs.clear();
+        for (void* p : allocs) cudaFree(p);
+        allocs.clear();
         tm = TileMesh{};
         return rc;
     }
