@@ -136,7 +136,11 @@ __device__ __forceinline__ double slope_rev_cell(const DevMesh& m, int e0, int c
         if (i < cnt) {
             const int2 en = ld(&m.cint[e0 + i]);
             const double2 xj = ld(&m.cxy[en.y]);
-            const double2 mp = ld(&m.mxy[en.x >> 1]);
+            const double4 geo = ld(&m.egeo[en.x >> 1]);  // {dist, 1 / dist, mx, my}
+            nb[i].dist = geo.x;
+            nb[i].w = geo.y;
+            nb[i].plain = m.geo_plain != 0;
+            const double2 mp = make_double2(geo.z, geo.w);
             nb[i].zj = m.st[en.y].w;
             nb[i].dx = xj.x - xy.x;
             nb[i].dy = xj.y - xy.y;

@@ -25,7 +25,20 @@ struct CellBar {
     double h, q, r, zb, zc, sx, sy;
 };
 
-SW2D_HD double dsqrt_bar(double y, double ybar) { return (y > 0.0) ? ybar * 0.5 / y : 0.0; }
+SW2D_HD double dsqrt_bar(double y, double ybar) { return (y > 0.0) ? sw2d_div(ybar * 0.5, y) : 0.0; }
+
+// Reverse of root = sqrt((b - 1) b u u + c c): adds to the adjoints of u and c.  Where the root is c
+// itself (b == 1, root_is_c) its derivative is 1 by c and 0 by u, without the root and the division.
+SW2D_HD void root_rev(double b, double u, double c, double root_bar, double& u_bar, double& c_bar)
+{
+    if (warp_all(root_is_c(b, u, c))) {
+        c_bar = c > 0.0 ? root_bar : 0.0;
+        return;
+    }
+    const double X_bar = dsqrt_bar(sqrt((b - 1.0) * b * u * u + c * c), root_bar);
+    u_bar += X_bar * (b - 1.0) * b * 2.0 * u;
+    c_bar = X_bar * 2.0 * c;
+}
 
 // ---- godunov_side (swSpHypGodunov.cpp:17-35)
 SW2D_HD void godunov_side_rev(double h, double q, double r, double b, double nx, double ny, const SideBar& sb,
@@ -33,20 +46,16 @@ SW2D_HD void godunov_side_rev(double h, double q, double r, double b, double nx,
 {
     const double sq = q * nx + r * ny;
     const double d = smax(h, kSmallReal);
-    const double u = sq / d;
-    const double c = sqrt(kGravity * h);
-    const double X = (b - 1.0) * b * u * u + c * c;
-    const double root = sqrt(X);
-    const double bu_bar = sb.lm + sb.lp;
-    const double root_bar = sb.lp - sb.lm;
-    const double X_bar = dsqrt_bar(root, root_bar);
-    const double u_bar = bu_bar * b + X_bar * (b - 1.0) * b * 2.0 * u;
-    const double c_bar = X_bar * 2.0 * c;
+    const double rd = 1.0 / d;
+    const double u = sq * rd;
+    const double c = sw2d_sqrt(kGravity * h);
+    double u_bar = (sb.lm + sb.lp) * b, c_bar;
+    root_rev(b, u, c, sb.lp - sb.lm, u_bar, c_bar);
     double h_bar = sb.z;                          // z = h + z_b
     cb.zb += sb.z;
     h_bar += dsqrt_bar(c, c_bar) * kGravity;      // c = sqrt(g h)
-    const double sq_bar = sb.q + u_bar / d;
-    if (!(h < kSmallReal)) h_bar += -u_bar * u / d;   // d = h
+    const double sq_bar = sb.q + u_bar * rd;
+    if (!(h < kSmallReal)) h_bar += -u_bar * u * rd;  // d = h
     const double sr_bar = sb.r;                   // sr = -q ny + r nx
     cb.h += h_bar;
     cb.q += sq_bar * nx - sr_bar * ny;
@@ -63,10 +72,10 @@ SW2D_HD void evr_side_rev(bool left, double h, double q, double r, double zb, do
     const double rl = r * nx - q * ny;
     const double hd = smax(kSmallReal, h);
     const double cl = sqrt(kGravity * hd);
-    const double ul = ql / hd;
-    const double vl = rl / hd;
-    const double X1 = (b - 1.0) * b * ul * ul + cl * cl;
-    const double root1 = sqrt(X1);
+    const double rhd = 1.0 / hd;
+    const double ul = sw2d_div(ql, hd);  // decides branches: the forward's division
+    const double vl = rl * rhd;
+    const double root1 = warp_all(root_is_c(b, ul, cl)) ? cl : sqrt((b - 1.0) * b * ul * ul + cl * cl);
     const double lmv = b * ul - root1;
     const double lpv = b * ul + root1;
     const double l1 = left ? smax(0.0, lmv) : smin(0.0, lmv);
@@ -82,17 +91,12 @@ SW2D_HD void evr_side_rev(bool left, double h, double q, double r, double zb, do
     const double hr = 0.5 * (h1 + h2);
     const double sq = hr * ul;
     const double d2 = smax(hr, kSmallReal);
-    const double u = sq / d2;
-    const double c = sqrt(kGravity * hr);
-    const double X = (b - 1.0) * b * u * u + c * c;
-    const double root = sqrt(X);
+    const double rd2 = 1.0 / d2;
+    const double u = sq * rd2;
+    const double c = sw2d_sqrt(kGravity * hr);
     // reverse (the derivative terms multiply by the reciprocals of the two denominators)
-    const double rd2 = 1.0 / d2, rhd = 1.0 / hd;
-    const double bu_bar = sb.lm + sb.lp;
-    const double root_bar = sb.lp - sb.lm;
-    const double X_bar = dsqrt_bar(root, root_bar);
-    const double u_bar = bu_bar * b + X_bar * (b - 1.0) * b * 2.0 * u;
-    const double c_bar = X_bar * 2.0 * c;
+    double u_bar = (sb.lm + sb.lp) * b, c_bar;
+    root_rev(b, u, c, sb.lp - sb.lm, u_bar, c_bar);
     double hr_bar = dsqrt_bar(c, c_bar) * kGravity;
     const double sq_bar = sb.q + u_bar * rd2;
     if (!(hr < kSmallReal)) hr_bar += -u_bar * u * rd2;
@@ -123,10 +127,8 @@ SW2D_HD void evr_side_rev(bool left, double h, double q, double r, double zb, do
         if (left ? (0.0 < lmv) : (lmv < 0.0)) lmv_bar += l1_bar;
     }
     ul_bar += b * (lmv_bar + lpv_bar);
-    const double root1_bar = lpv_bar - lmv_bar;
-    const double X1_bar = dsqrt_bar(root1, root1_bar);
-    ul_bar += X1_bar * (b - 1.0) * b * 2.0 * ul;
-    const double cl_bar = X1_bar * 2.0 * cl;
+    double cl_bar;
+    root_rev(b, ul, cl, lpv_bar - lmv_bar, ul_bar, cl_bar);
     const double ql_bar = ul_bar * rhd;
     const double rl_bar = vl_bar * rhd;
     double hd_bar = -ul_bar * ul * rhd - vl_bar * vl * rhd + dsqrt_bar(cl, cl_bar) * kGravity;
@@ -177,13 +179,16 @@ SW2D_HD void hllc_rev(bool blending, double bL, double bR, double phiL, double p
         const double duR = blending ? smax(hR, kSmallReal) : smax(kSmallReal, hR);
         const bool duL_h = blending ? !(hL < kSmallReal) : (kSmallReal < hL);
         const bool duR_h = blending ? !(hR < kSmallReal) : (kSmallReal < hR);
-        const double uL = L.q / duL, uR = R.q / duR;
+        // the reciprocal of each denominator, taken once (the sign of f1, the one branch that depends on
+        // a quotient, is its numerator's); max(h, small) is one value for u and v
+        const double rL = 1.0 / duL, rR = 1.0 / duR;
+        const double uL = L.q * rL, uR = R.q * rR;
         const double mR = smin(R.lm, 0.);
         const double L1 = smin(L.lm, mR);
         const double m2 = smax(R.lp, 0.);
         const double L2 = smax(L.lp, m2);
         const double dLL = L2 - L1;
-        const double den = smax(dLL, kSmallReal);
+        const double den = smax(dLL, kSmallReal), rden = 1.0 / den;
         const double phiLR = smin(phiL, phiR);
         const double pm = smin(phiL, phiR);
         double alpha = 0.0, ratio = 0.0, dzb = zbL - zbR;
@@ -192,46 +197,43 @@ SW2D_HD void hllc_rev(bool blending, double bL, double bR, double phiL, double p
         const double fact = 0.5 * pm * (hL + hR);
         if (blending) {
             if (fabs(dzb) > kSmallReal) {
-                ratio = (L.z - R.z) / dzb;
+                ratio = (L.z - R.z) / dzb;  // decides branches: the forward's division
                 const double inner = smin(1.0, ratio);
                 alpha = smax(0.0, inner);
                 alpha_free = (0.0 < inner) && (ratio < 1.0);
             }
-            F1h = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (hR - hL)) / den;
-            F1z = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)) / den;
+            F1h = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (hR - hL)) * rden;
+            F1z = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)) * rden;
             f1 = alpha * F1h + (1.0 - alpha) * F1z;
             s2z = (phiR * hR * hR - phiL * hL * hL) * 0.5 + fact * (L.z - R.z);
             s2h = (zbL > zbR) ? phiR * hR * (zbL - zbR) : phiL * hL * (zbL - zbR);
             s2a = alpha * s2h + (1.0 - alpha) * s2z;
         } else {
-            f1 = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)) / den;
+            f1 = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)) * rden;
             s2a = (phiR * hR * hR - phiL * hL * hL) * 0.5 + fact * (L.z - R.z);
         }
-        const double s2 = s2a * kGravity / den;
+        const double s2 = s2a * kGravity * rden;
         const double sl = -L1 * s2, sr = L2 * s2;
         const double FL = spec_force(bL, phiL, hL, uL);
         const double FR = spec_force(bR, phiR, hR, uR);
         const double P = phiR * R.q - phiL * L.q;
         const double N2 = L2 * (FL + sl) - L1 * (FR - sr) + L1 * L2 * P;
-        const double f2 = N2 / den;
-        const double dvL = smax(hL, kSmallReal), dvR = smax(hR, kSmallReal);
-        const double vL = L.r / dvL, vR = R.r / dvR;
-        // ---- reverse.  The derivative terms divide by the reciprocal of each denominator, taken
-        // once (the forward values above, which decide the branches, keep the forward's divisions)
-        const double rden = 1.0 / den, rdvL = 1.0 / dvL, rdvR = 1.0 / dvR, rduL = 1.0 / duL, rduR = 1.0 / duR;
+        const double f2 = N2 * rden;
+        const double vL = L.r * rL, vR = R.r * rR;
+        // ---- reverse
         double f1_bar = fb.f1, L1_bar = 0, L2_bar = 0, den_bar = 0;
         double Lq_bar = 0, Rq_bar = 0, Lz_bar = 0, Rz_bar = 0, Lr_bar = 0, Rr_bar = 0;
         double uL_bar = 0, uR_bar = 0;
         if (f1 >= 0) {
             f1_bar += fb.f3 * bL * vL;
             const double vL_bar = fb.f3 * bL * f1;
-            Lr_bar += vL_bar * rdvL;
-            if (!(hL < kSmallReal)) hL_bar += -vL_bar * vL * rdvL;
+            Lr_bar += vL_bar * rL;
+            if (!(hL < kSmallReal)) hL_bar += -vL_bar * vL * rL;
         } else {
             f1_bar += fb.f3 * bR * vR;
             const double vR_bar = fb.f3 * bR * f1;
-            Rr_bar += vR_bar * rdvR;
-            if (!(hR < kSmallReal)) hR_bar += -vR_bar * vR * rdvR;
+            Rr_bar += vR_bar * rR;
+            if (!(hR < kSmallReal)) hR_bar += -vR_bar * vR * rR;
         }
         const double N2_bar = fb.f2 * rden;
         den_bar += -fb.f2 * f2 * rden;
@@ -326,10 +328,10 @@ SW2D_HD void hllc_rev(bool blending, double bL, double bR, double phiL, double p
         } else {
             Lb.lp += L2_bar;
         }
-        Lq_bar += uL_bar * rduL;
-        if (duL_h) hL_bar += -uL_bar * uL * rduL;
-        Rq_bar += uR_bar * rduR;
-        if (duR_h) hR_bar += -uR_bar * uR * rduR;
+        Lq_bar += uL_bar * rL;
+        if (duL_h) hL_bar += -uL_bar * uL * rL;
+        Rq_bar += uR_bar * rR;
+        if (duR_h) hR_bar += -uR_bar * uR * rR;
         Lb.q += Lq_bar;
         Rb.q += Rq_bar;
         Lb.r += Lr_bar;
@@ -519,15 +521,16 @@ SW2D_HD void update_cell_rev(const UpdateParams& p, double hB, double qB, double
     // friction
     const double h_f = hh, q_f = qq, r_f = rr;   // inputs of the friction stage
     bool fr_wet = false;
-    double u = 0, v = 0, ul0 = 0, vl0 = 0, un = 0, f1 = 1, f2 = 1, P = 0;
+    double u = 0, v = 0, ul0 = 0, vl0 = 0, un = 0, f1 = 1, f2 = 1, P = 0, rh = 0;
     if (p.friction != 0) {
         if (hh > hthr) {
             fr_wet = true;
-            u = qq / hh;
-            v = rr / hh;
+            rh = 1.0 / hh;
+            u = qq * rh;
+            v = rr * rh;
             ul0 = u * p.fcos + v * p.fsin;
             vl0 = -u * p.fsin + v * p.fcos;
-            un = sqrt(u * u + v * v);
+            un = sw2d_sqrt(u * u + v * v);
             if (p.friction != 1 && hh > kSmallReal) P = p.P_given ? p.P : friction_power(hh);
             f1 = friction_factor_p(p.friction, p.k1, hh, un, p.dt, P);
             f2 = (p.k2 == p.k1) ? f1 : friction_factor_p(p.friction, p.k2, hh, un, p.dt, P);
@@ -638,7 +641,6 @@ SW2D_HD void update_cell_rev(const UpdateParams& p, double hB, double qB, double
             const double f1_bar = ul_bar * ul0, f2_bar = vl_bar * vl0;
             double un_bar = 0.0;
             // the derivative terms multiply by the reciprocals of h and |u|, taken once
-            const double rh = 1.0 / h_f;
             friction_factor_rev(p.friction, p.k1, h_f, un, p.dt, P, f1, f1_bar, k1b, h_bar, un_bar, rh);
             friction_factor_rev(p.friction, p.k2, h_f, un, p.dt, P, f2, f2_bar, k2b, h_bar, un_bar, rh);
             double u_bar = ul0_bar * p.fcos - vl0_bar * p.fsin;
@@ -679,7 +681,24 @@ constexpr int kMaxNbr = 8;
 struct SlopeNbr {
     double zj, dx, dy, ax, ay;  // neighbour z, centroid offset (j - c), midpoint offset (m - c)
     bool c_is_r;                // the cell is the R side of the shared edge
+    double dist = 0.0, w = 0.0; // |(dx, dy)| and 1 / dist when the caller has them (w = 0: computed here)
+    bool plain = false;         // the lengths allow div_known (slope_length_ok, slope_component_ok)
 };
+
+// distance and weight of a neighbour
+SW2D_HD void nbr_weight(const SlopeNbr& nb, double& dist, double& w)
+{
+    dist = nb.w > 0.0 ? nb.dist : sqrt(nb.dx * nb.dx + nb.dy * nb.dy);
+    w = nb.w > 0.0 ? nb.w : 1.0 / dist;
+}
+
+// num / den with den != 0 of either sign, a zero numerator written down directly (sw2d_div)
+SW2D_HD double div_signed(double num, double den)
+{
+    const bool z = num == 0.0 && den != 0.0;
+    const double q = (z ? den : num) / den;
+    return z ? (den < 0.0 ? -num : num) : q;
+}
 
 // The slope functions loop over a compile-time capacity N (with n <= N used entries); for
 // N <= 4 the loops are unrolled so that a kernel instantiated for triangles (N = 3) keeps every
@@ -702,15 +721,21 @@ SW2D_HD void slopes_fwd_t(double zc, int n, const SlopeNbr* nb, double& sx, doub
         SW2D_UNROLL_KU
         for (int k = 0; k < N; k++) {
             if (k < n) {
-                const double dist = sqrt(nb[k].dx * nb[k].dx + nb[k].dy * nb[k].dy);
-                const double w = 1.0 / dist;
-                sx += (nb[k].zj - zc) * nb[k].dx / dist / dist * w;
-                sy += (nb[k].zj - zc) * nb[k].dy / dist / dist * w;
+                double dist, w;
+                nbr_weight(nb[k], dist, w);
+                const double dz = nb[k].zj - zc;
+                if (nb[k].plain && div_range_ok(dz)) {
+                    sx += div_known(div_known(dz * nb[k].dx, dist, w), dist, w) * w;
+                    sy += div_known(div_known(dz * nb[k].dy, dist, w), dist, w) * w;
+                } else {
+                    sx += dz * nb[k].dx / dist / dist * w;
+                    sy += dz * nb[k].dy / dist / dist * w;
+                }
                 wsum += w;
             }
         }
-        sx /= wsum;
-        sy /= wsum;
+        sx = sw2d_div(sx, wsum);
+        sy = sw2d_div(sy, wsum);
     }
     SW2D_UNROLL_KU
     for (int k = 0; k < N; k++) {
@@ -721,13 +746,9 @@ SW2D_HD void slopes_fwd_t(double zc, int n, const SlopeNbr* nb, double& sx, doub
             const double zR = nb[k].c_is_r ? zc : nb[k].zj;
             const double fmx = smax(zL, zR), fmn = smin(zL, zR);
             const double rec = zc + nb[k].ax * sx + nb[k].ay * sy;
-            if (rec < fmn) {
-                const double fac = (fmn - zc) / (rec - zc);
-                sx *= fac;
-                sy *= fac;
-            }
-            if (rec > fmx) {
-                const double fac = (fmx - zc) / (rec - zc);
+            const bool under = rec < fmn;  // fmn <= fmx: at most one of the two rescalings
+            if (under || rec > fmx) {
+                const double fac = div_signed((under ? fmn : fmx) - zc, rec - zc);
                 sx *= fac;
                 sy *= fac;
             }
@@ -759,11 +780,12 @@ SW2D_HD void slopes_rev_t(double zc, int n, const SlopeNbr* nb, double sxb, doub
         const bool sel_left = under ? mn_left : mx_left;
         const double f = under ? fmn : fmx;
         const double den = rec - zc;
-        const double fac = (f - zc) / den;
+        const double rden = 1.0 / den;
+        const double fac = (f - zc) * rden;
         const double fac_bar = sxb * sx0 + syb * sy0;
         double sx0_bar = sxb * fac, sy0_bar = syb * fac;
-        const double num_bar = fac_bar / den;
-        const double den_bar = -fac_bar * fac / den;
+        const double num_bar = fac_bar * rden;
+        const double den_bar = -num_bar * fac;
         // f = zL or zR ; num = f - zc ; den = rec - zc ; rec = zc + ax sx0 + ay sy0
         const bool f_is_c = sel_left ? !nb[k].c_is_r : nb[k].c_is_r;
         if (f_is_c) zc_bar += num_bar;
@@ -775,17 +797,22 @@ SW2D_HD void slopes_rev_t(double zc, int n, const SlopeNbr* nb, double sxb, doub
         syb = sy0_bar;
     }
     if (n > 1) {
-        double wsum = 0.0;
+        double wsum = 0.0, wk[N];
         SW2D_UNROLL_KU
         for (int k = 0; k < N; k++)
-            if (k < n) wsum += 1.0 / sqrt(nb[k].dx * nb[k].dx + nb[k].dy * nb[k].dy);
-        const double Sx_bar = sxb / wsum, Sy_bar = syb / wsum;
+            if (k < n) {
+                double dist;
+                nbr_weight(nb[k], dist, wk[k]);
+                wsum += wk[k];
+            }
+        const double rws = 1.0 / wsum;
+        const double Sx_bar = sxb * rws, Sy_bar = syb * rws;
         SW2D_UNROLL_KU
         for (int k = 0; k < N; k++) {
             if (k < n) {
-                const double dist = sqrt(nb[k].dx * nb[k].dx + nb[k].dy * nb[k].dy);
-                const double w = 1.0 / dist;
-                const double t_bar = Sx_bar * (nb[k].dx / dist / dist * w) + Sy_bar * (nb[k].dy / dist / dist * w);
+                // d(slope term)/dz: (dx, dy) / dist^2 * w, w = 1 / dist
+                const double w3 = wk[k] * wk[k] * wk[k];
+                const double t_bar = Sx_bar * (nb[k].dx * w3) + Sy_bar * (nb[k].dy * w3);
                 zj_bar[k] += t_bar;
                 zc_bar -= t_bar;
             }

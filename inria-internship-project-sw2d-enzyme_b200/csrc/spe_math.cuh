@@ -39,7 +39,7 @@ constexpr double kDtFloor = 1e-6;        // assim/swSpE_hyp.cpp:634
 // source-transformation AD tool produces; the reference's gradient then zeroes non-finite entries).
 SW2D_HD double dsqrt(double s, double sb, bool ieee = false)
 {
-    if (s > 0.0) return sb * 0.5 / s;
+    if (s > 0.0) return sw2d_div(sb * 0.5, s);
     return (ieee && sb != 0.0) ? sb * 0.5 / s : 0.0;
 }
 
@@ -59,23 +59,28 @@ SW2D_HD void desing_rev(double q, double h, double yb, double& qb, double& hb)
     const double h2 = h * h;
     const double h4 = h2 * h2;
     const double e4 = kHDesing * kHDesing * kHDesing * kHDesing;
-    const double den = sqrt(h4 + smax(h4, e4));
+    const double rden = 1.0 / sqrt(h4 + smax(h4, e4));
     const double s = 1.4142135623730951;
     const double num = s * h * q;
-    qb += yb * (s * h) / den;
+    qb += yb * (s * h) * rden;
     const double dh4 = 4.0 * h2 * h;
     const double dS = dh4 + ((h4 < e4) ? 0.0 : dh4);  // d(h4 + max(h4, e4))/dh
-    const double denb = -yb * num / (den * den);
-    hb += yb * (s * q) / den + denb * dS * 0.5 / den;
+    const double denb = -yb * num * (rden * rden);
+    hb += yb * (s * q) * rden + denb * dS * 0.5 * rden;
 }
 
 // ---- wave speeds lambda-/+ = b u -/+ sqrt((b-1) b u^2 + c^2) (swSp.cpp:972-995) -----------
 // adds the adjoints of u and c given those of lambda- and lambda+
 SW2D_HD void lam_rev(double b, double c, double u, double lmb, double lpb, double& ub, double& cb, bool ieee = false)
 {
-    const double R = sqrt((b - 1.0) * b * u * u + c * c);
     ub += b * (lmb + lpb);
     const double Rb = lpb - lmb;
+    // b == 1: the root is c itself (sp_math.cuh, root_is_c), its derivative 1 by c and 0 by u
+    if (warp_all(root_is_c(b, u, c) && c > 0.0)) {
+        cb += Rb;
+        return;
+    }
+    const double R = sqrt((b - 1.0) * b * u * u + c * c);
     if (R > 0.0) {
         ub += Rb * (b - 1.0) * b * u / R;
         cb += Rb * c / R;
@@ -120,8 +125,9 @@ SW2D_HD void god_side_rev(double h, double q, double r, double b, double nx, dou
     hb += dsqrt(c, cb, ieee) * kGravity;
     double qnb = sb.q;
     if (h > h_min) {
-        qnb += ub / h;
-        hb -= ub * u / h;
+        const double rh = 1.0 / h;
+        qnb += ub * rh;
+        hb -= ub * u * rh;
     }
     qb += qnb * nx - sb.r * ny;
     rb += qnb * ny + sb.r * nx;
@@ -321,11 +327,15 @@ SW2D_HD EFlux hllc(double bL, double bR, double phiL, double phiR, double zbL, d
     return f;
 }
 
-// Adds the adjoints of phiL, phiR and of both Riemann states given the flux adjoints fb.
-SW2D_HD void hllc_rev(double bL, double bR, double phiL, double phiR, double zbL, double zbR, const ESide& L,
-                      const ESide& R, double h_min, double phi_min, const EFlux& fb, double& phiLb, double& phiRb,
-                      ESideBar& Lb, ESideBar& Rb)
+// Adds the adjoints of phiL, phiR and of both Riemann states given the flux adjoints fb; returns the
+// fluxes (hllc's to rounding: the reciprocal of each denominator is taken once, and the sign of f1, the
+// one branch that depends on a quotient, is its numerator's).
+SW2D_HD EFlux hllc_rev(double bL, double bR, double phiL, double phiR, double zbL, double zbR, const ESide& L,
+                       const ESide& R, double h_min, double phi_min, const EFlux& fb, double& phiLb, double& phiRb,
+                       ESideBar& Lb, ESideBar& Rb)
 {
+    EFlux out;
+    out.f1 = out.f2 = out.f3 = out.sl = out.sr = 0.0;
     const double dzL = L.z - zbL, dzR = R.z - zbR;
     const double hL = (dzL > 0.0) ? dzL : 0.0;
     const double hR = (dzR > 0.0) ? dzR : 0.0;
@@ -334,8 +344,9 @@ SW2D_HD void hllc_rev(double bL, double bR, double phiL, double phiR, double zbL
     if (reg == kRegBoth) {
         const double hLs = (hL > kSmallReal) ? hL : kSmallReal;
         const double hRs = (hR > kSmallReal) ? hR : kSmallReal;
-        const double uL = L.q / hLs;
-        const double uR = R.q / hRs;
+        const double rL = 1.0 / hLs, rR = 1.0 / hRs;
+        const double uL = L.q * rL;
+        const double uR = R.q * rR;
         const bool l1_left = (L.lm < R.lm);
         double L1 = l1_left ? L.lm : R.lm;
         const bool l1_clamped = (L1 > 0.0);
@@ -347,37 +358,43 @@ SW2D_HD void hllc_rev(double bL, double bR, double phiL, double phiR, double zbL
         double den = L2 - L1;
         const bool den_floor = (den < kSmallReal);
         if (den_floor) den = kSmallReal;
+        const double rden = 1.0 / den;
         const double dphi = phiL - phiR;
         const double sq = sqrt(dphi * dphi + kPhiSmoothEps * kPhiSmoothEps);
         const double phiLR = 0.5 * (phiL + phiR - sq);
         const double A = L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z);
-        const double f1 = phiLR * A / den;
+        const double f1 = phiLR * A * rden;
         const double fact = 0.5 * phiLR * (hL + hR);
         const double s2a = (phiR * hR * hR - phiL * hL * hL) * 0.5 + fact * (L.z - R.z);
-        const double s2 = s2a * kGravity / den;
+        const double s2 = s2a * kGravity * rden;
         const double sl = -L1 * s2, sr = L2 * s2;
         const double FL = spec_force(bL, phiL, hL, uL);
         const double FR = spec_force(bR, phiR, hR, uR);
         const double B = L2 * (FL + sl) - L1 * (FR - sr) + L1 * L2 * (phiR * R.q - phiL * L.q);
-        const double f2 = B / den;
-        const double vL = L.r / hLs, vR = R.r / hRs;
+        const double f2 = B * rden;
+        const double vL = L.r * rL, vR = R.r * rR;
+        out.f1 = f1;
+        out.f2 = f2;
+        out.f3 = (f1 >= 0.0) ? (bL * f1 * vL) : (bR * f1 * vR);
+        out.sl = sl;
+        out.sr = sr;
         double f1b = fb.f1, slb = fb.sl, srb = fb.sr;
         double hLsb = 0.0, hRsb = 0.0, uLb = 0.0, uRb = 0.0, L1b = 0.0, L2b = 0.0, denb = 0.0, phiLRb = 0.0;
         // f3
         if (f1 >= 0.0) {
             f1b += fb.f3 * bL * vL;
             const double vLb = fb.f3 * bL * f1;
-            Lb.r += vLb / hLs;
-            hLsb -= vLb * vL / hLs;
+            Lb.r += vLb * rL;
+            hLsb -= vLb * vL * rL;
         } else {
             f1b += fb.f3 * bR * vR;
             const double vRb = fb.f3 * bR * f1;
-            Rb.r += vRb / hRs;
-            hRsb -= vRb * vR / hRs;
+            Rb.r += vRb * rR;
+            hRsb -= vRb * vR * rR;
         }
         // f2 = B / den
-        const double Bb = fb.f2 / den;
-        denb -= fb.f2 * f2 / den;
+        const double Bb = fb.f2 * rden;
+        denb -= fb.f2 * f2 * rden;
         const double P = phiR * R.q - phiL * L.q;
         L2b += Bb * (FL + sl) + Bb * L1 * P;
         const double FLb = Bb * L2;
@@ -401,8 +418,8 @@ SW2D_HD void hllc_rev(double bL, double bR, double phiL, double phiR, double zbL
         L1b -= slb * s2;
         L2b += srb * s2;
         // s2 = s2a g / den
-        const double s2ab = s2b * kGravity / den;
-        denb -= s2b * s2 / den;
+        const double s2ab = s2b * kGravity * rden;
+        denb -= s2b * s2 * rden;
         phiRb += s2ab * 0.5 * hR * hR;
         hRb += s2ab * phiR * hR;
         phiLb -= s2ab * 0.5 * hL * hL;
@@ -414,9 +431,9 @@ SW2D_HD void hllc_rev(double bL, double bR, double phiL, double phiR, double zbL
         hLb += factb * 0.5 * phiLR;
         hRb += factb * 0.5 * phiLR;
         // f1 = phiLR A / den
-        phiLRb += f1b * A / den;
-        const double Ab = f1b * phiLR / den;
-        denb -= f1b * f1 / den;
+        phiLRb += f1b * A * rden;
+        const double Ab = f1b * phiLR * rden;
+        denb -= f1b * f1 * rden;
         L2b += Ab * (L.q + L1 * (R.z - L.z));
         Lb.q += Ab * L2;
         L1b += Ab * (-R.q + L2 * (R.z - L.z));
@@ -424,8 +441,9 @@ SW2D_HD void hllc_rev(double bL, double bR, double phiL, double phiR, double zbL
         Rb.z += Ab * L1 * L2;
         Lb.z -= Ab * L1 * L2;
         // smooth min of the porosities
-        phiLb += phiLRb * 0.5 * (1.0 - dphi / sq);
-        phiRb += phiLRb * 0.5 * (1.0 + dphi / sq);
+        const double ratio = sw2d_div(dphi, sq);
+        phiLb += phiLRb * 0.5 * (1.0 - ratio);
+        phiRb += phiLRb * 0.5 * (1.0 + ratio);
         // den = max(L2 - L1, small)
         if (!den_floor) {
             L2b += denb;
@@ -440,21 +458,24 @@ SW2D_HD void hllc_rev(double bL, double bR, double phiL, double phiR, double zbL
             else Rb.lp += L2b;
         }
         // velocities u = q / max(h, small)
-        Lb.q += uLb / hLs;
-        hLsb -= uLb * uL / hLs;
-        Rb.q += uRb / hRs;
-        hRsb -= uRb * uR / hRs;
+        Lb.q += uLb * rL;
+        hLsb -= uLb * uL * rL;
+        Rb.q += uRb * rR;
+        hRsb -= uRb * uR * rR;
         if (hL > kSmallReal) hLb += hLsb;
         if (hR > kSmallReal) hRb += hRsb;
     } else if (reg == kRegRhs) {
+        out.sr = phiR * 0.5 * kGravity * hR * hR;
         phiRb += fb.sr * 0.5 * kGravity * hR * hR;
         hRb += fb.sr * phiR * kGravity * hR;
     } else if (reg == kRegLhs) {
+        out.sl = -phiL * 0.5 * kGravity * hL * hL;
         phiLb -= fb.sl * 0.5 * kGravity * hL * hL;
         hLb -= fb.sl * phiL * kGravity * hL;
     }
     if (dzL > 0.0) Lb.z += hLb;
     if (dzR > 0.0) Rb.z += hRb;
+    return out;
 }
 
 // ---- boundary flux (assim/swSpE_hyp.cpp:143-240); type 0 q, 1 h, 2 z, 3 fr, other: no flux -

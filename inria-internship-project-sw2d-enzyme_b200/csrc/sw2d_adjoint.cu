@@ -122,15 +122,6 @@ __global__ void k_note_dt(const Ctrl* ctrl, double* dt_seq, double* t_seq, long 
     }
 }
 
-// in place of k_cfl in a replay: the recorded dt of step j (the host launches exactly the
-// recorded number of steps, so j stays inside dt_seq)
-__global__ void k_frozen_dt(Ctrl* ctrl, const double* dt_seq, long long base)
-{
-    const long long j = ctrl->steps - base;
-    ctrl->dt = dt_seq[j];
-    ctrl->go = 1;
-}
-
 // z = h + z_b of a state array after a change of z_b
 __global__ void k_refresh_z(double4* st, const double* zbv, int n)
 {
@@ -194,6 +185,10 @@ __global__ void __launch_bounds__(kBlock) k_update_rev(DevMesh m, const double4*
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
+    const int k0 = ld(&m.coff[c].y), k1 = ld(&m.coff[c + 1].y);
+    const double4 B = bal[c];
+    const double4 l = lam[c];
+    if (l.x == 0.0 && l.y == 0.0 && l.z == 0.0) return;  // no adjoint: nothing to add anywhere
     UpdateParams p;
     p.friction = kFriction;
     p.head_loss = kHeadLoss;
@@ -225,8 +220,6 @@ __global__ void __launch_bounds__(kBlock) k_update_rev(DevMesh m, const double4*
         p.hcos = b.x;
         p.hsin = b.y;
     }
-    const double4 B = bal[c];
-    const double4 l = lam[c];
     // bal.w: h^(-4/3) of the recomputed step's friction stage, its sign bit set where the
     // velocity cap acted
     p.P_given = true;
@@ -235,7 +228,6 @@ __global__ void __launch_bounds__(kBlock) k_update_rev(DevMesh m, const double4*
     p.cap_acted = signbit(B.w);
     // the adjoints of the cell's first kPre slots, in flight during the cell's reverse
     constexpr int kPre = 4;
-    const int k0 = ld(&m.coff[c].y), k1 = ld(&m.coff[c + 1].y);
     double4 s[kPre];
 #pragma unroll
     for (int i = 0; i < kPre; i++)
@@ -366,6 +358,17 @@ __global__ void __launch_bounds__(kB, kMinB) k_edges_rev(DevMesh m, double4* sig
             const double c = cf.y;
             const SlotFactors f{+c, +c * nx, -c * ny, +c * nx, +c * ny, +c * nx, +c * ny};
             slot_rev(f, sb, fb.f1, fb.f2, fb.f3, fb.sr);
+        }
+        if (fb.f1 == 0.0 && fb.f2 == 0.0 && fb.f3 == 0.0 && fb.sl == 0.0 && fb.sr == 0.0) {
+            // no adjoint has reached the edge's fluxes: none goes on to its states (and the slots'
+            // adjoints are zero already, unless they cancel)
+            if (sa.x != 0.0 || sa.y != 0.0 || sa.z != 0.0) st_sig_zero(&sig[sl.x]);
+            if (sb.x != 0.0 || sb.y != 0.0 || sb.z != 0.0) st_sig_zero(&sig[sl.y]);
+            ctb[sl.x] = make_double4(0.0, 0.0, 0.0, 0.0);
+            ctb[sl.y] = make_double4(0.0, 0.0, 0.0, 0.0);
+            cts[sl.x] = make_double2(0.0, 0.0);
+            cts[sl.y] = make_double2(0.0, 0.0);
+            return;
         }
         st_sig_zero(&sig[sl.x]);
         st_sig_zero(&sig[sl.y]);
@@ -658,10 +661,10 @@ int run_trajectory(sw2d_handle* h, bool record, F&& at_step)
         if (record) {
             launch_cfl_on(h, h->m);
             k_note_dt<<<1, 1, 0, h->stream>>>(h->ctrl, a->d_dt_seq, a->d_t_seq, a->base_steps);
-        } else {
-            k_frozen_dt<<<1, 1, 0, h->stream>>>(h->ctrl, a->d_dt_seq, a->base_steps);
         }
-        launch_update_on(h, h->m, false);
+        DevMesh mu = h->m;
+        if (!record) mu.dt_fixed = a->d_dt_seq + j;  // in place of k_cfl
+        launch_update_on(h, mu, false);
         at_step(j + 1);
     }
     if ((rc = ck_save(h, a->n_ck))) return rc;
@@ -845,7 +848,7 @@ int reverse_sweep(sw2d_handle* h)
             if (a->seg_rs) mj.rstate = a->seg_rs + (j - j0) * 5 * h->ni;
             launch_slopes_on(h, mj);
             launch_edges_on(h, mj);
-            k_frozen_dt<<<1, 1, 0, h->stream>>>(h->ctrl, a->d_dt_seq, a->base_steps);
+            mj.dt_fixed = a->d_dt_seq + j;
             launch_update_on(h, mj, true);
             const int k = obs_index(a, j + 1);
             if (k >= 0) cost_at(h, k, mj.st_out);

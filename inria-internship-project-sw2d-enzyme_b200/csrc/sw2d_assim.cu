@@ -467,6 +467,10 @@ __global__ void __launch_bounds__(kBlock) k_e_update_rev(DevMesh m, const double
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const double4 l = lam[c];
+    if (l.x == 0.0 && l.y == 0.0 && l.z == 0.0) {  // no adjoint: none before the update either
+        lamb[c] = make_double4(0.0, 0.0, 0.0, 0.0);
+        return;
+    }
     const double4 b = bal[c];
     spe::ECellParams p;
     p.friction = kFriction != SW2D_FRICTION_NONE;
@@ -512,14 +516,20 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
         const int e = i;
         const int2 lr = ld(&m.lr[e]);
         const int a = lr.x, b = lr.y;
+        const double4 lL = ld(&lamb[a]), lR = ld(&lamb[b]);
+        const int2 sl = ld(&m.eslot[e]);
+        if (lL.x == 0.0 && lL.y == 0.0 && lL.z == 0.0 && lR.x == 0.0 && lR.y == 0.0 && lR.z == 0.0) {
+            // neither cell has an adjoint: the edge passes none on
+            ctb[sl.x] = ctb[sl.y] = make_double4(0.0, 0.0, 0.0, 0.0);
+            if (kScheme != SW2D_SCHEME_GODUNOV) cts[sl.x] = cts[sl.y] = make_double2(0.0, 0.0);
+            return;
+        }
         const double2 n = ld(&m.nxy[e]);
         const double4 sa = ld(&m.st[a]), sb = ld(&m.st[b]);
         const double4 ca = ld(&m.cst[a]), cb = ld(&m.cst[b]);
         spe::ESide SL, SR;
         e_sides<kScheme>(m, e, a, b, n, sa, sb, ca, cb, dt, SL, SR);
         const double phiL = ld(&v.phi[a]), phiR = ld(&v.phi[b]);
-        const spe::EFlux f = spe::hllc(ca.y, cb.y, phiL, phiR, ca.x, cb.x, SL, SR, m.h_min, m.phi_min);
-        const double4 lL = ld(&lamb[a]), lR = ld(&lamb[b]);
         const double2 cf = ld(&v.coef[e]);
         const double cL = cf.x, cR = cf.y, nx = n.x, ny = n.y;
         spe::EFlux fb;
@@ -528,15 +538,17 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
         fb.f3 = dt * (cL * (ny * lL.y - nx * lL.z) + cR * (-ny * lR.y + nx * lR.z));
         fb.sl = dt * cL * (nx * lL.y + ny * lL.z);
         fb.sr = dt * cR * (nx * lR.y + ny * lR.z);
+        double pLb = 0.0, pRb = 0.0;
+        spe::ESideBar Lb{0, 0, 0, 0, 0}, Rb{0, 0, 0, 0, 0};
+        const spe::EFlux f =
+            spe::hllc_rev(ca.y, cb.y, phiL, phiR, ca.x, cb.x, SL, SR, m.h_min, m.phi_min, fb, pLb, pRb, Lb, Rb);
+        // the factors w / (A phi)
         const double cLb = dt * (-f.f1 * lL.x + (-nx * f.f2 + nx * f.sl + ny * f.f3) * lL.y +
                                  (-ny * f.f2 + ny * f.sl - nx * f.f3) * lL.z);
         const double cRb = dt * (f.f1 * lR.x + (nx * f.f2 + nx * f.sr - ny * f.f3) * lR.y +
                                  (ny * f.f2 + ny * f.sr + nx * f.f3) * lR.z);
-        double pLb = (phiL > m.phi_min) ? -cLb * cL / phiL : 0.0;
-        double pRb = (phiR > m.phi_min) ? -cRb * cR / phiR : 0.0;
-        spe::ESideBar Lb{0, 0, 0, 0, 0}, Rb{0, 0, 0, 0, 0};
-        spe::hllc_rev(ca.y, cb.y, phiL, phiR, ca.x, cb.x, SL, SR, m.h_min, m.phi_min, fb, pLb, pRb, Lb, Rb);
-        const int2 sl = ld(&m.eslot[e]);
+        if (phiL > m.phi_min) pLb -= sw2d_div(cLb * cL, phiL);
+        if (phiR > m.phi_min) pRb -= sw2d_div(cRb * cR, phiR);
         double hb = 0, qb = 0, rb = 0;
         if (kScheme == SW2D_SCHEME_GODUNOV) {
             spe::god_side_rev(sa.x, sa.y, sa.z, ca.y, nx, ny, m.h_min, Lb, hb, qb, rb, ieee);

@@ -178,6 +178,7 @@ struct DevMesh {
     double h_min, phi_min, cfl_max, dt_max, dt_map, v_max, fr_max;
     DryConsts dry;
     int neg_detect;
+    const double* dt_fixed;  // optional: the recorded dt a replayed step takes (else null: ctrl->dt)
     int geo_plain;   // the mesh's lengths allow div_known in the slopes (slope_length_ok)
     int rev_update;  // the cell update walks its blocks from the last cells to the first
     // dt reduction scratch

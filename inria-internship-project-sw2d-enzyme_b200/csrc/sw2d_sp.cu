@@ -157,8 +157,9 @@ template <int kFriction, bool kHeadLoss, bool kStoreB, bool kDissip>
 __global__ void __launch_bounds__(kBlock, 4) k_update(DevMesh m)
 {
     Ctrl* ctrl = m.ctrl;
-    if (!ctrl->go) return;
-    const double dt = ctrl->dt;
+    const bool fixed = m.dt_fixed != nullptr;  // a replayed step: its dt is recorded, and thread 0 keeps it
+    if (!fixed && !ctrl->go) return;
+    const double dt = fixed ? *m.dt_fixed : ctrl->dt;
     // with rev_update the blocks take the cells from the end: the flux kernel finishes on the last
     // tiles, whose slots and states are then still in L2
     const int blk = m.rev_update ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
@@ -166,6 +167,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_update(DevMesh m)
     if (c == 0) {
         ctrl->t = ctrl->t + dt;  // swSp.cpp:592; no other thread of this kernel reads t
         ctrl->steps += 1;
+        if (fixed) {
+            ctrl->dt = dt;
+            ctrl->go = 1;
+        }
     }
     if (c >= m.nc) return;
     update_cell<kFriction, kHeadLoss, kStoreB, kDissip, LdNc>(m, c, dt);
