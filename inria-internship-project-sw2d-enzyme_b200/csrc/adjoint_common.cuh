@@ -163,6 +163,7 @@ __device__ __forceinline__ double slope_rev_cell(const DevMesh& m, int e0, int c
 __global__ void __launch_bounds__(kBlock) k_limiter_rev(DevMesh m, const double2* __restrict__ sgb, double4* lam,
                                                         double* gzb, double* znb)
 {
+    chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const int e0 = ld(&m.coff[c].x), e1 = ld(&m.coff[c + 1].x);
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(kBlock) k_limiter_rev(DevMesh m, const double2
 __global__ void __launch_bounds__(kBlock) k_nbr_rev(DevMesh m, const int* __restrict__ mirror,
                                                     const double* __restrict__ znb, double4* lam, double* gzb)
 {
+    chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     constexpr int kPre = 4;

@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(kBlock) k_update_rev(DevMesh m, const double4*
                                                        double4* sig, double* gk1, double* gk2, double dt,
                                                        int flush_branch)
 {
+    chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const int k0 = ld(&m.coff[c].y), k1 = ld(&m.coff[c + 1].y);
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_edges_rev(DevMesh m, double4* sig
                                                          double dtp, const double2* __restrict__ rs,
                                                          const double2* __restrict__ eside)
 {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m.ni) {
         const int e = i;
@@ -468,6 +470,7 @@ __global__ void __launch_bounds__(kBlock) k_cells_rev(DevMesh m, double4* lam, c
                                                       const double2* __restrict__ cts, double* gzb, double2* sgb,
                                                       double dtp, const double4* __restrict__ sgeo)
 {
+    chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     constexpr bool kMuscl = kScheme == SW2D_SCHEME_MUSCL_EVR;
@@ -697,10 +700,10 @@ void launch_update_rev_f(sw2d_handle* h, const double4* bal, double dt)
     AdjointState* a = h->adj;
     const unsigned g = grid_for(h->nc);
     if (h->p.singular_head_loss)
-        k_update_rev<kF, true><<<g, kBlock, 0, h->stream>>>(h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
+        launch_chained(k_update_rev<kF, true>, g, kBlock, 0, h->stream, h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
                                                             h->adj_flush_branch);
     else
-        k_update_rev<kF, false><<<g, kBlock, 0, h->stream>>>(h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
+        launch_chained(k_update_rev<kF, false>, g, kBlock, 0, h->stream, h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
                                                              h->adj_flush_branch);
 }
 
@@ -729,10 +732,10 @@ void launch_edges_rev_v(sw2d_handle* h, const DevMesh& m, double t, double dtp, 
     AdjointState* a = h->adj;
     const unsigned n = (unsigned)(m.ni + m.nb);
     if (rs)
-        k_edges_rev<kScheme, kBlending, B, M, true><<<(n + B - 1) / B, B, 0, h->stream>>>(m, a->sig, a->ctb, a->cts, t,
+        launch_chained(k_edges_rev<kScheme, kBlending, B, M, true>, (n + B - 1) / B, B, 0, h->stream, m, a->sig, a->ctb, a->cts, t,
                                                                                           dtp, rs, a->eside);
     else
-        k_edges_rev<kScheme, kBlending, B, M, false><<<(n + B - 1) / B, B, 0, h->stream>>>(m, a->sig, a->ctb, a->cts, t,
+        launch_chained(k_edges_rev<kScheme, kBlending, B, M, false>, (n + B - 1) / B, B, 0, h->stream, m, a->sig, a->ctb, a->cts, t,
                                                                                            dtp, rs, nullptr);
 }
 
@@ -875,12 +878,12 @@ int reverse_sweep(sw2d_handle* h)
                              a->seg_rs ? a->seg_rs + (j - j0) * 5 * h->ni : nullptr);
             const double dtp = j > 0 ? a->dt_seq[j - 1] : a->dt_before;
             if (muscl) {
-                k_cells_rev<SW2D_SCHEME_MUSCL_EVR><<<gc, kBlock, 0, h->stream>>>(mr, a->lam, a->ctb, a->cts, a->g_zb,
+                launch_chained(k_cells_rev<SW2D_SCHEME_MUSCL_EVR>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_zb,
                                                                                   a->sgb, dtp, a->sgeo);
-                k_limiter_rev<<<gc, kBlock, 0, h->stream>>>(mr, a->sgb, a->lam, a->g_zb, a->znb);
-                k_nbr_rev<<<gc, kBlock, 0, h->stream>>>(mr, a->mirror, a->znb, a->lam, a->g_zb);
+                launch_chained(k_limiter_rev, gc, kBlock, 0, h->stream, mr, a->sgb, a->lam, a->g_zb, a->znb);
+                launch_chained(k_nbr_rev, gc, kBlock, 0, h->stream, mr, a->mirror, a->znb, a->lam, a->g_zb);
             } else {
-                k_cells_rev<SW2D_SCHEME_GODUNOV><<<gc, kBlock, 0, h->stream>>>(mr, a->lam, a->ctb, a->cts, a->g_zb,
+                launch_chained(k_cells_rev<SW2D_SCHEME_GODUNOV>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_zb,
                                                                                 a->sgb, dtp, a->sgeo);
             }
             if (a->d_trace && j < a->trace_steps)

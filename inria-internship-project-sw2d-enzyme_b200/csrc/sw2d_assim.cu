@@ -210,6 +210,7 @@ __device__ __forceinline__ double e_bc_value(const DevMesh& m, int e, double t, 
 template <int kScheme, bool kRecord>
 __global__ void __launch_bounds__(kBlock) k_e_edges(DevMesh m, EView v)
 {
+    chain_begin();
     if (kRecord && !step_active(m.ctrl)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m.ni) {
@@ -283,6 +284,7 @@ __device__ __forceinline__ double e_min_keep(double a, double b) { return (b < a
 __global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, const double* __restrict__ obs_t, const int* obs_idx,
                                                   int n_obs)
 {
+    chain_begin();
     Ctrl* ctrl = m.ctrl;
     if (!step_active(ctrl)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->go = 0;
@@ -349,6 +351,7 @@ __global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, const double* __res
 template <int kFriction, bool kHeadLoss, bool kStore>
 __global__ void __launch_bounds__(kBlock) k_e_update(DevMesh m, const double* __restrict__ dtp, const int* go)
 {
+    chain_begin();
     if (go && !*go) return;
     const double dt = *dtp;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -406,6 +409,7 @@ __global__ void __launch_bounds__(kBlock) k_e_update(DevMesh m, const double* __
 __global__ void k_e_advance(Ctrl* ctrl, int* obs_idx, const double* __restrict__ obs_t, int n_obs, double* dt_seq,
                             double* t_seq, int* trig, long long cap)
 {
+    chain_begin();
     if (!ctrl->go) return;
     const long long j = ctrl->steps;
     const double t0 = ctrl->t, dt = ctrl->dt;
@@ -464,6 +468,7 @@ template <int kFriction, bool kHeadLoss>
 __global__ void __launch_bounds__(kBlock) k_e_update_rev(DevMesh m, const double4* __restrict__ bal, double4* lam,
                                                          double4* lamb, double* gk1, double* gk2, double dt)
 {
+    chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const double4 l = lam[c];
@@ -511,6 +516,7 @@ template <int kScheme>
 __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, const double4* __restrict__ lamb,
                                                         double4* ctb, double2* cts, double dt, int ieee)
 {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m.ni) {
         const int e = i;
@@ -604,6 +610,7 @@ template <bool kMuscl>
 __global__ void __launch_bounds__(kBlock) k_e_cells_rev(DevMesh m, double4* lam, const double4* __restrict__ ctb,
                                                         const double2* __restrict__ cts, double* gphi, double2* sgb)
 {
+    chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
     const int k0 = ld(&m.coff[c].y), k1 = ld(&m.coff[c + 1].y);
@@ -782,8 +789,8 @@ void launch_edges(sw2d_handle* h, const DevMesh& m, const EView& v)
 {
     const unsigned g = grid_for(h->ni + h->nb);
     if (g == 0) return;
-    if (h->p.scheme == SW2D_SCHEME_GODUNOV) k_e_edges<SW2D_SCHEME_GODUNOV, kRecord><<<g, kBlock, 0, h->stream>>>(m, v);
-    else k_e_edges<SW2D_SCHEME_MUSCL_EVR, kRecord><<<g, kBlock, 0, h->stream>>>(m, v);
+    if (h->p.scheme == SW2D_SCHEME_GODUNOV) launch_chained(k_e_edges<SW2D_SCHEME_GODUNOV, kRecord>, g, kBlock, 0, h->stream, m, v);
+    else launch_chained(k_e_edges<SW2D_SCHEME_MUSCL_EVR, kRecord>, g, kBlock, 0, h->stream, m, v);
 }
 
 template <int kF>
@@ -791,11 +798,11 @@ void launch_update_f(sw2d_handle* h, const DevMesh& m, const double* dtp, const 
 {
     const unsigned g = grid_for(h->nc);
     if (h->p.singular_head_loss) {
-        if (store) k_e_update<kF, true, true><<<g, kBlock, 0, h->stream>>>(m, dtp, go);
-        else k_e_update<kF, true, false><<<g, kBlock, 0, h->stream>>>(m, dtp, go);
+        if (store) launch_chained(k_e_update<kF, true, true>, g, kBlock, 0, h->stream, m, dtp, go);
+        else launch_chained(k_e_update<kF, true, false>, g, kBlock, 0, h->stream, m, dtp, go);
     } else {
-        if (store) k_e_update<kF, false, true><<<g, kBlock, 0, h->stream>>>(m, dtp, go);
-        else k_e_update<kF, false, false><<<g, kBlock, 0, h->stream>>>(m, dtp, go);
+        if (store) launch_chained(k_e_update<kF, false, true>, g, kBlock, 0, h->stream, m, dtp, go);
+        else launch_chained(k_e_update<kF, false, false>, g, kBlock, 0, h->stream, m, dtp, go);
     }
 }
 
@@ -811,10 +818,10 @@ void launch_update_rev(sw2d_handle* h, const DevMesh& m, const double4* bal, dou
     AssimState* a = h->assim;
     const unsigned g = grid_for(h->nc);
     const bool fr = h->p.friction != SW2D_FRICTION_NONE, hl = h->p.singular_head_loss != 0;
-    if (fr && hl) k_e_update_rev<SW2D_FRICTION_STRICKLER, true><<<g, kBlock, 0, h->stream>>>(m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
-    else if (fr) k_e_update_rev<SW2D_FRICTION_STRICKLER, false><<<g, kBlock, 0, h->stream>>>(m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
-    else if (hl) k_e_update_rev<SW2D_FRICTION_NONE, true><<<g, kBlock, 0, h->stream>>>(m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
-    else k_e_update_rev<SW2D_FRICTION_NONE, false><<<g, kBlock, 0, h->stream>>>(m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    if (fr && hl) launch_chained(k_e_update_rev<SW2D_FRICTION_STRICKLER, true>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    else if (fr) launch_chained(k_e_update_rev<SW2D_FRICTION_STRICKLER, false>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    else if (hl) launch_chained(k_e_update_rev<SW2D_FRICTION_NONE, true>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    else launch_chained(k_e_update_rev<SW2D_FRICTION_NONE, false>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
 }
 
 int64_t obs_width(const AssimState* a, const sw2d_handle* h)
@@ -985,9 +992,9 @@ int record(sw2d_handle* h, int64_t stride)
         for (int64_t j = 0; j < stride; j++) {
             if (muscl) launch_slopes_on(h, m);
             launch_edges<true>(h, m, v);
-            if (gc > 0) k_e_cfl<<<gc, kBlock, 0, h->stream>>>(m, a->d_obs_t, a->d_obs_idx, (int)a->n_obs);
+            if (gc > 0) launch_chained(k_e_cfl, gc, kBlock, 0, h->stream, m, a->d_obs_t, a->d_obs_idx, (int)a->n_obs);
             launch_update(h, m, &a->ctrl->dt, &a->ctrl->go, false);
-            k_e_advance<<<1, 1, 0, h->stream>>>(a->ctrl, a->d_obs_idx, a->d_obs_t, (int)a->n_obs, a->d_dt, a->d_t,
+            launch_chained(k_e_advance, 1, 1, 0, h->stream, a->ctrl, a->d_obs_idx, a->d_obs_t, (int)a->n_obs, a->d_dt, a->d_t,
                                                  a->d_trig, (long long)a->cap);
         }
         CK(cudaGetLastError());
@@ -1181,16 +1188,16 @@ int reverse_segment(sw2d_handle* h, int64_t k)
         if (ge > 0) {
             const int ieee = h->assim_sqrt_zero;
             if (muscl)
-                k_e_edges_rev<SW2D_SCHEME_MUSCL_EVR><<<ge, kBlock, 0, h->stream>>>(mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
-            else k_e_edges_rev<SW2D_SCHEME_GODUNOV><<<ge, kBlock, 0, h->stream>>>(mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
+                launch_chained(k_e_edges_rev<SW2D_SCHEME_MUSCL_EVR>, ge, kBlock, 0, h->stream, mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
+            else launch_chained(k_e_edges_rev<SW2D_SCHEME_GODUNOV>, ge, kBlock, 0, h->stream, mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
         }
         if (gc > 0) {
             if (muscl) {
-                k_e_cells_rev<true><<<gc, kBlock, 0, h->stream>>>(mr, a->lam, a->ctb, a->cts, a->g_phi, a->sgb);
-                k_limiter_rev<<<gc, kBlock, 0, h->stream>>>(mr, a->sgb, a->lam, a->gzb, a->znb);
-                k_nbr_rev<<<gc, kBlock, 0, h->stream>>>(mr, a->mirror, a->znb, a->lam, a->gzb);
+                launch_chained(k_e_cells_rev<true>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_phi, a->sgb);
+                launch_chained(k_limiter_rev, gc, kBlock, 0, h->stream, mr, a->sgb, a->lam, a->gzb, a->znb);
+                launch_chained(k_nbr_rev, gc, kBlock, 0, h->stream, mr, a->mirror, a->znb, a->lam, a->gzb);
             } else {
-                k_e_cells_rev<false><<<gc, kBlock, 0, h->stream>>>(mr, a->lam, a->ctb, a->cts, a->g_phi, a->sgb);
+                launch_chained(k_e_cells_rev<false>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_phi, a->sgb);
             }
         }
     }

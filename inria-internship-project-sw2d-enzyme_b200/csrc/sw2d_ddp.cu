@@ -149,6 +149,7 @@ __device__ __forceinline__ void put_bnd_slot(const DevMesh& m, double4 g, int sb
 template <int kB, int kMinB>
 __global__ void __launch_bounds__(kB, kMinB) k_ddp_edges(DevMesh m)
 {
+    chain_begin();
     if (!step_active(m.ctrl)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned bad = 0;
@@ -337,6 +338,7 @@ __device__ __forceinline__ void finish_cell(const DevMesh& m, int c, double dt, 
 template <int kF, bool kHL, bool kDissip>
 __global__ void __launch_bounds__(kBlock, 3) k_ddp_update(DevMesh m)
 {
+    chain_begin();
     Ctrl* ctrl = m.ctrl;
     if (!ctrl->go) return;
     const double dt = ctrl->dt;
@@ -801,7 +803,7 @@ void launch_edges_v(sw2d_handle* h, const DevMesh& m)
 {
     constexpr int B = kDdpVariants[V].block, M = kDdpVariants[V].minb;
     const unsigned n = (unsigned)(m.ni + m.nb);
-    k_ddp_edges<B, M><<<(n + B - 1) / B, B, 0, h->stream>>>(m);
+    launch_chained(k_ddp_edges<B, M>, (n + B - 1) / B, B, 0, h->stream, m);
 }
 
 template <int kF, bool kHL>
@@ -810,8 +812,8 @@ void launch_tail_f(sw2d_handle* h, const DevMesh& m)
     const unsigned g = grid_for(m.nc);
     DdpState* d = h->ddp;
     if (d->div_corr == kDivCorrNone) {
-        if (h->dissipation) k_ddp_update<kF, kHL, true><<<g, kBlock, 0, h->stream>>>(m);
-        else k_ddp_update<kF, kHL, false><<<g, kBlock, 0, h->stream>>>(m);
+        if (h->dissipation) launch_chained(k_ddp_update<kF, kHL, true>, g, kBlock, 0, h->stream, m);
+        else launch_chained(k_ddp_update<kF, kHL, false>, g, kBlock, 0, h->stream, m);
         return;
     }
     k_ddp_balance<<<g, kBlock, 0, h->stream>>>(m, h->dissipation != 0);

@@ -226,6 +226,34 @@ __device__ __forceinline__ double ld_now(const double* p)
     return v;
 }
 
+// The kernels of a time step (forward and reverse) follow one another on one stream and are launched
+// as programmatic dependents (launch_chained): a kernel's blocks may be placed while the previous
+// kernel's last ones run.  Each begins with chain_begin, which waits until the previous kernel has
+// finished and its writes are visible, then lets the next one be placed; nothing is read or written
+// before it.
+__device__ __forceinline__ void chain_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... KArgs, class... Args>
+inline void launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                           Args&&... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);  // errors: cudaGetLastError, as after <<<>>>
+}
+
 __device__ __forceinline__ bool step_active(const Ctrl* c) { return c->t < c->t_max; }
 
 inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }

@@ -1031,6 +1031,7 @@ __global__ void k_closure_phig_min(DevMesh m, float* out)
 template <int kFriction, bool kHeadLoss>
 __global__ void __launch_bounds__(128) k_update_closure(DevMesh m, ClosureArgs a)
 {
+    chain_begin();
     __shared__ __align__(1024) uint16_t sX[kTileM * kInPad];
     __shared__ __align__(1024) uint16_t sH[kTileM * kHid];
     __shared__ __align__(1024) uint16_t sW1[kHid * kInPad];
@@ -1246,8 +1247,8 @@ cudaError_t closure_carveout()
 template <int kF>
 void launch_closure_f(sw2d_handle* h, const DevMesh& m, const ClosureArgs& a, unsigned g)
 {
-    if (h->p.singular_head_loss) k_update_closure<kF, true><<<g, 128, 0, h->stream>>>(m, a);
-    else k_update_closure<kF, false><<<g, 128, 0, h->stream>>>(m, a);
+    if (h->p.singular_head_loss) launch_chained(k_update_closure<kF, true>, g, 128, 0, h->stream, m, a);
+    else launch_chained(k_update_closure<kF, false>, g, 128, 0, h->stream, m, a);
 }
 
 ClosureNorm closure_norm(const ClosureState* c)

@@ -58,6 +58,7 @@ namespace {
 template <int kB, int kMinB>
 __global__ void __launch_bounds__(kB, kMinB) k_slopes(DevMesh m)
 {
+    chain_begin();
     if (!step_active(m.ctrl)) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_slopes(DevMesh m)
 template <int kScheme, bool kBlending, int kModel, int kB, int kMinB>
 __global__ void __launch_bounds__(kB, kMinB) k_edges(DevMesh m)
 {
+    chain_begin();
     if (!step_active(m.ctrl)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned bad = 0;
@@ -101,6 +103,7 @@ unsigned cfl_grid(sw2d_handle* h, int nc)
 template <bool kDdpSnap>
 __global__ void __launch_bounds__(kBlock) k_cfl(DevMesh m)
 {
+    chain_begin();
     Ctrl* ctrl = m.ctrl;
     if (!step_active(ctrl)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->go = 0;
@@ -156,6 +159,7 @@ __global__ void __launch_bounds__(kBlock) k_cfl(DevMesh m)
 template <int kFriction, bool kHeadLoss, bool kStoreB, bool kDissip>
 __global__ void __launch_bounds__(kBlock, 4) k_update(DevMesh m)
 {
+    chain_begin();
     Ctrl* ctrl = m.ctrl;
     const bool fixed = m.dt_fixed != nullptr;  // a replayed step: its dt is recorded, and thread 0 keeps it
     if (!fixed && !ctrl->go) return;
@@ -340,7 +344,7 @@ template <int kScheme, bool kBlending, int kModel, int V>
 void launch_edges_v(sw2d_handle* h, const DevMesh& m, unsigned n)
 {
     constexpr int B = kVariants[V].block, M = kVariants[V].minb;
-    k_edges<kScheme, kBlending, kModel, B, M><<<(n + B - 1) / B, B, 0, h->stream>>>(m);
+    launch_chained(k_edges<kScheme, kBlending, kModel, B, M>, (n + B - 1) / B, B, 0, h->stream, m);
 }
 
 template <int kScheme, bool kBlending, int kModel>
@@ -383,7 +387,7 @@ template <int V>
 void launch_slopes_v(sw2d_handle* h, const DevMesh& m)
 {
     constexpr int B = kVariants[V].block, M = kVariants[V].minb;
-    k_slopes<B, M><<<((unsigned)m.nc + B - 1) / B, B, 0, h->stream>>>(m);
+    launch_chained(k_slopes<B, M>, ((unsigned)m.nc + B - 1) / B, B, 0, h->stream, m);
 }
 
 void launch_slopes(sw2d_handle* h, const DevMesh& m, int v)
@@ -403,8 +407,8 @@ void launch_slopes(sw2d_handle* h, int v) { launch_slopes(h, h->m, v); }
 template <int kF, bool kStoreB, bool kDissip>
 void launch_update_f(sw2d_handle* h, const DevMesh& m, unsigned g)
 {
-    if (h->p.singular_head_loss) k_update<kF, true, kStoreB, kDissip><<<g, kBlock, 0, h->stream>>>(m);
-    else k_update<kF, false, kStoreB, kDissip><<<g, kBlock, 0, h->stream>>>(m);
+    if (h->p.singular_head_loss) launch_chained(k_update<kF, true, kStoreB, kDissip>, g, kBlock, 0, h->stream, m);
+    else launch_chained(k_update<kF, false, kStoreB, kDissip>, g, kBlock, 0, h->stream, m);
 }
 
 template <bool kStoreB, bool kDissip>
@@ -460,7 +464,7 @@ void launch_phase(sw2d_handle* h, int i)
             if (h->p.scheme == SW2D_SCHEME_MUSCL_EVR) launch_slopes(h, h->slope_variant);
             break;
         case 1: launch_edges(h, h->edge_variant); break;
-        case 2: k_cfl<false><<<cfl_grid(h, m.nc), kBlock, 0, h->stream>>>(m); break;
+        case 2: launch_chained(k_cfl<false>, cfl_grid(h, m.nc), kBlock, 0, h->stream, m); break;
         default: launch_update_s<false>(h, m); break;
     }
 }
@@ -492,9 +496,9 @@ void launch_slopes_on(sw2d_handle* h, const DevMesh& m)
 
 void launch_edges_on(sw2d_handle* h, const DevMesh& m) { launch_edges(h, m, h->edge_variant); }
 
-void launch_cfl_on(sw2d_handle* h, const DevMesh& m) { k_cfl<false><<<cfl_grid(h, m.nc), kBlock, 0, h->stream>>>(m); }
+void launch_cfl_on(sw2d_handle* h, const DevMesh& m) { launch_chained(k_cfl<false>, cfl_grid(h, m.nc), kBlock, 0, h->stream, m); }
 
-void launch_cfl_ddp_on(sw2d_handle* h, const DevMesh& m) { k_cfl<true><<<cfl_grid(h, m.nc), kBlock, 0, h->stream>>>(m); }
+void launch_cfl_ddp_on(sw2d_handle* h, const DevMesh& m) { launch_chained(k_cfl<true>, cfl_grid(h, m.nc), kBlock, 0, h->stream, m); }
 
 void launch_step_on(sw2d_handle* h) { launch_step(h); }
 
@@ -1308,7 +1312,7 @@ int sw2d_autotune_step(sw2d_handle* h, int iters, const int* tile_sizes, int n_t
             edge_v = v;
         }
     }
-    const double t_cfl = time_it([&] { k_cfl<false><<<cfl_grid(h, h->m.nc), kBlock, 0, h->stream>>>(h->m); });
+    const double t_cfl = time_it([&] { launch_chained(k_cfl<false>, cfl_grid(h, h->m.nc), kBlock, 0, h->stream, h->m); });
     const double t_four = t_slopes + t_edges + t_cfl;
     rep += "four-kernel=" + std::to_string(t_four) + "ms ";
     // fused forms: for MUSCL-EVR both places of the slopes, every tile size
