@@ -160,7 +160,7 @@ __device__ __forceinline__ double slope_rev_cell(const DevMesh& m, int e0, int c
 
 // Reverse of each cell's slope limiter (MUSCL-EVR): the cell's own z contribution is applied
 // here, the neighbours' go to znb (one value per internal-neighbour entry).
-__global__ void __launch_bounds__(kBlock) k_limiter_rev(DevMesh m, const double2* __restrict__ sgb, double4* lam,
+__global__ void __launch_bounds__(kBlock) k_limiter_rev(DevMesh m, const double2* sgb, double4* lam,
                                                         double* gzb, double* znb)
 {
     chain_begin();
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kBlock) k_limiter_rev(DevMesh m, const double2
 // z contributions of the neighbours' slope limiters, gathered in the cell's entry order (the
 // first kPre entries' loads in flight together)
 __global__ void __launch_bounds__(kBlock) k_nbr_rev(DevMesh m, const int* __restrict__ mirror,
-                                                    const double* __restrict__ znb, double4* lam, double* gzb)
+                                                    const double* znb, double4* lam, double* gzb)
 {
     chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kBlock) k_nbr_rev(DevMesh m, const int* __rest
         if (e0 + i < e1) mk[i] = ld_now(&mirror[e0 + i]);  // every internal edge has an entry on both sides
 #pragma unroll
     for (int i = 0; i < kPre; i++)
-        if (e0 + i < e1 && mk[i] >= 0) z[i] = ld_now(&znb[mk[i]]);
+        if (e0 + i < e1 && mk[i] >= 0) z[i] = ld_prev_now(&znb[mk[i]]);
     double s = 0.0;
 #pragma unroll
     for (int i = 0; i < kPre; i++)

@@ -11,12 +11,12 @@
 //   update_cell     one cell's balance, flush, clamp, sources  swSpHyp.cpp:184-273, swSpSourceFriction.cpp
 //
 // The load policy L says how a body reads the arrays that the step itself writes (states,
-// slopes, balance slots, CFL contributions, the control block).  LdNc: the step kernels, where
-// those arrays were written by an earlier kernel, through the read-only path.  LdL2: through L2
-// only.  LdCo: plain (coherent, L1-cached) loads, for the work-queue kernel, where other CTAs of
-// the same launch wrote the arrays: each item starts after a gpu-scope acquire of the counter
-// its prerequisites released, followed by a CTA barrier, and the memory model then orders its
-// plain loads after those writes (the read-only path gives no such guarantee).  The arithmetic
+// slopes, balance slots, CFL contributions, the control block).  LdL2: through L2 only.  LdCo:
+// plain (coherent, L1-cached) loads.  In the step kernels an earlier kernel wrote those arrays,
+// and the launch chain lets a kernel begin before the previous one has ended, so the read-only
+// path would not do.  In the work-queue kernel other CTAs of the same launch wrote them: each item
+// starts after a gpu-scope acquire of the counter its prerequisites released, followed by a CTA
+// barrier, and the memory model then orders its plain loads after those writes.  The arithmetic
 // is the same under every policy.
 #pragma once
 
@@ -40,16 +40,6 @@ __device__ __forceinline__ Slot ldl2(const Slot* p)
     const double* q = reinterpret_cast<const double*>(p);
     return make_slot(__ldcg(q), __ldcg(q + 1), __ldcg(q + 2));
 }
-
-struct LdNc {
-    // an array written by an earlier kernel
-    template <class T>
-    static __device__ __forceinline__ T in(const T* p) { return ld(p); }
-    // an array this thread reads and then writes (the update's own state and slots)
-    template <class T>
-    static __device__ __forceinline__ T own(const T* p) { return *p; }
-    static __device__ __forceinline__ double ctl(const double* p) { return *p; }
-};
 
 struct LdL2 {
     template <class T>
@@ -378,7 +368,7 @@ __device__ __forceinline__ double dt_snap(double dt_map, double t, double t_max,
 }
 
 // dt_finalize: dt_snap of the grid minimum into the control block's dt, go and store_map
-template <bool kDdpSnap, class L = LdNc>
+template <bool kDdpSnap, class L = LdCo>
 __device__ __forceinline__ void dt_finalize(const DevMesh& m, Ctrl* ctrl, double dt)
 {
     int store;

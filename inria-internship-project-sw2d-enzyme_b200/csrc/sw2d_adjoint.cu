@@ -179,7 +179,7 @@ __device__ __forceinline__ void st_sig_zero(double4* p) { st_sig(p, 0.0, 0.0, 0.
 // becomes the adjoint of the state before it (balance part); the slots' adjoints gain
 // dt * (adjoint of the post-balance state); friction-coefficient gradients accumulate.
 template <int kFriction, bool kHeadLoss>
-__global__ void __launch_bounds__(kBlock) k_update_rev(DevMesh m, const double4* __restrict__ bal, double4* lam,
+__global__ void __launch_bounds__(kBlock) k_update_rev(DevMesh m, const double4* bal, double4* lam,
                                                        double4* sig, double* gk1, double* gk2, double dt,
                                                        int flush_branch)
 {
@@ -272,7 +272,7 @@ __device__ __forceinline__ void slot_rev(const SlotFactors& f, const double4& s,
 // are rebuilt here from the cells.
 template <int kScheme, bool kBlending, int kB, int kMinB, bool kStored>
 __global__ void __launch_bounds__(kB, kMinB) k_edges_rev(DevMesh m, double4* sig, double4* ctb, double2* cts, double t,
-                                                         double dtp, const double2* __restrict__ rs,
+                                                         double dtp, const double2* rs,
                                                          const double2* __restrict__ eside)
 {
     chain_begin();
@@ -287,8 +287,8 @@ __global__ void __launch_bounds__(kB, kMinB) k_edges_rev(DevMesh m, double4* sig
         if (kStored) {
             const size_t ni = (size_t)m.ni;
             sl = ld_now(&m.eslot[e]);
-            const double2 r0 = ld_now(rs + e), r1 = ld_now(rs + ni + e), r2 = ld_now(rs + 2 * ni + e);
-            const double2 r3 = ld_now(rs + 3 * ni + e), r4 = ld_now(rs + 4 * ni + e);
+            const double2 r0 = ld_prev_now(rs + e), r1 = ld_prev_now(rs + ni + e), r2 = ld_prev_now(rs + 2 * ni + e);
+            const double2 r3 = ld_prev_now(rs + 3 * ni + e), r4 = ld_prev_now(rs + 4 * ni + e);
             const double2 z = ld_now(eside + e), bb = ld_now(eside + ni + e), ph = ld_now(eside + 2 * ni + e);
             n = ld_now(&m.nxy[e]);
             cf = ld_now(&m.coef[e]);
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_edges_rev(DevMesh m, double4* sig
             n = ld(&m.nxy[e]);
             sl = ld(&m.eslot[e]);
             const double4 ca = ld(&m.cst[a]), cb = ld(&m.cst[b]);
-            const double4 qa = ld(&m.st[a]), qb = ld(&m.st[b]);
+            const double4 qa = ld_prev(&m.st[a]), qb = ld_prev(&m.st[b]);
             if (kScheme == SW2D_SCHEME_GODUNOV) {
                 SL = godunov_side(qa.x, qa.y, qa.z, ca.x, ca.y, n.x, n.y);
                 SR = godunov_side(qb.x, qb.y, qb.z, cb.x, cb.y, n.x, n.y);
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_edges_rev(DevMesh m, double4* sig
     } else if (i < m.ni + m.nb) {
         const int e = i - m.ni;
         const int c = ld(&m.bcell[e]);
-        const double4 s = ld(&m.st[c]);
+        const double4 s = ld_prev(&m.st[c]);
         const double4 cs = ld(&m.cst[c]);
         const double4 g = ld(&m.bgeo[e]);
         const SideState S = godunov_side(s.x, s.y, s.z, cs.x, cs.y, g.x, g.y);
@@ -427,12 +427,6 @@ __global__ void k_slot_geom(DevMesh m, double4* sgeo, int n)
     }
 }
 
-__device__ __forceinline__ double4 ld_now4(const double4* p)
-{
-    const double2 a = ld_now(reinterpret_cast<const double2*>(p)), b = ld_now(reinterpret_cast<const double2*>(p) + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
-}
-
 // One internal slot of k_cells_rev: the reverse of the cell's reconstruction on that slot,
 // added to the cell's sums (skipped when the slot's adjoints are all zero)
 template <bool kMuscl>
@@ -466,8 +460,8 @@ __device__ __forceinline__ void cell_slot_rev(const double4& a, const double2& b
 // first kPre internal slots are loaded together, ahead of the boundary sums; a slot's geometry
 // only when its adjoints are not all zero.
 template <int kScheme>
-__global__ void __launch_bounds__(kBlock) k_cells_rev(DevMesh m, double4* lam, const double4* __restrict__ ctb,
-                                                      const double2* __restrict__ cts, double* gzb, double2* sgb,
+__global__ void __launch_bounds__(kBlock) k_cells_rev(DevMesh m, double4* lam, const double4* ctb,
+                                                      const double2* cts, double* gzb, double2* sgb,
                                                       double dtp, const double4* __restrict__ sgeo)
 {
     chain_begin();
@@ -483,8 +477,8 @@ __global__ void __launch_bounds__(kBlock) k_cells_rev(DevMesh m, double4* lam, c
 #pragma unroll
     for (int i = 0; i < kPre; i++)
         if (i < nint) {
-            A[i] = ld_now4(&ctb[k0 + nbnd + i]);
-            Bv[i] = ld_now(&cts[k0 + nbnd + i]);
+            A[i] = ld_prev_now(&ctb[k0 + nbnd + i]);
+            Bv[i] = ld_prev_now(&cts[k0 + nbnd + i]);
         }
     double hb = 0.0, qb = 0.0, rb = 0.0, zbb = 0.0, sxb = 0.0, syb = 0.0;
     for (int k = k0; k < k0 + nbnd; k++) {

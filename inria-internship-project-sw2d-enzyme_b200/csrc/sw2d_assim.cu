@@ -182,7 +182,7 @@ __device__ __forceinline__ void e_sides(const DevMesh& m, int e, int a, int b, d
         SR = spe::god_side(sb.x, sb.y, sb.z, cb.x, cb.y, n.x, n.y, m.h_min);
     } else {
         const double4 d = ld(&m.emc[e]);
-        const double2 ga = ld(&m.slope[a]), gb = ld(&m.slope[b]);
+        const double2 ga = ld_prev(&m.slope[a]), gb = ld_prev(&m.slope[b]);
         SL = spe::evr_side(true, sa.x, sa.y, sa.z, ca.x, ca.y, sa.w, ga.x, ga.y, d.x, d.y, n.x, n.y, dt);
         SR = spe::evr_side(false, sb.x, sb.y, sb.z, cb.x, cb.y, sb.w, gb.x, gb.y, d.z, d.w, n.x, n.y, dt);
     }
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kBlock) k_e_edges(DevMesh m, EView v)
         const int2 lr = ld(&m.lr[e]);
         const int a = lr.x, b = lr.y;
         const double2 n = ld(&m.nxy[e]);
-        const double4 sa = ld(&m.st[a]), sb = ld(&m.st[b]);
+        const double4 sa = ld_prev(&m.st[a]), sb = ld_prev(&m.st[b]);
         const double4 ca = ld(&m.cst[a]), cb = ld(&m.cst[b]);
         spe::ESide SL, SR;
         e_sides<kScheme>(m, e, a, b, n, sa, sb, ca, cb, (kScheme == SW2D_SCHEME_GODUNOV) ? 0.0 : *v.dtp, SL, SR);
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kBlock) k_e_edges(DevMesh m, EView v)
     } else if (i < m.ni + m.nb) {
         const int e = i - m.ni;
         const int c = ld(&m.bcell[e]);
-        const double4 s = ld(&m.st[c]);
+        const double4 s = ld_prev(&m.st[c]);
         const double4 cs = ld(&m.cst[c]);
         const double4 g = ld(&m.bgeo[e]);
         const spe::ESide S = e_bnd_side<kScheme>(m, s, cs, g.x, g.y);
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, const double* __res
     if (c < m.nc) {
         const int k0 = ld(&m.coff[c].y), k1 = ld(&m.coff[c + 1].y);
         double sw = 0.0;
-        for (int k = k0; k < k1; k++) sw += ld(&m.slot_w[k]);
+        for (int k = k0; k < k1; k++) sw += ld_prev(&m.slot_w[k]);
         const double den = smax(sw, kSmallReal);
         const double x = m.cfl_max * (ld(&m.area[c]) / den);
         if (x < best) best = x;
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, const double* __res
 // hypComputeBalance_E (swSpE_hyp.cpp:336-394) from the cell's slots in the reference's order,
 // then the dry-cell floor, friction and head loss (swSpE_checkpoint.cpp:675-702).
 template <int kFriction, bool kHeadLoss, bool kStore>
-__global__ void __launch_bounds__(kBlock) k_e_update(DevMesh m, const double* __restrict__ dtp, const int* go)
+__global__ void __launch_bounds__(kBlock) k_e_update(DevMesh m, const double* dtp, const int* go)
 {
     chain_begin();
     if (go && !*go) return;
@@ -465,7 +465,7 @@ __global__ void k_e_gauge_rev(const int* __restrict__ ucell, const int* __restri
 }
 
 template <int kFriction, bool kHeadLoss>
-__global__ void __launch_bounds__(kBlock) k_e_update_rev(DevMesh m, const double4* __restrict__ bal, double4* lam,
+__global__ void __launch_bounds__(kBlock) k_e_update_rev(DevMesh m, const double4* bal, double4* lam,
                                                          double4* lamb, double* gk1, double* gk2, double dt)
 {
     chain_begin();
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kBlock) k_e_update_rev(DevMesh m, const double
 // (coef = w / area / phi), then the reverse of the flux and of both Riemann states.  Each side's
 // contribution goes to its slot: ctb = {h, q, r, phi} adjoints of that cell, cts = its slope's.
 template <int kScheme>
-__global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, const double4* __restrict__ lamb,
+__global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, const double4* lamb,
                                                         double4* ctb, double2* cts, double dt, int ieee)
 {
     chain_begin();
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
         const int e = i;
         const int2 lr = ld(&m.lr[e]);
         const int a = lr.x, b = lr.y;
-        const double4 lL = ld(&lamb[a]), lR = ld(&lamb[b]);
+        const double4 lL = ld_prev(&lamb[a]), lR = ld_prev(&lamb[b]);
         const int2 sl = ld(&m.eslot[e]);
         if (lL.x == 0.0 && lL.y == 0.0 && lL.z == 0.0 && lR.x == 0.0 && lR.y == 0.0 && lR.z == 0.0) {
             // neither cell has an adjoint: the edge passes none on
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
             return;
         }
         const double2 n = ld(&m.nxy[e]);
-        const double4 sa = ld(&m.st[a]), sb = ld(&m.st[b]);
+        const double4 sa = ld_prev(&m.st[a]), sb = ld_prev(&m.st[b]);
         const double4 ca = ld(&m.cst[a]), cb = ld(&m.cst[b]);
         spe::ESide SL, SR;
         e_sides<kScheme>(m, e, a, b, n, sa, sb, ca, cb, dt, SL, SR);
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
             ctb[sl.y] = make_double4(hb, qb, rb, pRb);
         } else {
             const double4 d = ld(&m.emc[e]);
-            const double2 ga = ld(&m.slope[a]), gb = ld(&m.slope[b]);
+            const double2 ga = ld_prev(&m.slope[a]), gb = ld_prev(&m.slope[b]);
             double zcb = 0, sxb = 0, syb = 0;
             spe::evr_side_rev(true, sa.x, sa.y, sa.z, ca.x, ca.y, sa.w, ga.x, ga.y, d.x, d.y, nx, ny, dt, Lb, hb, qb, rb,
                               zcb, sxb, syb, ieee);
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
     } else if (i < m.ni + m.nb) {
         const int e = i - m.ni;
         const int c = ld(&m.bcell[e]);
-        const double4 s = ld(&m.st[c]);
+        const double4 s = ld_prev(&m.st[c]);
         const double4 cs = ld(&m.cst[c]);
         const double4 g = ld(&m.bgeo[e]);
         const spe::ESide S = e_bnd_side<kScheme>(m, s, cs, g.x, g.y);
@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
         const double bcv = e_bc_value(m, e, *v.tp, &type);
         const double phi = ld(&v.phi[c]);
         const spe::EBndFlux F = spe::boundary_flux(cs.y, phi, cs.x, S, type, bcv, m.h_min, m.phi_min);
-        const double4 l = ld(&lamb[c]);
+        const double4 l = ld_prev(&lamb[c]);
         const double cf = ld(&v.coefb[e]), nx = g.x, ny = g.y;
         const double f1b = cf * dt * l.x;
         const double f2b = dt * cf * (nx * l.y + ny * l.z);
@@ -607,8 +607,8 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
 
 // ordered gather of the slot contributions of each cell
 template <bool kMuscl>
-__global__ void __launch_bounds__(kBlock) k_e_cells_rev(DevMesh m, double4* lam, const double4* __restrict__ ctb,
-                                                        const double2* __restrict__ cts, double* gphi, double2* sgb)
+__global__ void __launch_bounds__(kBlock) k_e_cells_rev(DevMesh m, double4* lam, const double4* ctb,
+                                                        const double2* cts, double* gphi, double2* sgb)
 {
     chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -617,13 +617,13 @@ __global__ void __launch_bounds__(kBlock) k_e_cells_rev(DevMesh m, double4* lam,
     double4 l = lam[c];
     double gp = 0.0, sx = 0.0, sy = 0.0;
     for (int k = k0; k < k1; k++) {
-        const double4 v = ld(&ctb[k]);
+        const double4 v = ld_prev(&ctb[k]);
         l.x += v.x;
         l.y += v.y;
         l.z += v.z;
         gp += v.w;
         if (kMuscl) {
-            const double2 s = ld(&cts[k]);
+            const double2 s = ld_prev(&cts[k]);
             sx += s.x;
             sy += s.y;
         }

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_ddp_edges(DevMesh m)
         const double len_e = ld(&m.len[e]);
         const int ao = ld_now(&m.ctoff[a]), an = ld_now(&m.ctoff[a + 1]) - ao;
         const int bo = ld_now(&m.ctoff[b]), bn = ld_now(&m.ctoff[b + 1]) - bo;
-        const double4 sa = ld(&m.st[a]), sb = ld(&m.st[b]);   // {theta, theta u, theta v, z}
+        const double4 sa = ld_prev(&m.st[a]), sb = ld_prev(&m.st[b]);   // {theta, theta u, theta v, z}
         const double2 va = ld(reinterpret_cast<const double2*>(&m.dv[a]));  // {phiW, thetaW} at z
         const double2 vb = ld(reinterpret_cast<const double2*>(&m.dv[b]));
         const double2 ca = ld(reinterpret_cast<const double2*>(&m.cst[a]));  // {z_b, boussinesq}
@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(kB, kMinB) k_ddp_edges(DevMesh m)
             in.gamma_R = gs[1];
             in.theta_RL = ddp::phi_theta(m.ctab + bo, bn, sa.w, bad).theta;
             in.theta_LR = ddp::phi_theta(m.ctab + ao, an, sb.w, bad).theta;
-            in.force_omega_L = ld(&m.dv[a].z);
-            in.force_omega_R = ld(&m.dv[b].z);
+            in.force_omega_L = ld_prev(&m.dv[a].z);
+            in.force_omega_R = ld_prev(&m.dv[b].z);
             in.force_gamma_L = fg[0];
             in.force_gamma_R = fg[1];
             const double2 e0 = ld(reinterpret_cast<const double2*>(&m.des[2 * e]));
@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(kB, kMinB) k_ddp_edges(DevMesh m)
     } else if (i < m.ni + m.nb) {
         const int e = i - m.ni;
         const int c = ld(&m.bcell[e]);
-        const double4 s = ld(&m.st[c]);
-        const double4 v = ld(&m.dv[c]);
+        const double4 s = ld_prev(&m.st[c]);
+        const double4 v = ld_prev(&m.dv[c]);
         const double4 cs = ld(&m.cst[c]);
         const double4 g = ld(&m.bgeo[e]);  // {nx, ny, length, w / area}
         const double theta_in = s.x, z_in = s.w;

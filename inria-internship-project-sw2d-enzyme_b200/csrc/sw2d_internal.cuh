@@ -230,7 +230,30 @@ __device__ __forceinline__ double ld_now(const double* p)
 // as programmatic dependents (launch_chained): a kernel's blocks may be placed while the previous
 // kernel's last ones run.  Each begins with chain_begin, which waits until the previous kernel has
 // finished and its writes are visible, then lets the next one be placed; nothing is read or written
-// before it.
+// before it.  A kernel's lifetime so overlaps the previous one's, and only that one's: what the
+// previous kernel may write is read on the coherent path (ld_prev), never on the read-only path.
+template <class T>
+__device__ __forceinline__ T ld_prev(const T* p) { return *p; }
+// the same, issued where it stands (as ld_now)
+__device__ __forceinline__ double2 ld_prev_now(const double2* p)
+{
+    double2 v;
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double4 ld_prev_now(const double4* p)
+{
+    const double2* q = reinterpret_cast<const double2*>(p);
+    const double2 a = ld_prev_now(q), b = ld_prev_now(q + 1);
+    return make_double4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ double ld_prev_now(const double* p)
+{
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ void chain_begin()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

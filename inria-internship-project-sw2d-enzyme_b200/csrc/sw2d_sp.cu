@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kB, kMinB) k_slopes(DevMesh m)
     if (!step_active(m.ctrl)) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
-    slopes_cell<LdNc>(m, c);
+    slopes_cell<LdCo>(m, c);
 }
 
 // k_edges: one thread per internal edge, then one per boundary edge (edge_internal and
@@ -74,8 +74,8 @@ __global__ void __launch_bounds__(kB, kMinB) k_edges(DevMesh m)
     if (!step_active(m.ctrl)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned bad = 0;
-    if (i < m.ni) bad = edge_internal<kScheme, kBlending, kModel, LdNc>(m, i);
-    else if (i < m.ni + m.nb) bad = edge_boundary<kScheme, kModel, LdNc>(m, i - m.ni);
+    if (i < m.ni) bad = edge_internal<kScheme, kBlending, kModel, LdCo>(m, i);
+    else if (i < m.ni + m.nb) bad = edge_boundary<kScheme, kModel, LdCo>(m, i - m.ni);
     if (bad) atomicOr(&m.ctrl->status, bad);
 }
 
@@ -87,21 +87,23 @@ __global__ void __launch_bounds__(kB, kMinB) k_edges(DevMesh m)
 // +0 to the (non-negative) sum changes no bit, so the sum is the reference's.
 // ------------------------------------------------------------------------------------------
 
-// k_cfl's grid: 8 blocks of kBlock threads per SM (a full SM), at most one block per kBlock cells
-unsigned cfl_grid(sw2d_handle* h, int nc)
+int sm_count(sw2d_handle* h)
 {
     if (!h->sms) {
         int sms = 0;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess || sms <= 0) sms = 148;
         h->sms = sms;
     }
-    return std::min<unsigned>(grid_for(nc), (unsigned)(8 * h->sms));
+    return h->sms;
 }
+
+// k_cfl's grid: 8 blocks of kBlock threads per SM (a full SM), at most one block per kBlock cells
+unsigned cfl_grid(sw2d_handle* h, int nc) { return std::min<unsigned>(grid_for(nc), (unsigned)(8 * sm_count(h))); }
 
 // kDdpSnap: the DDP model's form of the snap, which truncates t and t + dt to integers before
 // dividing by dt_map (swDdpHyp.cpp:588-600: `(int)t / dt_map`).
 template <bool kDdpSnap>
-__global__ void __launch_bounds__(kBlock) k_cfl(DevMesh m)
+__global__ void __launch_bounds__(kBlock, 8) k_cfl(DevMesh m)
 {
     chain_begin();
     Ctrl* ctrl = m.ctrl;
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(kBlock) k_cfl(DevMesh m)
     const int stride = gridDim.x * blockDim.x;
 #pragma unroll 4
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m.nc; c += stride) {
-        const double x = cfl_cell<LdNc>(m, c);
+        const double x = cfl_cell<LdCo>(m, c);
         if (x < best) best = x;
     }
     // warp then block minimum (NaN candidates never win: comparisons with NaN are false)
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_update(DevMesh m)
         }
     }
     if (c >= m.nc) return;
-    update_cell<kFriction, kHeadLoss, kStoreB, kDissip, LdNc>(m, c, dt);
+    update_cell<kFriction, kHeadLoss, kStoreB, kDissip, LdCo>(m, c, dt);
 }
 
 // swSp::computeEdgeFactors coefficient w / area / phi (swSp.cpp:364-368, 397-405)
