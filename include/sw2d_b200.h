@@ -450,6 +450,14 @@ const char* sw2d_phase_name(int i);
  * they are (still counted by sw2d_adjoint_nonfinite) instead of zeroing them, to locate them.
  * "adjoint_store_states" (0/1, default 1): the segment recompute keeps each step's slopes and
  * Riemann states for the reverse steps when they fit in half of the free device memory.
+ * "adjoint_kept_segments" (at least 1): sw2d_adjoint on a trajectory whose checkpoints a change of
+ * the parameters has outdated runs it first, and keeps the steps of its last segments meanwhile
+ * instead of recomputing them: this many at most, and what an eighth of the free device memory
+ * holds (the default).  The same bits either way.  Takes effect at the next sw2d_record.
+ * "run_kernel" (0/1, default 1): sw2d_step_n and sw2d_execute take the steps of a small SP or DIP
+ * mesh (one whose cells fit the chip's shared memory) in one launch; 0 takes them kernel by kernel.
+ * "run_wait_polls": the poll limit of that launch's waits, after which it gives up with an error
+ * status (negative: the default).
  * "adjoint_trace" (0/1): record the state adjoint's magnitude per reverse step
  * (sw2d_adjoint_trace). */
 int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value);

@@ -65,11 +65,15 @@ struct AdjointState {
     Slot* ck_slot = nullptr;             // (n_ck + 1) * nslot
     Ctrl* ck_ctrl = nullptr;             // n_ck + 1
     bool ck_valid = false;
-    // one segment of recomputed steps
+    // the steps of n_seg segments: buffer 0 for the recomputed ones, all of them for the last n_seg
+    // segments when a gradient runs the trajectory itself (per buffer:)
+    int64_t n_seg = 1;
     double4* seg_st = nullptr;           // (every + 1) * nc
     double4* seg_bal = nullptr;          // every * nc
     double2* seg_slope = nullptr;        // every * nc: each step's MUSCL-EVR slopes
     double2* seg_rs = nullptr;           // every * ni * 5: each step's Riemann states (when memory allows)
+    double4 *more_st = nullptr, *more_bal = nullptr;  // the buffers after the first
+    double2 *more_slope = nullptr, *more_rs = nullptr;
     double2* eside = nullptr;            // 3 * ni: {z_b}, {b}, {phi} of each internal edge's (L, R) cells
     // adjoint buffers
     double4* lam = nullptr;              // nc: adjoint of the state {h, q, r, -}
@@ -641,17 +645,17 @@ int obs_index(const AdjointState* a, int64_t step)
     return a->obs_at[step];
 }
 
-// Forward over the recorded trajectory from checkpoint 0 with the recorded dt (replay) or the
-// CFL dt (record), storing checkpoints; `at_step(j)` is called with the state after j steps
-// (j = 0 .. n_steps) in the model's state buffer.
+// Forward over the first j_end steps of the recorded trajectory from checkpoint 0 with the recorded
+// dt (replay) or the CFL dt (record), storing checkpoints; `at_step(j)` is called with the state
+// after j steps (j = 0 .. j_end) in the model's state buffer.
 template <class F>
-int run_trajectory(sw2d_handle* h, bool record, F&& at_step)
+int run_steps(sw2d_handle* h, bool record, int64_t j_end, F&& at_step)
 {
     AdjointState* a = h->adj;
     int rc = ck_load(h, 0);
     if (rc) return rc;
     at_step(0);
-    for (int64_t j = 0; j < a->n_steps; j++) {
+    for (int64_t j = 0; j < j_end; j++) {
         if (j % a->every == 0 && j > 0 && (rc = ck_save(h, j / a->every))) return rc;
         launch_slopes_on(h, h->m);
         launch_edges_on(h, h->m);
@@ -664,7 +668,15 @@ int run_trajectory(sw2d_handle* h, bool record, F&& at_step)
         launch_update_on(h, mu, false);
         at_step(j + 1);
     }
-    if ((rc = ck_save(h, a->n_ck))) return rc;
+    return SW2D_OK;
+}
+
+// the whole trajectory, with the checkpoint at its end
+template <class F>
+int run_trajectory(sw2d_handle* h, bool record, F&& at_step)
+{
+    int rc = run_steps(h, record, h->adj->n_steps, at_step);
+    if (rc || (rc = ck_save(h, h->adj->n_ck))) return rc;
     CK(cudaGetLastError());
     return SW2D_OK;
 }
@@ -798,9 +810,84 @@ int check_observations(sw2d_handle* h)
     return SW2D_OK;
 }
 
-// Reverse sweep over the segments (checkpoints must be valid).  Leaves the gradients in lam,
-// g_zb, g_k1, g_k2, the per-observation costs in d_Jobs, and the model at the trajectory's end.
-int reverse_sweep(sw2d_handle* h)
+// One segment's buffer of kept steps: step j of the segment [j0, ..) reads st(j) and writes st(j + 1)
+struct SegmentBuffer {
+    double4 *st_, *bal_;
+    double2 *slope_, *rs_;
+    int64_t j0, nc, ni;
+    double4* st(int64_t j) const { return st_ + (j - j0) * nc; }
+    double4* bal(int64_t j) const { return bal_ + (j - j0) * nc; }
+    double2* slope(int64_t j) const { return slope_ ? slope_ + (j - j0) * nc : nullptr; }
+    double2* rs(int64_t j) const { return rs_ ? rs_ + (j - j0) * 5 * ni : nullptr; }
+};
+
+// buffer of segment s: one of its own for the trajectory's last n_seg segments, else the first one,
+// which the reverse sweep is then done with
+SegmentBuffer segment_buffer(const sw2d_handle* h, int64_t s)
+{
+    const AdjointState* a = h->adj;
+    const int64_t seg = std::min(a->every, a->n_requested), k = s - (a->n_ck - a->n_seg) - 1;
+    if (k < 0) return {a->seg_st, a->seg_bal, a->seg_slope, a->seg_rs, s * a->every, h->nc, h->ni};
+    return {a->more_st + k * (seg + 1) * h->nc,
+            a->more_bal + k * seg * h->nc,
+            a->more_slope ? a->more_slope + k * seg * h->nc : nullptr,
+            a->more_rs + k * seg * 5 * h->ni,
+            s * a->every,
+            h->nc,
+            h->ni};
+}
+
+// The steps of segment s from the model's state with the recorded dt, keeping each step's state and
+// post-balance state (and slopes and Riemann states), with the costs of the observations they end
+// on.  dt is frozen, so the CFL contributions are not written.
+int run_segment(sw2d_handle* h, int64_t s)
+{
+    AdjointState* a = h->adj;
+    const SegmentBuffer b = segment_buffer(h, s);
+    const int64_t j1 = std::min(a->n_steps, b.j0 + a->every);
+    CK(cudaMemcpyAsync(b.st(b.j0), h->m.st, h->nc * sizeof(double4), cudaMemcpyDeviceToDevice, h->stream));
+    for (int64_t j = b.j0; j < j1; j++) {
+        DevMesh mj = h->m;
+        mj.st = b.st(j);
+        mj.st_out = b.st(j + 1);
+        mj.slot_w = nullptr;
+        mj.bal = b.bal(j);
+        if (b.slope_) mj.slope = b.slope(j);
+        mj.rstate = b.rs(j);
+        launch_slopes_on(h, mj);
+        launch_edges_on(h, mj);
+        mj.dt_fixed = a->d_dt_seq + j;
+        launch_update_on(h, mj, true);
+        const int k = obs_index(a, j + 1);
+        if (k >= 0) cost_at(h, k, mj.st_out);
+    }
+    return SW2D_OK;
+}
+
+// The trajectory's replay at the head of a gradient: the checkpoints, and the steps of the last n_seg
+// segments kept as run_segment keeps them, so that the reverse sweep need not recompute those.
+// 100 steps of 100k cells, all kept: 11.5 -> 8.9 ms per gradient.
+int run_keeping(sw2d_handle* h)
+{
+    AdjointState* a = h->adj;
+    const int64_t s0 = std::max<int64_t>(0, a->n_ck - a->n_seg);
+    int rc = run_steps(h, false, s0 * a->every, [](int64_t) {});
+    if (rc) return rc;
+    for (int64_t s = s0; s < a->n_ck; s++) {
+        if (s > 0 && (rc = ck_save(h, s))) return rc;
+        if ((rc = run_segment(h, s))) return rc;
+        const double4* end = segment_buffer(h, s).st(std::min(a->n_steps, (s + 1) * a->every));
+        CK(cudaMemcpyAsync(h->m.st, end, h->nc * sizeof(double4), cudaMemcpyDeviceToDevice, h->stream));
+    }
+    if ((rc = ck_save(h, a->n_ck))) return rc;
+    CK(cudaGetLastError());
+    return SW2D_OK;
+}
+
+// Reverse sweep over the segments (checkpoints must be valid; the last `kept` segments' steps are in
+// their buffers, run_keeping).  Leaves the gradients in lam, g_zb, g_k1, g_k2, the per-observation
+// costs in d_Jobs, and the model at the trajectory's end.
+int reverse_sweep(sw2d_handle* h, int64_t kept)
 {
     AdjointState* a = h->adj;
     const int64_t nc = h->nc;
@@ -830,38 +917,20 @@ int reverse_sweep(sw2d_handle* h)
     }
     for (int64_t s = a->n_ck - 1; s >= 0; s--) {
         const int64_t j0 = s * a->every, j1 = std::min(a->n_steps, j0 + a->every);
-        if ((rc = ck_load(h, s))) return rc;
-        // recompute the segment, keeping each step's state and post-balance state: step j reads
-        // seg_st[j - j0] and writes seg_st[j + 1 - j0]; its dt is frozen, so the CFL
-        // contributions are not written
-        CK(cudaMemcpyAsync(a->seg_st, h->m.st, nc * sizeof(double4), cudaMemcpyDeviceToDevice, h->stream));
-        for (int64_t j = j0; j < j1; j++) {
-            DevMesh mj = h->m;
-            mj.st = a->seg_st + (j - j0) * nc;
-            mj.st_out = a->seg_st + (j + 1 - j0) * nc;
-            mj.slot_w = nullptr;
-            mj.bal = a->seg_bal + (j - j0) * nc;
-            if (a->seg_slope) mj.slope = a->seg_slope + (j - j0) * nc;
-            if (a->seg_rs) mj.rstate = a->seg_rs + (j - j0) * 5 * h->ni;
-            launch_slopes_on(h, mj);
-            launch_edges_on(h, mj);
-            mj.dt_fixed = a->d_dt_seq + j;
-            launch_update_on(h, mj, true);
-            const int k = obs_index(a, j + 1);
-            if (k >= 0) cost_at(h, k, mj.st_out);
-        }
+        const SegmentBuffer b = segment_buffer(h, s);
+        if (s < a->n_ck - kept && ((rc = ck_load(h, s)) || (rc = run_segment(h, s)))) return rc;
         // reverse steps
         for (int64_t j = j1 - 1; j >= j0; j--) {
             const int k = obs_index(a, j + 1);
             if (k >= 0 && a->n_pts > 0)
-                k_obs_rev<<<grid_for(a->n_pts), kBlock, 0, h->stream>>>(obs_view(a, k), a->seg_st + (j + 1 - j0) * nc,
+                k_obs_rev<<<grid_for(a->n_pts), kBlock, 0, h->stream>>>(obs_view(a, k), b.st(j + 1),
                                                                         a->lam);
-            launch_update_rev(h, a->seg_bal + (j - j0) * nc, a->dt_seq[j]);
+            launch_update_rev(h, b.bal(j), a->dt_seq[j]);
             DevMesh mr = h->m;
-            mr.st = a->seg_st + (j - j0) * nc;
+            mr.st = b.st(j);
             if (muscl) {
-                if (a->seg_slope) {
-                    mr.slope = a->seg_slope + (j - j0) * nc;  // kept by the segment's recompute
+                if (b.slope_) {
+                    mr.slope = b.slope(j);  // kept with the segment's steps
                 } else {
                     DevMesh ms = mr;
                     ms.ctrl = a->ctrl_rev;  // always active: recompute the slopes of step j
@@ -869,7 +938,7 @@ int reverse_sweep(sw2d_handle* h)
                 }
             }
             launch_edges_rev(h, mr, a->t_seq[j], j > 0 ? a->dt_seq[j - 1] : a->dt_before,
-                             a->seg_rs ? a->seg_rs + (j - j0) * 5 * h->ni : nullptr);
+                             b.rs(j));
             const double dtp = j > 0 ? a->dt_seq[j - 1] : a->dt_before;
             if (muscl) {
                 launch_chained(k_cells_rev<SW2D_SCHEME_MUSCL_EVR>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_zb,
@@ -902,6 +971,30 @@ int reverse_sweep(sw2d_handle* h)
     return SW2D_OK;
 }
 
+// Buffers for more of the trajectory's last segments (each costs what the first one does): as many
+// as an eighth of the free device memory holds
+void more_segments(sw2d_handle* h, int64_t seg)
+{
+    AdjointState* a = h->adj;
+    const int64_t nc = h->nc;
+    size_t free_b = 0, total_b = 0;
+    if (!a->seg_rs || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return;
+    const size_t one = (size_t)(2 * seg + 1) * nc * sizeof(double4) +
+                       (size_t)seg * ((a->seg_slope ? nc : 0) + 5 * h->ni) * sizeof(double2);
+    const int64_t n = std::min({a->n_ck - 1, (int64_t)(free_b / 8 / one), h->adj_kept_segments - 1});
+    if (n <= 0) return;
+    std::vector<void*> L;
+    if (adj_alloc(h, L, n * (seg + 1) * nc, &a->more_st) || adj_alloc(h, L, n * seg * nc, &a->more_bal) ||
+        (a->seg_slope && adj_alloc(h, L, n * seg * nc, &a->more_slope)) ||
+        adj_alloc(h, L, n * seg * h->ni * 5, &a->more_rs)) {
+        free_list(L);
+        h->err.clear();
+        return;
+    }
+    a->traj_allocs.insert(a->traj_allocs.end(), L.begin(), L.end());
+    a->n_seg = 1 + n;
+}
+
 int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
 {
     AdjointState* a = h->adj;
@@ -911,6 +1004,8 @@ int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
     a->n_steps = n_steps;
     a->every = every;
     a->n_ck = (n_steps + every - 1) / every;
+    a->n_seg = 1;
+    a->more_slope = nullptr;
     const int64_t nc = h->nc, seg = std::min(every, n_steps);
     auto& L = a->traj_allocs;
     int rc = SW2D_OK;
@@ -941,6 +1036,7 @@ int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
             h->err.clear();
         }
     }
+    more_segments(h, seg);
     a->n_requested = n_steps;
     return SW2D_OK;
 }
@@ -1275,12 +1371,14 @@ int sw2d_adjoint(sw2d_handle* h, double* J, const sw2d_gradient* grad)
     CK(cudaSetDevice(h->device));
     AdjointState* a = h->adj;
     if ((rc = check_observations(h))) return rc;
+    int64_t kept = 0;
     if (!a->ck_valid) {
-        if ((rc = run_trajectory(h, false))) return rc;
+        if ((rc = run_keeping(h))) return rc;
         if ((rc = read_status(h))) return rc;
         a->ck_valid = true;
+        kept = a->n_seg;
     }
-    if ((rc = reverse_sweep(h))) return rc;
+    if ((rc = reverse_sweep(h, kept))) return rc;
     if ((rc = read_status(h))) return rc;
     if ((rc = total_cost(h, J))) return rc;
     if (grad) {

@@ -319,6 +319,7 @@ struct sw2d_handle {
     int adj_keep_nonfinite = 0;         // option "adjoint_keep_nonfinite"
     int adj_trace = 0;                  // option "adjoint_trace"
     int adj_store_states = 1;           // option "adjoint_store_states"
+    int64_t adj_kept_segments = INT32_MAX;  // option "adjoint_kept_segments"
     void* saved_point = nullptr;        // sw2d_save_point: state, balance slots, control block
     int adj_edge_variant = 0;           // option "adjoint_edge_variant"
     sw2d::AssimState* assim = nullptr;  // porosity assimilation with the differentiated step

@@ -1440,6 +1440,13 @@ int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value)
         // the reverse steps rebuild them (the same bits).  Takes effect at the next sw2d_record.
         h->adj_store_states = value ? 1 : 0;
         return SW2D_OK;
+    } else if (std::strcmp(name, "adjoint_kept_segments") == 0) {
+        // how many of the last segments a gradient that has to run the trajectory itself may keep
+        // while it does (at least 1; default: what an eighth of the free device memory holds).
+        // Takes effect at the next sw2d_record.
+        if (value < 1) return fail(h, SW2D_E_ARG, "adjoint_kept_segments must be at least 1");
+        h->adj_kept_segments = value;
+        return SW2D_OK;
     } else if (std::strcmp(name, "adjoint_trace") == 0) {
         // 1: sw2d_adjoint records, after each reverse step, the non-finite entries and the largest
         // magnitudes of the state adjoint (sw2d_adjoint_trace)
