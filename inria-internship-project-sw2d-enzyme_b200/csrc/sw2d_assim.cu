@@ -23,7 +23,6 @@
 //   k_e_cfl               (record) per cell swept sums -> grid minimum -> dt, t_max clip, 1e-6
 //                         floor, observation snap
 //   k_e_update            per cell: ordered gather of its slots, flush, clamp, friction, head loss
-//   k_e_advance           (record) dt, t and trigger of the step; t += dt
 // Reverse of one step:
 //   k_obs_rev / k_e_gauge_rev   misfit gradient when the step ends on an observation
 //   k_e_update_rev        per cell: reverse of the update -> adjoint of the raw post-balance state
@@ -92,6 +91,7 @@ struct AssimState {
     int* d_trig = nullptr;
     std::vector<double4*> ck;        // state at the start of each segment
     std::vector<double4*> cs;        // the same states along the replay (option assim_chained_recompute)
+    std::vector<double4*> ck_spare;  // those of the record before, for the next one to take
     bool recorded = false;
     // window (get_spatial_gradient_checkpointed)
     int64_t first = 0, truncation = -1;
@@ -104,6 +104,7 @@ struct AssimState {
     int64_t nslot = 0, ncint = 0, seg_cap = 0;
     double4* seg_st = nullptr;       // (seg_cap + 1) * nc
     double4* seg_bal = nullptr;      // seg_cap * nc
+    double2* seg_slope = nullptr;    // seg_cap * nc: each step's slopes (MUSCL-EVR, when memory allows)
     double4 *lam = nullptr, *lamb = nullptr, *ctb = nullptr;
     double2 *cts = nullptr, *sgb = nullptr;
     double *znb = nullptr, *gzb = nullptr;
@@ -279,10 +280,44 @@ __global__ void __launch_bounds__(kBlock) k_e_edges(DevMesh m, EView v)
 
 __device__ __forceinline__ double e_min_keep(double a, double b) { return (b < a) ? b : a; }
 
+// The recorded sequence and the next observation to come
+struct ERecord {
+    const double* obs_t;
+    int n_obs;
+    int* obs_idx;
+    double *dt_seq, *t_seq;
+    int* trig;
+    long long cap;
+};
+
+// The step's bookkeeping in build_checkpoint_records (swSpE_checkpoint.cpp:315-377): keep dt and
+// t of the step, t += dt, pass observations already overtaken, trigger the one landed on.  The
+// update, which follows, reads only dt and go of the control block.
+__device__ __forceinline__ void e_advance(Ctrl* ctrl, const ERecord& r, double dt)
+{
+    const long long j = ctrl->steps;
+    const double t0 = ctrl->t;
+    const double t = t0 + dt;
+    int k = *r.obs_idx;
+    while (k < r.n_obs && t > r.obs_t[k] + 1e-6) k++;
+    int tr = -1;
+    if (k < r.n_obs && fabs(t - r.obs_t[k]) < 1e-6) {
+        tr = k;
+        k++;
+    }
+    if (j < r.cap) {
+        r.dt_seq[j] = dt;
+        r.t_seq[j] = t0;
+        r.trig[j] = tr;
+    }
+    *r.obs_idx = k;
+    ctrl->t = t;
+    ctrl->steps = j + 1;
+}
+
 // hypComputeTimeStep_E (assim/swSpE_hyp.cpp:578-638) and the observation snap of
-// build_checkpoint_records (swSpE_checkpoint.cpp:228-250), on the device.
-__global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, const double* __restrict__ obs_t, const int* obs_idx,
-                                                  int n_obs)
+// build_checkpoint_records (swSpE_checkpoint.cpp:228-250), on the device, and the step's bookkeeping.
+__global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, ERecord rec)
 {
     chain_begin();
     Ctrl* ctrl = m.ctrl;
@@ -332,9 +367,9 @@ __global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, const double* __res
         if ((t + dt) > t_max) dt = t_max - t;
         if (dt < spe::kDtFloor) dt = spe::kDtFloor;
         double dt_target = m.dt_max;
-        const int k = *obs_idx;
-        if (k < n_obs) {
-            const double to = obs_t[k] - t;
+        const int k = *rec.obs_idx;
+        if (k < rec.n_obs) {
+            const double to = rec.obs_t[k] - t;
             if (to - 10e-6 > 0.0 && to < dt_target) dt_target = to;
         }
         double cur = (dt < dt_target) ? dt : dt_target;
@@ -343,6 +378,7 @@ __global__ void __launch_bounds__(kBlock) k_e_cfl(DevMesh m, const double* __res
         ctrl->dt = cur;
         ctrl->go = 1;
         ctrl->blocks_done = 0;
+        e_advance(ctrl, rec, cur);
     }
 }
 
@@ -402,34 +438,6 @@ __global__ void __launch_bounds__(kBlock) k_e_update(DevMesh m, const double* dt
     }
     spe::cell_update(hh, qq, rr, p, dt);
     m.st[c] = make_double4(hh, qq, rr, hh + ld(&m.zbv[c]));
-}
-
-// The step's bookkeeping in build_checkpoint_records (swSpE_checkpoint.cpp:315-377): keep dt and
-// t of the step, t += dt, pass observations already overtaken, trigger the one landed on.
-__global__ void k_e_advance(Ctrl* ctrl, int* obs_idx, const double* __restrict__ obs_t, int n_obs, double* dt_seq,
-                            double* t_seq, int* trig, long long cap)
-{
-    chain_begin();
-    if (!ctrl->go) return;
-    const long long j = ctrl->steps;
-    const double t0 = ctrl->t, dt = ctrl->dt;
-    const double t = t0 + dt;
-    int k = *obs_idx;
-    while (k < n_obs && t > obs_t[k] + 1e-6) k++;
-    int tr = -1;
-    if (k < n_obs && fabs(t - obs_t[k]) < 1e-6) {
-        tr = k;
-        k++;
-    }
-    if (j < cap) {
-        dt_seq[j] = dt;
-        t_seq[j] = t0;
-        trig[j] = tr;
-    }
-    *obs_idx = k;
-    ctrl->t = t;
-    ctrl->steps = j + 1;
-    ctrl->go = 0;
 }
 
 // the cost of an observation: per-block partials (fixed tree), then one thread adds them in
@@ -905,12 +913,33 @@ int ensure_steps(sw2d_handle* h, int64_t need)
     return SW2D_OK;
 }
 
-void free_checkpoints(AssimState* a)
+// The checkpoints of a record serve the next one: an assimilation records again at each iterate, and
+// allocating and freeing 5 of them each time took 0.9 ms of a record of 10k cells and 134 steps, more
+// where other processes of the machine kept the driver busy.
+void spare_checkpoints(AssimState* a)
 {
-    for (double4* p : a->ck) cudaFree(p);
+    a->ck_spare.insert(a->ck_spare.end(), a->ck.begin(), a->ck.end());
     a->ck.clear();
-    for (double4* p : a->cs) cudaFree(p);
+    a->ck_spare.insert(a->ck_spare.end(), a->cs.begin(), a->cs.end());
     a->cs.clear();
+}
+
+void free_spares(AssimState* a)
+{
+    for (double4* p : a->ck_spare) cudaFree(p);
+    a->ck_spare.clear();
+}
+
+int take_checkpoint(sw2d_handle* h, double4** out)
+{
+    AssimState* a = h->assim;
+    if (!a->ck_spare.empty()) {
+        *out = a->ck_spare.back();
+        a->ck_spare.pop_back();
+        return SW2D_OK;
+    }
+    CK(cudaMalloc(out, std::max<int64_t>(1, h->nc) * sizeof(double4)));
+    return SW2D_OK;
 }
 
 
@@ -964,7 +993,7 @@ int record(sw2d_handle* h, int64_t stride)
 {
     AssimState* a = h->assim;
     const int64_t nc = h->nc;
-    free_checkpoints(a);
+    spare_checkpoints(a);
     a->segs.clear();
     a->recorded = false;
     a->stride = stride;
@@ -985,24 +1014,23 @@ int record(sw2d_handle* h, int64_t stride)
     while (t_host < h->p.t_max) {
         int rc = ensure_steps(h, done + stride);
         if (rc) return rc;
+        const ERecord rec{a->d_obs_t, (int)a->n_obs, a->d_obs_idx, a->d_dt, a->d_t, a->d_trig, (long long)a->cap};
         double4* ck = nullptr;
-        CK(cudaMalloc(&ck, std::max<int64_t>(1, nc) * sizeof(double4)));
+        if ((rc = take_checkpoint(h, &ck))) return rc;
         a->ck.push_back(ck);
         CK(cudaMemcpyAsync(ck, h->m.st, nc * sizeof(double4), cudaMemcpyDeviceToDevice, h->stream));
         for (int64_t j = 0; j < stride; j++) {
             if (muscl) launch_slopes_on(h, m);
             launch_edges<true>(h, m, v);
-            if (gc > 0) launch_chained(k_e_cfl, gc, kBlock, 0, h->stream, m, a->d_obs_t, a->d_obs_idx, (int)a->n_obs);
+            if (gc > 0) launch_chained(k_e_cfl, gc, kBlock, 0, h->stream, m, rec);
             launch_update(h, m, &a->ctrl->dt, &a->ctrl->go, false);
-            launch_chained(k_e_advance, 1, 1, 0, h->stream, a->ctrl, a->d_obs_idx, a->d_obs_t, (int)a->n_obs, a->d_dt, a->d_t,
-                                                 a->d_trig, (long long)a->cap);
         }
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(&ch, a->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
         const int64_t n = ch.steps - done;
         if (n <= 0) {
-            cudaFree(a->ck.back());
+            a->ck_spare.push_back(a->ck.back());
             a->ck.pop_back();
             break;
         }
@@ -1025,18 +1053,20 @@ int record(sw2d_handle* h, int64_t stride)
         CK(cudaMemcpyAsync(a->trig.data(), a->d_trig, done * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
     }
+    free_spares(a);  // what this record no longer needs
     compute_window(a, h->p.t_max);
     a->recorded = true;
     return SW2D_OK;
 }
 
 // One replayed step j of ckpt_segment_E on the handle's state (dt and boundary time frozen);
-// with bal, the raw post-balance state is kept there.
-void replay_step(sw2d_handle* h, int64_t j, double4* bal)
+// with bal, the raw post-balance state is kept there, with slope the slopes.
+void replay_step(sw2d_handle* h, int64_t j, double4* bal, double2* slope = nullptr)
 {
     AssimState* a = h->assim;
     DevMesh m = view_with(h, a->ctrl_on);
     m.bal = bal;
+    if (slope) m.slope = slope;
     const EView v = eview(a, a->d_dt + j, a->d_t + j);
     if (h->p.scheme == SW2D_SCHEME_MUSCL_EVR) launch_slopes_on(h, m);
     launch_edges<false>(h, m, v);
@@ -1087,7 +1117,8 @@ int chain_states(sw2d_handle* h)
     const int64_t K = (int64_t)a->segs.size(), nc = h->nc;
     while ((int64_t)a->cs.size() < K) {
         double4* p = nullptr;
-        CK(cudaMalloc(&p, std::max<int64_t>(1, nc) * sizeof(double4)));
+        int rc = take_checkpoint(h, &p);
+        if (rc) return rc;
         a->cs.push_back(p);
     }
     for (const auto& r : replay_runs(a)) {
@@ -1138,6 +1169,16 @@ int seg_buffers(sw2d_handle* h)
     if ((rc = adj_alloc(h, a->seg_allocs, (longest + 1) * h->nc, &a->seg_st)) ||
         (rc = adj_alloc(h, a->seg_allocs, longest * h->nc, &a->seg_bal)))
         return rc;
+    // the slopes too, when they fit in half of the free device memory (else the reverse steps rebuild
+    // them: 10k cells, 134 steps, 0.7 ms more per gradient)
+    a->seg_slope = nullptr;
+    size_t free_b = 0, total_b = 0;
+    if (h->p.scheme == SW2D_SCHEME_MUSCL_EVR && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+        (size_t)longest * h->nc * sizeof(double2) < free_b / 2 &&
+        adj_alloc(h, a->seg_allocs, longest * h->nc, &a->seg_slope)) {
+        a->seg_slope = nullptr;
+        h->err.clear();
+    }
     a->seg_cap = longest;
     return SW2D_OK;
 }
@@ -1171,7 +1212,7 @@ int reverse_segment(sw2d_handle* h, int64_t k)
     for (int64_t j = sg.j0; j < sg.j0 + sg.n; j++) {
         CK(cudaMemcpyAsync(a->seg_st + (j - sg.j0) * nc, h->m.st, nc * sizeof(double4), cudaMemcpyDeviceToDevice,
                            h->stream));
-        replay_step(h, j, a->seg_bal + (j - sg.j0) * nc);
+        replay_step(h, j, a->seg_bal + (j - sg.j0) * nc, a->seg_slope ? a->seg_slope + (j - sg.j0) * nc : nullptr);
     }
     CK(cudaMemcpyAsync(a->seg_st + sg.n * nc, h->m.st, nc * sizeof(double4), cudaMemcpyDeviceToDevice, h->stream));
     const unsigned gc = grid_for(nc);
@@ -1183,7 +1224,8 @@ int reverse_segment(sw2d_handle* h, int64_t k)
         mr.st = a->seg_st + r * nc;
         const double dt = a->dt_seq[j];
         if (gc > 0) launch_update_rev(h, mr, a->seg_bal + r * nc, dt);
-        if (muscl) launch_slopes_on(h, mr);
+        if (a->seg_slope) mr.slope = a->seg_slope + r * nc;
+        else if (muscl) launch_slopes_on(h, mr);
         const EView v = eview(a, a->d_dt + j, a->d_t + j);
         if (ge > 0) {
             const int ieee = h->assim_sqrt_zero;
@@ -1232,7 +1274,8 @@ void assim_release(sw2d_handle* h)
 {
     if (!h || !h->assim) return;
     AssimState* a = h->assim;
-    free_checkpoints(a);
+    spare_checkpoints(a);
+    free_spares(a);
     free_steps(a);
     free_list(a->seg_allocs);
     free_list(a->traj_allocs);
