@@ -158,30 +158,25 @@ __device__ __forceinline__ double slope_rev_cell(const DevMesh& m, int e0, int c
 }
 
 
-// Reverse of each cell's slope limiter (MUSCL-EVR): the cell's own z contribution is applied
-// here, the neighbours' go to znb (one value per internal-neighbour entry).
-__global__ void __launch_bounds__(kBlock) k_limiter_rev(DevMesh m, const double2* sgb, double4* lam,
-                                                        double* gzb, double* znb)
+// Reverse of the slope limiter of cell c (MUSCL-EVR) from the adjoint of its slope: the cell's own z
+// contribution is returned, the neighbours' go to znb (one value per internal-neighbour entry).  It
+// ends the kernel that gathers the slope's adjoint (as a kernel of its own it took 8 to 10 us at 10k
+// and 100k cells, two thirds of it placement and round trips to memory).
+__device__ __forceinline__ double limiter_rev(const DevMesh& m, int c, int e0, int e1, double sxb, double syb,
+                                              double* znb)
 {
-    chain_begin();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= m.nc) return;
-    const int e0 = ld(&m.coff[c].x), e1 = ld(&m.coff[c + 1].x);
     const int cnt = e1 - e0;
-    const double2 b = sgb[c];
-    if (b.x == 0.0 && b.y == 0.0) {
+    if (sxb == 0.0 && syb == 0.0) {
         for (int i = e0; i < e1; i++) znb[i] = 0.0;
-        return;
+        return 0.0;
     }
     const double zc = m.st[c].w;
     const double2 xy = ld(&m.cxy[c]);
-    double zcb = 0.0;
-    if (cnt <= 3) zcb = slope_rev_cell<3>(m, e0, cnt, zc, xy, b.x, b.y, znb);
-    else if (cnt == 4) zcb = slope_rev_cell<4>(m, e0, cnt, zc, xy, b.x, b.y, znb);
-    else if (cnt <= kMaxNbr) zcb = slope_rev_cell<kMaxNbr>(m, e0, cnt, zc, xy, b.x, b.y, znb);
-    else atomicOr(&m.ctrl->status, kStatusUnsupported);  // degree beyond the reverse's table
-    lam[c].x += zcb;
-    gzb[c] += zcb;
+    if (cnt <= 3) return slope_rev_cell<3>(m, e0, cnt, zc, xy, sxb, syb, znb);
+    if (cnt == 4) return slope_rev_cell<4>(m, e0, cnt, zc, xy, sxb, syb, znb);
+    if (cnt <= kMaxNbr) return slope_rev_cell<kMaxNbr>(m, e0, cnt, zc, xy, sxb, syb, znb);
+    atomicOr(&m.ctrl->status, kStatusUnsupported);  // degree beyond the reverse's table
+    return 0.0;
 }
 
 

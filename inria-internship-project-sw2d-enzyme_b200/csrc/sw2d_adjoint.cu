@@ -27,8 +27,8 @@
 //                                       for the edges whose flux the step computed; those slots'
 //                                       adjoints reset
 //   k_cells_rev     per cell            ordered gather over the cell's slots, with the reverse of the
-//                                       cell's reconstruction on each internal slot
-//   k_limiter_rev   per cell            reverse of the cell's slope limiter (per-neighbour
+//                                       cell's reconstruction on each internal slot, then the
+//                                       reverse of the cell's slope limiter (per-neighbour
 //                                       contributions) (MUSCL-EVR)
 //   k_nbr_rev       per cell            ordered gather of the neighbours' slope contributions
 //
@@ -81,7 +81,6 @@ struct AdjointState {
     double4* ctb = nullptr;              // nslot: per-slot contributions {h, q, r, z_b}
     double2* cts = nullptr;              // nslot: per-slot slope contributions {sx, sy}
     double* znb = nullptr;               // ncint: per-neighbour-entry z contributions
-    double2* sgb = nullptr;              // nc: adjoint of each cell's limited slope
     int* mirror = nullptr;               // ncint: entry of the same edge in the neighbour's list
     double4* sgeo = nullptr;             // ncint: {nx, ny, midpoint - centroid} of each entry's edge
     double* g_zb = nullptr;
@@ -460,12 +459,13 @@ __device__ __forceinline__ void cell_slot_rev(const double4& a, const double2& b
 // Ordered gather, over the slots of each cell in the reference's order: boundary slots hold
 // their final contributions; internal slots hold the adjoints of this cell's Riemann state,
 // taken back here through the cell's reconstruction (godunov_side / evr_side).  For MUSCL-EVR
-// the adjoint of the cell's limited slope goes to sgb for k_limiter_rev.  The adjoints of the
+// the reverse of the cell's limiter follows.  The adjoints of the
 // first kPre internal slots are loaded together, ahead of the boundary sums; a slot's geometry
-// only when its adjoints are not all zero.
+// only when its adjoints are not all zero.  Held to 128 registers: free, the limiter's reverse takes
+// 194 and a gradient of 100k cells 8.74 instead of 8.22 ms, of 300k 19.4 instead of 17.5.
 template <int kScheme>
-__global__ void __launch_bounds__(kBlock) k_cells_rev(DevMesh m, double4* lam, const double4* ctb,
-                                                      const double2* cts, double* gzb, double2* sgb,
+__global__ void __launch_bounds__(kBlock, 2) k_cells_rev(DevMesh m, double4* lam, const double4* ctb,
+                                                      const double2* cts, double* gzb, double* znb,
                                                       double dtp, const double4* __restrict__ sgeo)
 {
     chain_begin();
@@ -509,13 +509,19 @@ __global__ void __launch_bounds__(kBlock) k_cells_rev(DevMesh m, double4* lam, c
         cell_slot_rev<kMuscl>(ctb[k], cts[k], ld(&m.cint[e0 + i]).x, sgeo[e0 + i], s, cs, g, dtp, hb, qb, rb, zbb,
                               sxb, syb);
     }
-    if (kMuscl) sgb[c] = make_double2(sxb, syb);
     double4 l = lam[c];
+    double gz = gzb[c];
     l.x += hb;
     l.y += qb;
     l.z += rb;
+    gz += zbb;
+    if (kMuscl) {
+        const double zcb = limiter_rev(m, c, e0, e1, sxb, syb, znb);
+        l.x += zcb;
+        gz += zcb;
+    }
     lam[c] = l;
-    gzb[c] += zbb;
+    gzb[c] = gz;
 }
 
 // one reverse step of the trace: non-finite entries of the state adjoint (count, first cell)
@@ -570,7 +576,7 @@ int adjoint_fixed(sw2d_handle* h)
     auto& L = a->fixed_allocs;
     if ((rc = adj_alloc(h, L, h->nc, &a->lam)) || (rc = adj_alloc(h, L, a->nslot, &a->sig)) ||
         (rc = adj_alloc(h, L, a->nslot, &a->ctb)) || (rc = adj_alloc(h, L, a->nslot, &a->cts)) ||
-        (rc = adj_alloc(h, L, a->ncint, &a->znb)) || (rc = adj_alloc(h, L, h->nc, &a->sgb)) || (rc = adj_alloc(h, L, a->ncint, &a->mirror)) ||
+        (rc = adj_alloc(h, L, a->ncint, &a->znb)) || (rc = adj_alloc(h, L, a->ncint, &a->mirror)) ||
         (rc = adj_alloc(h, L, h->nc, &a->g_zb)) || (rc = adj_alloc(h, L, h->nc, &a->g_k1)) ||
         (rc = adj_alloc(h, L, h->nc, &a->g_k2)) || (rc = adj_alloc(h, L, 1, &a->ctrl_rev)) ||
         (rc = adj_alloc(h, L, kCostBlocks, &a->d_part)) ||
@@ -704,12 +710,11 @@ template <int kF>
 void launch_update_rev_f(sw2d_handle* h, const double4* bal, double dt)
 {
     AdjointState* a = h->adj;
-    const unsigned g = grid_for(h->nc);
     if (h->p.singular_head_loss)
-        launch_chained(k_update_rev<kF, true>, g, kBlock, 0, h->stream, h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
+        launch_spread(k_update_rev<kF, true>, h->nc, h->stream, h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
                                                             h->adj_flush_branch);
     else
-        launch_chained(k_update_rev<kF, false>, g, kBlock, 0, h->stream, h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
+        launch_spread(k_update_rev<kF, false>, h->nc, h->stream, h->m, bal, a->lam, a->sig, a->g_k1, a->g_k2, dt,
                                                              h->adj_flush_branch);
 }
 
@@ -941,13 +946,12 @@ int reverse_sweep(sw2d_handle* h, int64_t kept)
                              b.rs(j));
             const double dtp = j > 0 ? a->dt_seq[j - 1] : a->dt_before;
             if (muscl) {
-                launch_chained(k_cells_rev<SW2D_SCHEME_MUSCL_EVR>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_zb,
-                                                                                  a->sgb, dtp, a->sgeo);
-                launch_chained(k_limiter_rev, gc, kBlock, 0, h->stream, mr, a->sgb, a->lam, a->g_zb, a->znb);
-                launch_chained(k_nbr_rev, gc, kBlock, 0, h->stream, mr, a->mirror, a->znb, a->lam, a->g_zb);
+                launch_spread(k_cells_rev<SW2D_SCHEME_MUSCL_EVR>, nc, h->stream, mr, a->lam, a->ctb, a->cts, a->g_zb,
+                                                                                  a->znb, dtp, a->sgeo);
+                launch_spread(k_nbr_rev, nc, h->stream, mr, a->mirror, a->znb, a->lam, a->g_zb);
             } else {
-                launch_chained(k_cells_rev<SW2D_SCHEME_GODUNOV>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_zb,
-                                                                                a->sgb, dtp, a->sgeo);
+                launch_spread(k_cells_rev<SW2D_SCHEME_GODUNOV>, nc, h->stream, mr, a->lam, a->ctb, a->cts, a->g_zb,
+                                                                                a->znb, dtp, a->sgeo);
             }
             if (a->d_trace && j < a->trace_steps)
                 k_trace<<<gc, kBlock, 0, h->stream>>>(a->lam, (int)nc, a->d_trace + 4 * j);

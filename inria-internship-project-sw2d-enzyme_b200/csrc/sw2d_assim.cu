@@ -30,8 +30,9 @@
 //   k_e_edges_rev         per edge: fluxes recomputed, their adjoints from both cells' post-balance
 //                         adjoints, the edge factors' adjoints (-> porosity), the reverse of the
 //                         flux and of the Riemann states -> per-slot contributions
-//   k_e_cells_rev         per cell: ordered gather of the slot contributions
-//   k_limiter_rev, k_nbr_rev    reverse of the slope limiter (MUSCL-EVR)
+//   k_e_cells_rev         per cell: ordered gather of the slot contributions, then the reverse of the
+//                         cell's slope limiter (MUSCL-EVR)
+//   k_nbr_rev             its contributions to the neighbours (MUSCL-EVR)
 // All sums run in a fixed order and no floating-point atomics are used: the gradient is
 // bitwise reproducible.
 #include <cuda_runtime.h>
@@ -106,7 +107,7 @@ struct AssimState {
     double4* seg_bal = nullptr;      // seg_cap * nc
     double2* seg_slope = nullptr;    // seg_cap * nc: each step's slopes (MUSCL-EVR, when memory allows)
     double4 *lam = nullptr, *lamb = nullptr, *ctb = nullptr;
-    double2 *cts = nullptr, *sgb = nullptr;
+    double2* cts = nullptr;
     double *znb = nullptr, *gzb = nullptr;
     int* mirror = nullptr;
     double *g_phi = nullptr, *g_k1 = nullptr, *g_k2 = nullptr, *g_w = nullptr;   // g_w: watermark
@@ -613,15 +614,16 @@ __global__ void __launch_bounds__(kBlock) k_e_edges_rev(DevMesh m, EView v, cons
     }
 }
 
-// ordered gather of the slot contributions of each cell
+// ordered gather of the slot contributions of each cell, then the reverse of its limiter
 template <bool kMuscl>
-__global__ void __launch_bounds__(kBlock) k_e_cells_rev(DevMesh m, double4* lam, const double4* ctb,
-                                                        const double2* cts, double* gphi, double2* sgb)
+__global__ void __launch_bounds__(kBlock, 2) k_e_cells_rev(DevMesh m, double4* lam, const double4* ctb,
+                                                        const double2* cts, double* gphi, double* gzb, double* znb)
 {
     chain_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.nc) return;
-    const int k0 = ld(&m.coff[c].y), k1 = ld(&m.coff[c + 1].y);
+    const int2 o0 = ld(&m.coff[c]), o1 = ld(&m.coff[c + 1]);
+    const int k0 = o0.y, k1 = o1.y;
     double4 l = lam[c];
     double gp = 0.0, sx = 0.0, sy = 0.0;
     for (int k = k0; k < k1; k++) {
@@ -636,9 +638,13 @@ __global__ void __launch_bounds__(kBlock) k_e_cells_rev(DevMesh m, double4* lam,
             sy += s.y;
         }
     }
+    if (kMuscl) {
+        const double zcb = limiter_rev(m, c, o0.x, o1.x, sx, sy, znb);
+        l.x += zcb;
+        gzb[c] += zcb;
+    }
     lam[c] = l;
     gphi[c] += gp;
-    if (kMuscl) sgb[c] = make_double2(sx, sy);
 }
 
 // sum of squares of the h adjoint: per-block partials in a fixed tree
@@ -731,7 +737,7 @@ int fixed_buffers(sw2d_handle* h)
         (rc = adj_alloc(h, L, 1, &a->ctrl)) || (rc = adj_alloc(h, L, 1, &a->ctrl_on)) ||
         (rc = adj_alloc(h, L, 1, &a->d_obs_idx)) || (rc = adj_alloc(h, L, nc, &a->lam)) ||
         (rc = adj_alloc(h, L, nc, &a->lamb)) || (rc = adj_alloc(h, L, a->nslot, &a->ctb)) ||
-        (rc = adj_alloc(h, L, a->nslot, &a->cts)) || (rc = adj_alloc(h, L, nc, &a->sgb)) ||
+        (rc = adj_alloc(h, L, a->nslot, &a->cts)) ||
         (rc = adj_alloc(h, L, a->ncint, &a->znb)) || (rc = adj_alloc(h, L, nc, &a->gzb)) ||
         (rc = adj_alloc(h, L, a->ncint, &a->mirror)) || (rc = adj_alloc(h, L, nc, &a->g_phi)) ||
         (rc = adj_alloc(h, L, nc, &a->g_k1)) || (rc = adj_alloc(h, L, nc, &a->g_k2)) ||
@@ -795,22 +801,20 @@ EView eview(const AssimState* a, const double* dtp, const double* tp)
 template <bool kRecord>
 void launch_edges(sw2d_handle* h, const DevMesh& m, const EView& v)
 {
-    const unsigned g = grid_for(h->ni + h->nb);
-    if (g == 0) return;
-    if (h->p.scheme == SW2D_SCHEME_GODUNOV) launch_chained(k_e_edges<SW2D_SCHEME_GODUNOV, kRecord>, g, kBlock, 0, h->stream, m, v);
-    else launch_chained(k_e_edges<SW2D_SCHEME_MUSCL_EVR, kRecord>, g, kBlock, 0, h->stream, m, v);
+    if (h->ni + h->nb == 0) return;
+    if (h->p.scheme == SW2D_SCHEME_GODUNOV) launch_spread(k_e_edges<SW2D_SCHEME_GODUNOV, kRecord>, h->ni + h->nb, h->stream, m, v);
+    else launch_spread(k_e_edges<SW2D_SCHEME_MUSCL_EVR, kRecord>, h->ni + h->nb, h->stream, m, v);
 }
 
 template <int kF>
 void launch_update_f(sw2d_handle* h, const DevMesh& m, const double* dtp, const int* go, bool store)
 {
-    const unsigned g = grid_for(h->nc);
     if (h->p.singular_head_loss) {
-        if (store) launch_chained(k_e_update<kF, true, true>, g, kBlock, 0, h->stream, m, dtp, go);
-        else launch_chained(k_e_update<kF, true, false>, g, kBlock, 0, h->stream, m, dtp, go);
+        if (store) launch_spread(k_e_update<kF, true, true>, h->nc, h->stream, m, dtp, go);
+        else launch_spread(k_e_update<kF, true, false>, h->nc, h->stream, m, dtp, go);
     } else {
-        if (store) launch_chained(k_e_update<kF, false, true>, g, kBlock, 0, h->stream, m, dtp, go);
-        else launch_chained(k_e_update<kF, false, false>, g, kBlock, 0, h->stream, m, dtp, go);
+        if (store) launch_spread(k_e_update<kF, false, true>, h->nc, h->stream, m, dtp, go);
+        else launch_spread(k_e_update<kF, false, false>, h->nc, h->stream, m, dtp, go);
     }
 }
 
@@ -824,12 +828,11 @@ void launch_update(sw2d_handle* h, const DevMesh& m, const double* dtp, const in
 void launch_update_rev(sw2d_handle* h, const DevMesh& m, const double4* bal, double dt)
 {
     AssimState* a = h->assim;
-    const unsigned g = grid_for(h->nc);
     const bool fr = h->p.friction != SW2D_FRICTION_NONE, hl = h->p.singular_head_loss != 0;
-    if (fr && hl) launch_chained(k_e_update_rev<SW2D_FRICTION_STRICKLER, true>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
-    else if (fr) launch_chained(k_e_update_rev<SW2D_FRICTION_STRICKLER, false>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
-    else if (hl) launch_chained(k_e_update_rev<SW2D_FRICTION_NONE, true>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
-    else launch_chained(k_e_update_rev<SW2D_FRICTION_NONE, false>, g, kBlock, 0, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    if (fr && hl) launch_spread(k_e_update_rev<SW2D_FRICTION_STRICKLER, true>, h->nc, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    else if (fr) launch_spread(k_e_update_rev<SW2D_FRICTION_STRICKLER, false>, h->nc, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    else if (hl) launch_spread(k_e_update_rev<SW2D_FRICTION_NONE, true>, h->nc, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
+    else launch_spread(k_e_update_rev<SW2D_FRICTION_NONE, false>, h->nc, h->stream, m, bal, a->lam, a->lamb, a->g_k1, a->g_k2, dt);
 }
 
 int64_t obs_width(const AssimState* a, const sw2d_handle* h)
@@ -1230,16 +1233,15 @@ int reverse_segment(sw2d_handle* h, int64_t k)
         if (ge > 0) {
             const int ieee = h->assim_sqrt_zero;
             if (muscl)
-                launch_chained(k_e_edges_rev<SW2D_SCHEME_MUSCL_EVR>, ge, kBlock, 0, h->stream, mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
-            else launch_chained(k_e_edges_rev<SW2D_SCHEME_GODUNOV>, ge, kBlock, 0, h->stream, mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
+                launch_spread(k_e_edges_rev<SW2D_SCHEME_MUSCL_EVR>, h->ni + h->nb, h->stream, mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
+            else launch_spread(k_e_edges_rev<SW2D_SCHEME_GODUNOV>, h->ni + h->nb, h->stream, mr, v, a->lamb, a->ctb, a->cts, dt, ieee);
         }
         if (gc > 0) {
             if (muscl) {
-                launch_chained(k_e_cells_rev<true>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_phi, a->sgb);
-                launch_chained(k_limiter_rev, gc, kBlock, 0, h->stream, mr, a->sgb, a->lam, a->gzb, a->znb);
-                launch_chained(k_nbr_rev, gc, kBlock, 0, h->stream, mr, a->mirror, a->znb, a->lam, a->gzb);
+                launch_spread(k_e_cells_rev<true>, nc, h->stream, mr, a->lam, a->ctb, a->cts, a->g_phi, a->gzb, a->znb);
+                launch_spread(k_nbr_rev, nc, h->stream, mr, a->mirror, a->znb, a->lam, a->gzb);
             } else {
-                launch_chained(k_e_cells_rev<false>, gc, kBlock, 0, h->stream, mr, a->lam, a->ctb, a->cts, a->g_phi, a->sgb);
+                launch_spread(k_e_cells_rev<false>, nc, h->stream, mr, a->lam, a->ctb, a->cts, a->g_phi, a->gzb, a->znb);
             }
         }
     }

@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(kB, kMinB) k_ddp_edges(DevMesh m)
         const int ao = ld_now(&m.ctoff[a]), an = ld_now(&m.ctoff[a + 1]) - ao;
         const int bo = ld_now(&m.ctoff[b]), bn = ld_now(&m.ctoff[b + 1]) - bo;
         const double4 sa = ld_prev(&m.st[a]), sb = ld_prev(&m.st[b]);   // {theta, theta u, theta v, z}
-        const double2 va = ld(reinterpret_cast<const double2*>(&m.dv[a]));  // {phiW, thetaW} at z
-        const double2 vb = ld(reinterpret_cast<const double2*>(&m.dv[b]));
+        const double2 va = ld_prev(reinterpret_cast<const double2*>(&m.dv[a]));  // {phiW, thetaW} at z
+        const double2 vb = ld_prev(reinterpret_cast<const double2*>(&m.dv[b]));
         const double2 ca = ld(reinterpret_cast<const double2*>(&m.cst[a]));  // {z_b, boussinesq}
         const double2 cb = ld(reinterpret_cast<const double2*>(&m.cst[b]));
         const double ta0 = ld(&m.cst[a].z), tb0 = ld(&m.cst[b].z);  // lowest table levels
@@ -809,13 +809,13 @@ void launch_edges_v(sw2d_handle* h, const DevMesh& m)
 template <int kF, bool kHL>
 void launch_tail_f(sw2d_handle* h, const DevMesh& m)
 {
-    const unsigned g = grid_for(m.nc);
     DdpState* d = h->ddp;
     if (d->div_corr == kDivCorrNone) {
-        if (h->dissipation) launch_chained(k_ddp_update<kF, kHL, true>, g, kBlock, 0, h->stream, m);
-        else launch_chained(k_ddp_update<kF, kHL, false>, g, kBlock, 0, h->stream, m);
+        if (h->dissipation) launch_spread(k_ddp_update<kF, kHL, true>, m.nc, h->stream, m);
+        else launch_spread(k_ddp_update<kF, kHL, false>, m.nc, h->stream, m);
         return;
     }
+    const unsigned g = grid_for(m.nc);
     k_ddp_balance<<<g, kBlock, 0, h->stream>>>(m, h->dissipation != 0);
     if (d->div_corr == kDivCorrTimestep) {
         k_dc_ts_scan<<<g, kBlock, 0, h->stream>>>(m, h->d_cell_perm);

@@ -277,6 +277,17 @@ inline void launch_chained(void (*kernel)(KArgs...), unsigned grid, unsigned blo
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);  // errors: cudaGetLastError, as after <<<>>>
 }
 
+// One thread per item, for kernels that take any block of whole warps up to kBlock, in small blocks:
+// the SMs share a small mesh evenly, and in a large one a finished block's place is taken at once
+// (256 -> 64 threads: k_update of 4M cells 116.5 -> 112.1 us, of 250k 15.8 -> 14.6; a gradient of 100k
+// cells 8.83 -> 8.59 ms, of 10k cells with porosity 9.57 -> 9.27 ms).
+template <class... KArgs, class... Args>
+inline void launch_spread(void (*kernel)(KArgs...), long long n, cudaStream_t stream, Args&&... args)
+{
+    constexpr unsigned b = 64;
+    launch_chained(kernel, (unsigned)((n + b - 1) / b), b, 0, stream, args...);
+}
+
 __device__ __forceinline__ bool step_active(const Ctrl* c) { return c->t < c->t_max; }
 
 inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }

@@ -407,21 +407,20 @@ void launch_slopes(sw2d_handle* h, const DevMesh& m, int v)
 void launch_slopes(sw2d_handle* h, int v) { launch_slopes(h, h->m, v); }
 
 template <int kF, bool kStoreB, bool kDissip>
-void launch_update_f(sw2d_handle* h, const DevMesh& m, unsigned g)
+void launch_update_f(sw2d_handle* h, const DevMesh& m)
 {
-    if (h->p.singular_head_loss) launch_chained(k_update<kF, true, kStoreB, kDissip>, g, kBlock, 0, h->stream, m);
-    else launch_chained(k_update<kF, false, kStoreB, kDissip>, g, kBlock, 0, h->stream, m);
+    if (h->p.singular_head_loss) launch_spread(k_update<kF, true, kStoreB, kDissip>, m.nc, h->stream, m);
+    else launch_spread(k_update<kF, false, kStoreB, kDissip>, m.nc, h->stream, m);
 }
 
 template <bool kStoreB, bool kDissip>
 void launch_update_d(sw2d_handle* h, const DevMesh& m)
 {
-    const unsigned g = grid_for(m.nc);
     switch (h->p.friction) {
-        case SW2D_FRICTION_CHEZY: launch_update_f<SW2D_FRICTION_CHEZY, kStoreB, kDissip>(h, m, g); break;
-        case SW2D_FRICTION_MANNING: launch_update_f<SW2D_FRICTION_MANNING, kStoreB, kDissip>(h, m, g); break;
-        case SW2D_FRICTION_STRICKLER: launch_update_f<SW2D_FRICTION_STRICKLER, kStoreB, kDissip>(h, m, g); break;
-        default: launch_update_f<SW2D_FRICTION_NONE, kStoreB, kDissip>(h, m, g); break;
+        case SW2D_FRICTION_CHEZY: launch_update_f<SW2D_FRICTION_CHEZY, kStoreB, kDissip>(h, m); break;
+        case SW2D_FRICTION_MANNING: launch_update_f<SW2D_FRICTION_MANNING, kStoreB, kDissip>(h, m); break;
+        case SW2D_FRICTION_STRICKLER: launch_update_f<SW2D_FRICTION_STRICKLER, kStoreB, kDissip>(h, m); break;
+        default: launch_update_f<SW2D_FRICTION_NONE, kStoreB, kDissip>(h, m); break;
     }
 }
 
