@@ -66,6 +66,60 @@ SW2D_HD void for_levels(const Lvl* t, int n, F&& f)
     }
 }
 
+// A query's state in table_pass: phi and theta at z
+struct Query {
+    bool run = true;
+    int l = 0;
+    double th = 0;
+    SW2D_HD void visit(int k, double z, const Lvl& lv, double theta)
+    {
+        run = run && z > lv.z;
+        l = run ? k + 1 : l;
+        th = run ? theta : th;
+    }
+    SW2D_HD PhiTheta result(const Lvl* t, double z0, double z, unsigned& bad) const
+    {
+        if (z <= z0) return PhiTheta{0.0, 0.0};
+        if (l == 0) {
+            bad |= kStatusTable;
+            return PhiTheta{quiet_nan(), quiet_nan()};
+        }
+        const Lvl a = load_level(t + (l - 1));
+        double theta = th;
+        if (z > a.z) theta += (z - a.z) * a.phi;
+        return PhiTheta{a.phi, theta};
+    }
+};
+
+// A force's state in table_pass
+struct Force {
+    bool run = false;
+    int c = 0;
+    double acc = 0;
+    Force() = default;
+    SW2D_HD Force(double z, double z0) : run(z > z0) {}
+    SW2D_HD void visit(int k, double z, const Lvl& prev, const Lvl& lv, double mid, double dz2)
+    {
+        run = run && z >= lv.z;
+        const double dz1 = z - mid;
+        const double sum = acc + prev.phi * dz1 * dz2;
+        acc = run ? sum : acc;
+        c = run ? k : c;
+    }
+    SW2D_HD double result(const Lvl* t, double z0, double z) const
+    {
+        double v = 0;
+        if (z > z0) {
+            const Lvl cur = load_level(t + c);
+            v = acc;
+            const double dz1 = smax(0., z - cur.z);
+            v += cur.phi * dz1 * dz1 / 2.;
+        }
+        v *= kGravity;
+        return v;
+    }
+};
+
 // One pass over a table answering phiWOfZ / thetaWOfZ (equally phiGIntOfZ / thetaGIntOfZ;
 // swDdp.cpp:1049-1097, 2678-2736) at the NQ elevations zq and the pressure-force integral
 // pressureForceOmegaOfZ / pressureForceGammaOfZ (swDdp.cpp:1214-1273) at the NP elevations zp,
@@ -75,83 +129,35 @@ SW2D_HD void for_levels(const Lvl* t, int n, F&& f)
 //   force at z: when z > z_0, sum over the leading levels k >= 1 with z >= z_k of
 //     phi_(k-1) (z - (z_(k-1) + z_k) / 2) (z_k - z_(k-1)), then phi_l max(0, z - z_l)^2 / 2 at
 //     the last such level l; times g.
+// The walk keeps the level's index and theta only and loads the level again after it (it is in L1);
+// keeping the levels themselves took six selects a query and level (k_ddp_edges of 200k cells 56.6 ->
+// 55.4 us at 256 x 2, 51.4 at 128 x 5, which the fewer live values allow).
 template <int NQ, int NP>
 SW2D_HD void table_pass(const Lvl* t, int n, const double* zq, PhiTheta* pq, const double* zp, double* pp,
                         unsigned& bad)
 {
     const double z0 = load_level(t).z;
-    bool run[NQ > 0 ? NQ : 1];
-    bool hit[NQ > 0 ? NQ : 1];
-    LvlT a[NQ > 0 ? NQ : 1];
-    bool prun[NP > 0 ? NP : 1];
-    bool started[NP > 0 ? NP : 1];
-    double acc[NP > 0 ? NP : 1];
-    LvlT cur[NP > 0 ? NP : 1];
+    Query q[NQ > 0 ? NQ : 1];
+    Force f[NP > 0 ? NP : 1];
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-        run[q] = true;
-        hit[q] = false;
-        a[q] = LvlT{0, 0, 0};
-    }
-#pragma unroll
-    for (int p = 0; p < NP; p++) {
-        started[p] = zp[p] > z0;
-        prun[p] = started[p];
-        acc[p] = 0;
-        cur[p] = LvlT{0, 0, 0};
-    }
-    LvlT prev{0, 0, 0};
+    for (int p = 0; p < NP; p++) f[p] = Force(zp[p], z0);
+    Lvl prev{0, 0};
     for_levels(t, n, [&](int k, const LvlT& lv) {
+        const Lvl cur{lv.z, lv.phi};
 #pragma unroll
-        for (int q = 0; q < NQ; q++) {
-            if (run[q]) {
-                if (zq[q] > lv.z) {
-                    hit[q] = true;
-                    a[q] = lv;
-                } else {
-                    run[q] = false;
-                }
-            }
-        }
+        for (int i = 0; i < NQ; i++) q[i].visit(k, zq[i], cur, lv.theta);
+        if (NP > 0 && k > 0) {
+            const double mid = (prev.z + lv.z) / 2.;
+            const double dz2 = lv.z - prev.z;
 #pragma unroll
-        for (int p = 0; p < NP; p++) {
-            if (k == 0) {
-                cur[p] = lv;
-            } else if (prun[p] && zp[p] >= lv.z) {
-                const double dz1 = zp[p] - (prev.z + lv.z) / 2.;
-                const double dz2 = lv.z - prev.z;
-                acc[p] += prev.phi * dz1 * dz2;
-                cur[p] = lv;
-            } else {
-                prun[p] = false;
-            }
+            for (int p = 0; p < NP; p++) f[p].visit(k, zp[p], prev, cur, mid, dz2);
         }
-        prev = lv;
+        prev = cur;
     });
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-        if (zq[q] <= z0) {
-            pq[q] = PhiTheta{0.0, 0.0};
-        } else if (!hit[q]) {
-            bad |= kStatusTable;
-            pq[q] = PhiTheta{quiet_nan(), quiet_nan()};
-        } else {
-            double theta = a[q].theta;
-            if (zq[q] > a[q].z) theta += (zq[q] - a[q].z) * a[q].phi;
-            pq[q] = PhiTheta{a[q].phi, theta};
-        }
-    }
+    for (int i = 0; i < NQ; i++) pq[i] = q[i].result(t, z0, zq[i], bad);
 #pragma unroll
-    for (int p = 0; p < NP; p++) {
-        double v = 0;
-        if (started[p]) {
-            v = acc[p];
-            const double dz1 = smax(0., zp[p] - cur[p].z);
-            v += cur[p].phi * dz1 * dz1 / 2.;
-        }
-        v *= kGravity;
-        pp[p] = v;
-    }
+    for (int p = 0; p < NP; p++) pp[p] = f[p].result(t, z0, zp[p]);
 }
 
 // phiWOfZ and thetaWOfZ at one elevation
@@ -180,27 +186,22 @@ SW2D_HD double pressure_force(const Lvl* t, int n, double z)
 // swDdp::zOfThetaW (swDdp.cpp:3368-3388): theta_0 ... scanned while theta > theta_k
 SW2D_HD double z_of_theta(const Lvl* t, int n, double theta, unsigned& bad)
 {
-    bool run = true, hit = false;
-    LvlT a{0, 0, 0};
-    double z0 = 0;
+    bool run = true;
+    int l = 0;      // leading levels below theta, and the last one's theta
+    double th = 0;
     for_levels(t, n, [&](int k, const LvlT& lv) {
-        if (k == 0) z0 = lv.z;
-        if (run) {
-            if (theta > lv.theta) {
-                hit = true;
-                a = lv;
-            } else {
-                run = false;
-            }
-        }
+        run = run && theta > lv.theta;
+        l = run ? k + 1 : l;
+        th = run ? lv.theta : th;
     });
-    if (theta <= 0) return z0;
-    if (!hit) {
+    if (theta <= 0) return load_level(t).z;
+    if (l == 0) {
         bad |= kStatusTable;
         return quiet_nan();
     }
+    const Lvl a = load_level(t + (l - 1));
     double z = a.z;
-    z += (theta - a.theta) / a.phi;
+    z += (theta - th) / a.phi;
     return z;
 }
 

@@ -1121,7 +1121,10 @@ int ddp_setup(sw2d_handle* h, const sw2d_mesh* mesh, const sw2d_cell_fields* fie
     (void)fields;
     DdpState* d = new DdpState();
     h->ddp = d;
-    h->edge_variant = 0;  // {256, 2}: the DDP edge kernel's registers without spills
+    // the launch variant where the lines between the measured ones lie (us per step): {128, 5}, 96
+    // registers with a few spilled, once the grid is several waves deep (200k cells: 67.2, {256, 2}
+    // 70.8; 600k: 170 against 187), else {256, 2} without spills (20k: 22.4 against 23.0; 50k: 26.4, 27.4)
+    h->edge_variant = h->nc < 100000 ? 0 : 4;
     d->div_corr = ddp->div_corr;
     d->n_it_div_max = (int)ddp->n_it_div_max;
     const int64_t nc = h->nc, ni = h->ni, nb = h->nb;
