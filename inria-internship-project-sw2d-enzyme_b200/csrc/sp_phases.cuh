@@ -117,7 +117,7 @@ __device__ __forceinline__ double2 slope_gradient(const double4* st, const doubl
 // reciprocal (the weight) from the edge's record {dist, 1 / dist, mx, my}: both are statics of the
 // mesh, the same bits from either side.  That removes a square root and a division per neighbour,
 // and the four divisions by dist become div_known.  The kernel was bound by instruction issue on
-// those sequences (918 per warp, 35 % of them FP64): 54 -> 36 us per launch at 1M cells.
+// those sequences (918 per warp, 35 % of them FP64): 54 -> 41 us per launch at 1M cells.
 template <class L>
 __device__ __forceinline__ void slopes_cell(const DevMesh& m, int c)
 {

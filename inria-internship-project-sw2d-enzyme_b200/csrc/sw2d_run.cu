@@ -23,10 +23,10 @@
 // of the CTA (up to about 20k cells on 148 SMs): one component of the slope, one side's Riemann state.
 // Divisions and roots are the forms that keep zeros off the general routine (DivZero).
 //
-// Measured (B200, us per step, graph of the four kernels -> k_run): MUSCL-EVR 500 cells 18.0 -> 7.9, 2,000
-// 18.4 -> 8.2, 20,000 19.7 -> 10.6, 40,000 22.6 -> 13.4, 59,000 23.4 -> 17.3; Godunov 4,800 (channel)
-// 17.1 -> 8.1, 10,000 14.9 -> 6.9, 59,000 16.9 -> 11.3; DIP 15,000 21.9 -> 11.7, Godunov 30,000
-// 18.3 -> 9.6.  A tile of about 450 cells fills the shared memory of an SM, which ends the range.
+// Measured (B200, us per step, graph of the chained four kernels -> k_run): MUSCL-EVR 500 cells 15.8 -> 7.6,
+// 2,000 16.7 -> 8.2, 20,000 18.7 -> 10.7, 40,000 20.8 -> 12.1, 60,000 24.3 -> 15.0; Godunov 5,000 15.9 -> 7.7,
+// 20,000 16.1 -> 9.0, 60,000 18.9 -> 12.6; DIP 20,000 20.5 -> 12.3, 60,000 27.4 -> 20.2, its Godunov 20,000
+// 15.4 -> 8.8.  A tile of about 450 cells fills the shared memory of an SM, which ends the range.
 #include <cuda_runtime.h>
 
 #include <algorithm>
