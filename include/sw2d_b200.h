@@ -453,7 +453,7 @@ const char* sw2d_phase_name(int i);
  * "adjoint_kept_segments" (at least 1): sw2d_adjoint on a trajectory whose checkpoints a change of
  * the parameters has outdated runs it first, and keeps the steps of its last segments meanwhile
  * instead of recomputing them: this many at most, and what an eighth of the free device memory
- * holds (the default).  The same bits either way.  Takes effect at the next sw2d_record.
+ * and, over all handles, 1/32 of the device's holds (the default).  The same bits either way.  Takes effect at the next sw2d_record.
  * "run_kernel" (0/1, default 1): sw2d_step_n and sw2d_execute take the steps of a small SP or DIP
  * mesh (one whose cells fit the chip's shared memory) in one launch; 0 takes them kernel by kernel.
  * "run_wait_polls": the poll limit of that launch's waits, after which it gives up with an error

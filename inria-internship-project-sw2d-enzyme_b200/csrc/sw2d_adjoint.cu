@@ -40,6 +40,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -74,6 +75,9 @@ struct AdjointState {
     double2* seg_rs = nullptr;           // every * ni * 5: each step's Riemann states (when memory allows)
     double4 *more_st = nullptr, *more_bal = nullptr;  // the buffers after the first
     double2 *more_slope = nullptr, *more_rs = nullptr;
+    std::vector<void*> more_allocs;
+    size_t more_bytes = 0;
+    bool more_busy = false;              // a gradient is using them
     double2* eside = nullptr;            // 3 * ni: {z_b}, {b}, {phi} of each internal edge's (L, R) cells
     // adjoint buffers
     double4* lam = nullptr;              // nc: adjoint of the state {h, q, r, -}
@@ -975,27 +979,87 @@ int reverse_sweep(sw2d_handle* h, int64_t kept)
     return SW2D_OK;
 }
 
+// The handles that hold buffers for more segments than the first, and the bytes of them all: at most
+// 1/32 of the device's memory, so that ensembles of handles leave each other room, and given back
+// when a trajectory's own arrays find none.
+struct MorePool {
+    std::mutex mu;
+    std::vector<AdjointState*> holders;
+    size_t bytes = 0;
+};
+MorePool& more_pool()
+{
+    static MorePool* p = new MorePool;
+    return *p;
+}
+
+// with the pool's mutex held
+void drop_more(AdjointState* a)
+{
+    MorePool& p = more_pool();
+    free_list(a->more_allocs);
+    p.bytes -= a->more_bytes;
+    p.holders.erase(std::remove(p.holders.begin(), p.holders.end(), a), p.holders.end());
+    a->more_bytes = 0;
+    a->more_st = a->more_bal = nullptr;
+    a->more_slope = a->more_rs = nullptr;
+    a->n_seg = 1;
+}
+
+// frees the buffers that no gradient is using; whether there were any
+bool give_back_more()
+{
+    MorePool& p = more_pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    const std::vector<AdjointState*> all = p.holders;
+    bool any = false;
+    for (AdjointState* a : all)
+        if (!a->more_busy) {
+            drop_more(a);
+            any = true;
+        }
+    return any;
+}
+
+// keeps a handle's buffers from being given back meanwhile
+struct MoreUse {
+    AdjointState* a;
+    explicit MoreUse(AdjointState* a_) : a(a_) { set(true); }
+    ~MoreUse() { set(false); }
+    void set(bool on)
+    {
+        std::lock_guard<std::mutex> lock(more_pool().mu);
+        a->more_busy = on;
+    }
+};
+
 // Buffers for more of the trajectory's last segments (each costs what the first one does): as many
-// as an eighth of the free device memory holds
+// as an eighth of the free device memory and the pool's share hold
 void more_segments(sw2d_handle* h, int64_t seg)
 {
     AdjointState* a = h->adj;
     const int64_t nc = h->nc;
+    MorePool& p = more_pool();
+    std::lock_guard<std::mutex> lock(p.mu);
     size_t free_b = 0, total_b = 0;
     if (!a->seg_rs || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return;
     const size_t one = (size_t)(2 * seg + 1) * nc * sizeof(double4) +
                        (size_t)seg * ((a->seg_slope ? nc : 0) + 5 * h->ni) * sizeof(double2);
-    const int64_t n = std::min({a->n_ck - 1, (int64_t)(free_b / 8 / one), h->adj_kept_segments - 1});
+    const size_t share = std::min(free_b / 8, total_b / 32 - std::min(p.bytes, total_b / 32));
+    const int64_t n = std::min({a->n_ck - 1, (int64_t)(share / one), h->adj_kept_segments - 1});
     if (n <= 0) return;
-    std::vector<void*> L;
+    std::vector<void*>& L = a->more_allocs;
     if (adj_alloc(h, L, n * (seg + 1) * nc, &a->more_st) || adj_alloc(h, L, n * seg * nc, &a->more_bal) ||
         (a->seg_slope && adj_alloc(h, L, n * seg * nc, &a->more_slope)) ||
         adj_alloc(h, L, n * seg * h->ni * 5, &a->more_rs)) {
-        free_list(L);
+        cudaGetLastError();
+        drop_more(a);
         h->err.clear();
         return;
     }
-    a->traj_allocs.insert(a->traj_allocs.end(), L.begin(), L.end());
+    p.holders.push_back(a);
+    a->more_bytes = n * one;
+    p.bytes += a->more_bytes;
     a->n_seg = 1 + n;
 }
 
@@ -1003,24 +1067,32 @@ int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
 {
     AdjointState* a = h->adj;
     free_list(a->traj_allocs);
+    {
+        std::lock_guard<std::mutex> lock(more_pool().mu);
+        drop_more(a);
+    }
     a->ck_valid = false;
     a->n_requested = 0;
     a->n_steps = n_steps;
     a->every = every;
     a->n_ck = (n_steps + every - 1) / every;
-    a->n_seg = 1;
-    a->more_slope = nullptr;
     const int64_t nc = h->nc, seg = std::min(every, n_steps);
     auto& L = a->traj_allocs;
     int rc = SW2D_OK;
-    if ((rc = adj_alloc(h, L, (a->n_ck + 1) * nc, &a->ck_st)) ||
-        (rc = adj_alloc(h, L, (a->n_ck + 1) * a->nslot, &a->ck_slot)) ||
-        (rc = adj_alloc(h, L, a->n_ck + 1, &a->ck_ctrl)) || (rc = adj_alloc(h, L, (seg + 1) * nc, &a->seg_st)) ||
-        (rc = adj_alloc(h, L, seg * nc, &a->seg_bal)) || (rc = adj_alloc(h, L, n_steps, &a->d_dt_seq)) ||
-        (rc = adj_alloc(h, L, n_steps, &a->d_t_seq))) {
+    for (bool again = true;; again = false) {
+        if (!(rc = adj_alloc(h, L, (a->n_ck + 1) * nc, &a->ck_st)) &&
+            !(rc = adj_alloc(h, L, (a->n_ck + 1) * a->nslot, &a->ck_slot)) &&
+            !(rc = adj_alloc(h, L, a->n_ck + 1, &a->ck_ctrl)) && !(rc = adj_alloc(h, L, (seg + 1) * nc, &a->seg_st)) &&
+            !(rc = adj_alloc(h, L, seg * nc, &a->seg_bal)) && !(rc = adj_alloc(h, L, n_steps, &a->d_dt_seq)) &&
+            !(rc = adj_alloc(h, L, n_steps, &a->d_t_seq)))
+            break;
         free_list(a->traj_allocs);
-        a->n_steps = 0;
-        return rc;
+        if (!again || !give_back_more()) {
+            a->n_steps = 0;
+            return rc;
+        }
+        cudaGetLastError();
+        h->err.clear();
     }
     // each step's slopes and Riemann states, kept by the segment's forward recompute for the
     // reverse steps, when they fit in half of the free device memory (else rebuilt there)
@@ -1094,6 +1166,10 @@ void adjoint_release(sw2d_handle* h)
     if (!h || !h->adj) return;
     cudaFree(h->adj->d_trace);
     free_list(h->adj->traj_allocs);
+    {
+        std::lock_guard<std::mutex> lock(more_pool().mu);
+        drop_more(h->adj);
+    }
     free_list(h->adj->obs_allocs);
     free_list(h->adj->fixed_allocs);
     delete h->adj;
@@ -1375,6 +1451,7 @@ int sw2d_adjoint(sw2d_handle* h, double* J, const sw2d_gradient* grad)
     CK(cudaSetDevice(h->device));
     AdjointState* a = h->adj;
     if ((rc = check_observations(h))) return rc;
+    const MoreUse use(a);
     int64_t kept = 0;
     if (!a->ck_valid) {
         if ((rc = run_keeping(h))) return rc;

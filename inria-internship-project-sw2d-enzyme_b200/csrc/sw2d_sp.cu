@@ -1441,7 +1441,8 @@ int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value)
         return SW2D_OK;
     } else if (std::strcmp(name, "adjoint_kept_segments") == 0) {
         // how many of the last segments a gradient that has to run the trajectory itself may keep
-        // while it does (at least 1; default: what an eighth of the free device memory holds).
+        // while it does (at least 1; default: what an eighth of the free device memory holds, and
+        // 1/32 of the device's over all handles).
         // Takes effect at the next sw2d_record.
         if (value < 1) return fail(h, SW2D_E_ARG, "adjoint_kept_segments must be at least 1");
         h->adj_kept_segments = value;

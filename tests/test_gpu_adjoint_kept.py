@@ -57,3 +57,25 @@ def test_kept_segments_option(pkg):
     model = pkg.SpModel(pkg.workloads.dam_break(n_cells=400))
     with pytest.raises(pkg.Sw2dError):
         model.set_option("adjoint_kept_segments", 0)
+
+
+def test_recording_again_and_closing(pkg):
+    """The kept buffers go with the trajectory: handles that record again, or are closed, leave the
+    others' gradients alone."""
+    case = pkg.workloads.dam_break(n_cells=1500)
+
+    def observe(model, n):
+        model.set_observations([3, 40], [n // 2, n], np.full((2, 2), 1.0))
+        model.set_param("friction", case.friction[0] * 1.1)
+        return _bits(model.adjoint())
+
+    a, b = pkg.SpModel(case), pkg.SpModel(case)
+    for model in (a, b):
+        model.record(30, 8)
+    want = observe(a, 30)
+    assert all(np.array_equal(x, y) for x, y in zip(observe(b, 30), want))
+    c = pkg.SpModel(case)
+    c.record(12, 3)
+    c.close()
+    a.close()
+    assert all(np.array_equal(x, y) for x, y in zip(observe(b, 30), want))
