@@ -254,9 +254,10 @@ __device__ __forceinline__ double ld_prev_now(const double* p)
     return v;
 }
 
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin()
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    chain_wait();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
