@@ -888,6 +888,11 @@ int run_keeping(sw2d_handle* h)
         const double4* end = segment_buffer(h, s).st(std::min(a->n_steps, (s + 1) * a->every));
         CK(cudaMemcpyAsync(h->m.st, end, h->nc * sizeof(double4), cudaMemcpyDeviceToDevice, h->stream));
     }
+    // the model is left at the trajectory's end, with the slopes of its last step (sw2d_get_array)
+    if (a->n_steps > 0 && h->p.scheme == SW2D_SCHEME_MUSCL_EVR) {
+        const double2* last = segment_buffer(h, a->n_ck - 1).slope(a->n_steps - 1);
+        if (last) CK(cudaMemcpyAsync(h->m.slope, last, h->nc * sizeof(double2), cudaMemcpyDeviceToDevice, h->stream));
+    }
     if ((rc = ck_save(h, a->n_ck))) return rc;
     CK(cudaGetLastError());
     return SW2D_OK;
