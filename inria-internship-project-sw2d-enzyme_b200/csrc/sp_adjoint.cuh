@@ -29,9 +29,11 @@ SW2D_HD double dsqrt_bar(double y, double ybar) { return (y > 0.0) ? sw2d_div(yb
 
 // Reverse of root = sqrt((b - 1) b u u + c c): adds to the adjoints of u and c.  Where the root is c
 // itself (b == 1, root_is_c) its derivative is 1 by c and 0 by u, without the root and the division.
+// The two forms round differently, so each lane's own values choose (no vote of the warp): a cell's
+// gradient does not depend on its neighbours in the warp.
 SW2D_HD void root_rev(double b, double u, double c, double root_bar, double& u_bar, double& c_bar)
 {
-    if (warp_all(root_is_c(b, u, c))) {
+    if (root_is_c(b, u, c)) {
         c_bar = c > 0.0 ? root_bar : 0.0;
         return;
     }

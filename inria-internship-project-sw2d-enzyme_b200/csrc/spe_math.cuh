@@ -75,8 +75,9 @@ SW2D_HD void lam_rev(double b, double c, double u, double lmb, double lpb, doubl
 {
     ub += b * (lmb + lpb);
     const double Rb = lpb - lmb;
-    // b == 1: the root is c itself (sp_math.cuh, root_is_c), its derivative 1 by c and 0 by u
-    if (warp_all(root_is_c(b, u, c) && c > 0.0)) {
+    // b == 1: the root is c itself (sp_math.cuh, root_is_c), its derivative 1 by c and 0 by u; the
+    // lane's own values choose, as in root_rev (sp_adjoint.cuh)
+    if (root_is_c(b, u, c) && c > 0.0) {
         cb += Rb;
         return;
     }
