@@ -181,8 +181,9 @@ SW2D_HD void hllc_rev(bool blending, double bL, double bR, double phiL, double p
         const double duR = blending ? smax(hR, kSmallReal) : smax(kSmallReal, hR);
         const bool duL_h = blending ? !(hL < kSmallReal) : (kSmallReal < hL);
         const bool duR_h = blending ? !(hR < kSmallReal) : (kSmallReal < hR);
-        // the reciprocal of each denominator, taken once (the sign of f1, the one branch that depends on
-        // a quotient, is its numerator's); max(h, small) is one value for u and v
+        // the reciprocal of each denominator, taken once; max(h, small) is one value for u and v.  The one
+        // branch that depends on a quotient is the sign of f1: without blending its numerator's, with it
+        // that of a sum of two quotients, which are the forward's divisions (tests/adjoint_side_check.cpp)
         const double rL = 1.0 / duL, rR = 1.0 / duR;
         const double uL = L.q * rL, uR = R.q * rR;
         const double mR = smin(R.lm, 0.);
@@ -204,8 +205,8 @@ SW2D_HD void hllc_rev(bool blending, double bL, double bR, double phiL, double p
                 alpha = smax(0.0, inner);
                 alpha_free = (0.0 < inner) && (ratio < 1.0);
             }
-            F1h = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (hR - hL)) * rden;
-            F1z = phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)) * rden;
+            F1h = sw2d_div(phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (hR - hL)), den);
+            F1z = sw2d_div(phiLR * (L2 * L.q - L1 * R.q + L1 * L2 * (R.z - L.z)), den);
             f1 = alpha * F1h + (1.0 - alpha) * F1z;
             s2z = (phiR * hR * hR - phiL * hL * hL) * 0.5 + fact * (L.z - R.z);
             s2h = (zbL > zbR) ? phiR * hR * (zbL - zbR) : phiL * hL * (zbL - zbR);
