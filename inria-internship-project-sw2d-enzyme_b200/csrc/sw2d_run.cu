@@ -590,7 +590,8 @@ RunLayout run_layout(const TileMesh& tm, bool muscl, bool dip, bool friction)
     sec(&o.elen, 8 * ne);
     sec(&o.esl, 8 * ne);
     sec(&o.epg, dip ? 8 * ne : 0);
-    sec(&o.eg, muscl ? 32 * na : 0);
+    // at least one record: the pairs' slopes read the first one where a cell has fewer neighbours
+    sec(&o.eg, muscl ? 32 * std::max<size_t>(na, 1) : 0);
     sec(&o.ell, 4 * na);
     sec(&o.ent, muscl ? 4 * (size_t)tm.nent_max : 0);
     sec(&o.so, muscl ? 4 * (nf + 1) : 0);
