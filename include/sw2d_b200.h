@@ -455,15 +455,22 @@ const char* sw2d_phase_name(int i);
  * instead of recomputing them: this many at most, and what an eighth of the free device memory
  * and, over all handles, 1/32 of the device's holds (the default).  The same bits either way.  Takes effect at the next sw2d_record.
  * "run_kernel" (0/1, default 1): sw2d_step_n and sw2d_execute take the steps of a small SP or DIP
- * mesh (one whose cells fit the chip's shared memory) in one launch; 0 takes them kernel by kernel.
+ * mesh (one whose cells fit the chip's shared memory) in one launch; 0 takes them kernel by kernel, as
+ * is done where there is no memory for the mesh's tiles.  "run_steps" (read only): steps taken so.
  * "run_wait_polls": the poll limit of that launch's waits, after which it gives up with an error
  * status (negative: the default).
  * "adjoint_trace" (0/1): record the state adjoint's magnitude per reverse step
  * (sw2d_adjoint_trace). */
 int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value);
 /* Current value of "fused_step", "flux_variant", "tile_cells" (0 without tiles),
- * "record_fluxes" or "record_wave_speeds".  No counterpart in the reference. */
+ * "record_fluxes", "record_wave_speeds", "run_kernel" or "run_steps".  No counterpart in the
+ * reference. */
 int sw2d_get_option(sw2d_handle* h, const char* name, int64_t* value);
+
+/* For tests: of the memory requests (device and pinned) that the library makes next in the calling
+ * thread, the first `skip` are served and the `count` after them fail, as on a full device.  Returns
+ * how many requests the thread has made since the last call of this function. */
+int64_t sw2d_test_fail_allocations(int64_t skip, int64_t count);
 
 /* Launch-configuration autotuner (no counterpart in the reference): times every
  * {threads per block, register cap} variant of the kernels of the handle's current step form

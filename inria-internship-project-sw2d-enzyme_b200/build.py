@@ -16,7 +16,7 @@ LIBDIR = os.path.join(HERE, "lib")
 SOURCES = ["sw2d_sp.cu", "sw2d_tile.cu", "sw2d_run.cu", "sw2d_queue.cu", "sw2d_adjoint.cu", "sw2d_batch.cu", "sw2d_assim.cu", "sw2d_ddp.cu", "sw2d_case.cpp", "sw2d_mlp.cu",
            "sw2d_result.cu", "sw2d_mapper.cu"]
 HEADERS = ["sw2d_internal.cuh", "sp_math.cuh", "dip_math.cuh", "sp_adjoint.cuh", "portable_math.h", "adjoint_common.cuh",
-           "spe_math.cuh", "ddp_math.cuh", "umma.cuh", "sp_phases.cuh", "tile_phases.cuh"]
+           "spe_math.cuh", "ddp_math.cuh", "umma.cuh", "device_memory.cuh", "sp_phases.cuh", "tile_phases.cuh"]
 OUT = os.path.join(LIBDIR, "libsw2d_b200.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-fmad=false",

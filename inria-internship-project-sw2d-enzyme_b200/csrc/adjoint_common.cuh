@@ -231,7 +231,7 @@ template <class T>
 int adj_alloc(sw2d_handle* h, std::vector<void*>& list, size_t n, T** out)
 {
     void* p = nullptr;
-    CK(cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(T)));
+    CK(device_malloc(&p, std::max<size_t>(1, n) * sizeof(T)));
     list.push_back(p);
     CK(cudaMemsetAsync(p, 0, std::max<size_t>(1, n) * sizeof(T), h->stream));
     *out = static_cast<T*>(p);

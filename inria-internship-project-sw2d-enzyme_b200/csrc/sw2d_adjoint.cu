@@ -918,7 +918,7 @@ int reverse_sweep(sw2d_handle* h, int64_t kept)
         if (a->trace_steps != a->n_steps) {
             cudaFree(a->d_trace);
             a->d_trace = nullptr;
-            CK(cudaMalloc(&a->d_trace, 4 * a->n_steps * sizeof(unsigned long long)));
+            CK(device_malloc(&a->d_trace, 4 * a->n_steps * sizeof(unsigned long long)));
             a->trace_steps = a->n_steps;
         }
         std::vector<unsigned long long> init(4 * a->n_steps, 0ull);

@@ -897,10 +897,10 @@ int ensure_steps(sw2d_handle* h, int64_t need)
     int64_t cap = std::max<int64_t>(need, 2 * a->cap + 1024);
     double *dt = nullptr, *t = nullptr, *cost = nullptr;
     int* tr = nullptr;
-    CK(cudaMalloc(&dt, cap * sizeof(double)));
-    CK(cudaMalloc(&t, cap * sizeof(double)));
-    CK(cudaMalloc(&cost, cap * sizeof(double)));
-    CK(cudaMalloc(&tr, cap * sizeof(int)));
+    CK(device_malloc(&dt, cap * sizeof(double)));
+    CK(device_malloc(&t, cap * sizeof(double)));
+    CK(device_malloc(&cost, cap * sizeof(double)));
+    CK(device_malloc(&tr, cap * sizeof(int)));
     if (a->cap > 0) {
         CK(cudaMemcpyAsync(dt, a->d_dt, a->cap * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
         CK(cudaMemcpyAsync(t, a->d_t, a->cap * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
@@ -941,7 +941,7 @@ int take_checkpoint(sw2d_handle* h, double4** out)
         a->ck_spare.pop_back();
         return SW2D_OK;
     }
-    CK(cudaMalloc(out, std::max<int64_t>(1, h->nc) * sizeof(double4)));
+    CK(device_malloc(out, std::max<int64_t>(1, h->nc) * sizeof(double4)));
     return SW2D_OK;
 }
 

@@ -331,7 +331,7 @@ int sw2d_batch_autotune(sw2d_batch* b, int steps, const int* tile_sizes, int n_t
         BCK(cudaStreamSynchronize(h->stream));
         st_bytes[i] = (size_t)h->nc * sizeof(double4);
         sl_bytes[i] = (size_t)h->h_coff.back().y * sizeof(Slot);
-        if (cudaMalloc(&saved[i], st_bytes[i] + sl_bytes[i] + sizeof(Ctrl)) != cudaSuccess) {
+        if (device_malloc(&saved[i], st_bytes[i] + sl_bytes[i] + sizeof(Ctrl)) != cudaSuccess) {
             release();
             return bfail(b, SW2D_E_CUDA, "autotune: no memory for the members' saved states");
         }

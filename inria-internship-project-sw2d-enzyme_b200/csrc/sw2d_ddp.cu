@@ -1246,7 +1246,7 @@ int ddp_setup(sw2d_handle* h, const sw2d_mesh* mesh, const sw2d_cell_fields* fie
     CK(cudaGetLastError());
     // initial conditions from the caller's arrays
     double* tmp = nullptr;
-    CK(cudaMalloc(&tmp, 3 * std::max<int64_t>(1, nc) * sizeof(double)));
+    CK(device_malloc(&tmp, 3 * std::max<int64_t>(1, nc) * sizeof(double)));
     cudaError_t ce = cudaMemcpyAsync(tmp, ic_level, nc * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(tmp + nc, ic_x, nc * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     if (ce == cudaSuccess)
@@ -1287,7 +1287,7 @@ int64_t ddp_get_array(sw2d_handle* h, const char* name, double* out, int64_t cap
     CK(cudaSetDevice(h->device));
     DdpState* d = h->ddp;
     const int64_t span = std::max<int64_t>(1, std::max(h->nc, h->ni));
-    if (!d->outbuf) CK(cudaMalloc(&d->outbuf, 5 * span * sizeof(double)));
+    if (!d->outbuf) CK(device_malloc(&d->outbuf, 5 * span * sizeof(double)));
     double* stage = d->outbuf + 4 * span;
     if (hmin) {
         k_scatter_field<<<grid_for(h->ni), kBlock, 0, h->stream>>>(reinterpret_cast<const double*>(h->m.des), 8, 0,

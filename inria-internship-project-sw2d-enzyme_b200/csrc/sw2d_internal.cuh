@@ -13,6 +13,7 @@
 #include "../../include/sw2d_b200.h"
 #include "dip_math.cuh"
 #include "ddp_math.cuh"
+#include "device_memory.cuh"
 
 namespace sw2d {
 
@@ -351,6 +352,7 @@ struct sw2d_handle {
     sw2d::RunState* run = nullptr;      // run kernel of small meshes
     int run_kernel = 1;                 // option "run_kernel"
     int64_t run_polls = -1;             // option "run_wait_polls" (< 0: the default)
+    int64_t run_taken = 0;              // steps the run kernel has taken (option "run_steps")
     std::string err;
 };
 
@@ -373,7 +375,7 @@ int dev_upload(sw2d_handle* h, const std::vector<T>& v, T** out)
 {
     size_t bytes = std::max<size_t>(1, v.size()) * sizeof(T);
     void* p = nullptr;
-    CK(cudaMalloc(&p, bytes));
+    CK(device_malloc(&p, bytes));
     h->allocs.push_back(p);
     if (!v.empty()) CK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
     *out = static_cast<T*>(p);
@@ -384,7 +386,7 @@ template <class T>
 int dev_alloc(sw2d_handle* h, size_t n, T** out)
 {
     void* p = nullptr;
-    CK(cudaMalloc(&p, std::max<size_t>(1, n) * sizeof(T)));
+    CK(device_malloc(&p, std::max<size_t>(1, n) * sizeof(T)));
     h->allocs.push_back(p);
     CK(cudaMemsetAsync(p, 0, std::max<size_t>(1, n) * sizeof(T), h->stream));
     *out = static_cast<T*>(p);
@@ -431,9 +433,11 @@ int tiles_make(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<
                std::vector<void*>& allocs, std::string& why);
 
 // The run kernel of small meshes (sw2d_run.cu): whether the handle's next steps may take it (its
-// tiles are built the first time), the launches of n steps, the release.
+// tiles are built the first time), the launches of n steps, another try at tiles that found no memory,
+// the release.
 int run_ready(sw2d_handle* h, bool* ready);
 int run_steps(sw2d_handle* h, int64_t n);
+void run_retry(sw2d_handle* h);
 void run_release(sw2d_handle* h);
 
 // The CFL kernel with the DDP model's map-storage snap (swDdpHyp.cpp:588-600).

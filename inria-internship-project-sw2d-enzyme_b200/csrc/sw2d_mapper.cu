@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/sw2d_b200.h"
+#include "device_memory.cuh"
 
 namespace {
 
@@ -449,7 +450,7 @@ struct DevBuf {
     cudaError_t up(const T* src, size_t n, T** dst)
     {
         void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+        cudaError_t e = sw2d::device_malloc(&q, std::max<size_t>(n, 1) * sizeof(T));
         if (e != cudaSuccess) return e;
         p.push_back(q);
         *dst = static_cast<T*>(q);

@@ -278,7 +278,7 @@ template <class T>
 int malloc_dev(sw2d_mlp* m, size_t n, T** p)
 {
     void* q = nullptr;
-    MCK(cudaMalloc(&q, std::max<size_t>(1, n) * sizeof(T)));
+    MCK(sw2d::device_malloc(&q, std::max<size_t>(1, n) * sizeof(T)));
     m->allocs.push_back(q);
     MCK(cudaMemsetAsync(q, 0, std::max<size_t>(1, n) * sizeof(T), m->stream));
     *p = static_cast<T*>(q);
@@ -713,7 +713,7 @@ int ensure_train(sw2d_mlp* m, int64_t n)
     int rc;
     if (m->host) MCK(cudaFreeHost(m->host));
     m->host = nullptr;
-    MCK(cudaMallocHost(&m->host, result_floats(n) * sizeof(float)));
+    MCK(sw2d::pinned_malloc(&m->host, result_floats(n) * sizeof(float)));
     float* grad = nullptr;
     const int64_t parts = std::min<int64_t>((n + kTileM - 1) / kTileM, m->sms);  // one per CTA
     if (parts > m->parts) {
@@ -1323,7 +1323,7 @@ int closure_record(sw2d_handle* h, int on)
     if (on && !c->rec) {
         void* p = nullptr;
         const size_t bytes = (size_t)std::max<int64_t>(h->nc, 1) * kRec * sizeof(float);
-        if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(h, SW2D_E_CUDA, "closure record buffer");
+        if (device_malloc(&p, bytes) != cudaSuccess) return fail(h, SW2D_E_CUDA, "closure record buffer");
         c->allocs.push_back(p);
         if (cudaMemset(p, 0, bytes) != cudaSuccess) return fail(h, SW2D_E_CUDA, "closure record buffer");
         c->rec = static_cast<float*>(p);
@@ -1363,7 +1363,7 @@ int sw2d_set_closure(sw2d_handle* h, sw2d_mlp* net, const float* hull_lo, const 
     std::memcpy(c->hi, hull_hi, sizeof(c->hi));
     c->scale = scale;
     void* p = nullptr;
-    if (cudaMalloc(&p, (size_t)std::max<int64_t>(h->nc, 1) * sizeof(float)) != cudaSuccess) {
+    if (device_malloc(&p, (size_t)std::max<int64_t>(h->nc, 1) * sizeof(float)) != cudaSuccess) {
         closure_free(c);
         return fail(h, SW2D_E_CUDA, "closure buffers");
     }

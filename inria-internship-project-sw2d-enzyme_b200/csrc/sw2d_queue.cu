@@ -361,11 +361,11 @@ int queue_build(QueueState*& q, sw2d_handle* const* members, int n, int variant,
     q->d_dmin = nullptr;
     q->d_items = nullptr;
     q->n = n;
-    cudaError_t e = cudaMalloc(&q->d_mem, n * sizeof(QMember));
-    if (e == cudaSuccess) e = cudaMalloc(&q->d_sync, n * sizeof(QSync));
-    if (e == cudaSuccess) e = cudaMalloc(&q->d_dmin, n * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&q->d_items, items.size() * sizeof(unsigned));
-    if (e == cudaSuccess && !q->d_next) e = cudaMalloc(&q->d_next, 2 * sizeof(unsigned));
+    cudaError_t e = device_malloc(&q->d_mem, n * sizeof(QMember));
+    if (e == cudaSuccess) e = device_malloc(&q->d_sync, n * sizeof(QSync));
+    if (e == cudaSuccess) e = device_malloc(&q->d_dmin, n * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = device_malloc(&q->d_items, items.size() * sizeof(unsigned));
+    if (e == cudaSuccess && !q->d_next) e = device_malloc(&q->d_next, 2 * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemcpy(q->d_mem, q->h_mem.data(), n * sizeof(QMember), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(q->d_items, items.data(), items.size() * sizeof(unsigned), cudaMemcpyHostToDevice);

@@ -474,14 +474,14 @@ int sw2d_result_open(sw2d_handle* h, const char* path, const char* geometry_path
     }
     cudaError_t e = cudaSuccess;
     if (mode != SW2D_RESULT_NONE) {
-        e = cudaMalloc(&w->d_ring, (size_t)w->ring * (size_t)frame_bytes);
-        if (e == cudaSuccess) e = cudaMalloc(&w->d_fc, sizeof(FrameCtl));
+        e = device_malloc(&w->d_ring, (size_t)w->ring * (size_t)frame_bytes);
+        if (e == cudaSuccess) e = device_malloc(&w->d_fc, sizeof(FrameCtl));
         if (e == cudaSuccess) e = cudaMemset(w->d_fc, 0, sizeof(FrameCtl));
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->cs, cudaStreamNonBlocking);
         w->host.assign(w->ring, nullptr);
         w->ev.assign(w->ring, nullptr);
         for (int s = 0; s < w->ring && e == cudaSuccess; s++) {
-            e = cudaMallocHost(&w->host[s], (size_t)frame_bytes);
+            e = pinned_malloc(&w->host[s], (size_t)frame_bytes);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->ev[s], cudaEventDisableTiming);
         }
     }

@@ -625,6 +625,15 @@ constexpr int64_t kRunCellsMax = 66000;  // above it no tile fits (see the figur
 constexpr int kRunTileLeast = 64;
 constexpr int kRunSmemMax = 220 * 1024;
 
+void run_free(RunState* r)
+{
+    for (void* p : r->tile_allocs) cudaFree(p);
+    r->tile_allocs.clear();
+    for (void* p : r->allocs) cudaFree(p);
+    r->allocs.clear();
+}
+
+// The tiles and words of a handle's run kernel; RunState.ok tells whether they fit the chip
 int run_build(sw2d_handle* h)
 {
     RunState* r = h->run = new RunState();
@@ -636,8 +645,7 @@ int run_build(sw2d_handle* h)
     const int tile = (int)std::max<int64_t>(kRunTileLeast, (h->nc + h->sms - 1) / h->sms);
     std::string why;
     const int rc = tiles_make(h, h->h_coff, h->h_cint, h->h_lr, h->h_bcell, tile, true, 1, r->tm, r->tile_allocs, why);
-    if (rc == SW2D_E_UNSUPPORTED) return SW2D_OK;
-    if (rc) return fail(h, rc, why.empty() ? h->err : why);
+    if (rc) return rc;
     const bool muscl = h->p.scheme == SW2D_SCHEME_MUSCL_EVR;
     r->lay = run_layout(r->tm, muscl, h->model == kModelDip, h->p.friction != SW2D_FRICTION_NONE);
     if (r->lay.smem > kRunSmemMax) return SW2D_OK;
@@ -650,7 +658,7 @@ int run_build(sw2d_handle* h)
     if (per_sm < 1 || (int64_t)per_sm * h->sms < r->tm.ntiles) return SW2D_OK;
     auto alloc = [&](size_t n, ulonglong2** p) -> int {
         void* q = nullptr;
-        CK(cudaMalloc(&q, n * sizeof(ulonglong2)));
+        CK(device_malloc(&q, n * sizeof(ulonglong2)));
         r->allocs.push_back(q);
         CK(cudaMemsetAsync(q, 0, n * sizeof(ulonglong2), h->stream));
         *p = static_cast<ulonglong2*>(q);
@@ -671,11 +679,12 @@ int run_ready(sw2d_handle* h, bool* ready)
     if (!h->run_kernel || h->model == kModelDdp || h->fused || h->closure || h->result || h->nc > kRunCellsMax) return SW2D_OK;
     if (h->m.lmax || h->m.lmaxb || h->m.flux || h->m.bflux) return SW2D_OK;  // recorded by the step's kernels
     if (!h->run) {
-        const int rc = run_build(h);
-        if (rc) {
-            run_release(h);
-            return rc;
+        // no memory for the tiles (or no kernel to hold them): the step's kernels need none of it and serve
+        if (run_build(h) != SW2D_OK) {
+            cudaGetLastError();
+            h->err.clear();
         }
+        if (!h->run->ok) run_free(h->run);
     }
     *ready = h->run->ok;
     return SW2D_OK;
@@ -710,11 +719,15 @@ int run_steps(sw2d_handle* h, int64_t n)
     return SW2D_OK;
 }
 
+void run_retry(sw2d_handle* h)
+{
+    if (h->run && !h->run->ok) run_release(h);
+}
+
 void run_release(sw2d_handle* h)
 {
     if (!h->run) return;
-    for (void* p : h->run->tile_allocs) cudaFree(p);
-    for (void* p : h->run->allocs) cudaFree(p);
+    run_free(h->run);
     delete h->run;
     h->run = nullptr;
 }

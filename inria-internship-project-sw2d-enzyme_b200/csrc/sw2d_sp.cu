@@ -925,9 +925,9 @@ int create_model(const sw2d_mesh* mesh, const sw2d_params* params, const sw2d_ce
         volatile double c0 = m.dry.c0;
         m.dry.r0 = std::sqrt(c0 * c0);
     }
-    if (cudaMalloc(&h->ctrl, sizeof(Ctrl)) != cudaSuccess) return bail(fail(h, SW2D_E_CUDA, "cudaMalloc ctrl"));
+    if (device_malloc(&h->ctrl, sizeof(Ctrl)) != cudaSuccess) return bail(fail(h, SW2D_E_CUDA, "cudaMalloc ctrl"));
     h->allocs.push_back(h->ctrl);
-    if (cudaMallocHost(&h->ctrl_host, 2 * sizeof(Ctrl)) != cudaSuccess) return bail(fail(h, SW2D_E_CUDA, "cudaMallocHost"));
+    if (pinned_malloc(&h->ctrl_host, 2 * sizeof(Ctrl)) != cudaSuccess) return bail(fail(h, SW2D_E_CUDA, "cudaMallocHost"));
     m.ctrl = h->ctrl;
     Ctrl c0{};
     c0.t = params->t_0;
@@ -991,6 +991,7 @@ int sw2d_step_n(sw2d_handle* h, int64_t n_steps, int64_t* steps_done)
         if (const int rc = run_steps(h, n_steps)) return rc;
         CK(cudaMemcpyAsync(host, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
+        h->run_taken += host[0].steps - host[1].steps;
         if (steps_done) *steps_done = host[0].steps - host[1].steps;
         return status_to_code(h, host[0].status);
     }
@@ -1520,8 +1521,10 @@ int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value)
         h->m.rev_update = value ? 1 : 0;
     } else if (std::strcmp(name, "run_kernel") == 0) {
         // 1 (default): sw2d_step_n and sw2d_execute take the steps of a small SP or DIP mesh in one
-        // launch (sw2d_run.cu); 0: by the step's kernels (the same results)
+        // launch (sw2d_run.cu); 0: by the step's kernels (the same results).  Set again, it also
+        // tries again for a mesh that found no memory for its tiles.
         h->run_kernel = value ? 1 : 0;
+        run_retry(h);
     } else if (std::strcmp(name, "run_wait_polls") == 0) {
         // poll limit of the run kernel's waits (< 0: the default)
         h->run_polls = value;
@@ -1544,12 +1547,21 @@ int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value)
     return SW2D_OK;
 }
 
+int64_t sw2d_test_fail_allocations(int64_t skip, int64_t count)
+{
+    AllocationFaults& f = allocation_faults();
+    const int64_t seen = f.seen;
+    f = AllocationFaults{skip, count, 0};
+    return seen;
+}
+
 int sw2d_get_option(sw2d_handle* h, const char* name, int64_t* value)
 {
     if (!h || !name || !value) return fail(h, SW2D_E_ARG, "invalid arguments");
     if (std::strcmp(name, "fused_step") == 0) *value = h->fused;
     else if (std::strcmp(name, "flux_variant") == 0) *value = h->flux_variant;
     else if (std::strcmp(name, "run_kernel") == 0) *value = h->run_kernel;
+    else if (std::strcmp(name, "run_steps") == 0) *value = h->run_taken;
     else if (std::strcmp(name, "update_reverse") == 0) *value = h->m.rev_update;
     else if (std::strcmp(name, "fused_slopes") == 0) *value = h->fused_slopes;
     else if (std::strcmp(name, "tile_cells") == 0) *value = h->tiles.tile_cells;
@@ -1621,7 +1633,7 @@ int sw2d_save_point(sw2d_handle* h)
     CK(cudaSetDevice(h->device));
     size_t st, sl;
     const size_t bytes = point_bytes(h, &st, &sl);
-    if (!h->saved_point) CK(cudaMalloc(&h->saved_point, bytes));
+    if (!h->saved_point) CK(device_malloc(&h->saved_point, bytes));
     char* d = static_cast<char*>(h->saved_point);
     CK(cudaMemcpyAsync(d, h->m.st, st, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(d + st, h->m.slot, sl, cudaMemcpyDeviceToDevice, h->stream));
@@ -1720,7 +1732,7 @@ int64_t sw2d_get_array(sw2d_handle* h, const char* name, double* out, int64_t ca
         if (capacity < e.len) return fail(h, SW2D_E_ARG, "output buffer too small");
         CK(cudaSetDevice(h->device));
         double* tmp = nullptr;
-        CK(cudaMalloc(&tmp, std::max<int64_t>(1, e.len) * sizeof(double)));
+        CK(device_malloc(&tmp, std::max<int64_t>(1, e.len) * sizeof(double)));
         k_scatter_strided<<<grid_for(e.len), kBlock, 0, h->stream>>>(e.p, e.stride, e.offset, e.perm, tmp, (int)e.len);
         cudaError_t ce = cudaMemcpyAsync(out, tmp, e.len * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
         cudaStreamSynchronize(h->stream);
@@ -1884,8 +1896,8 @@ int sw2d_eval_math(int device, int fn, const double* x, double* y, int64_t n)
         return fail(h, SW2D_E_NO_DEVICE, "no usable CUDA device");
     CK(cudaSetDevice(device));
     double *dx = nullptr, *dy = nullptr;
-    CK(cudaMalloc(&dx, std::max<int64_t>(1, n) * sizeof(double)));
-    if (cudaMalloc(&dy, std::max<int64_t>(1, n) * sizeof(double)) != cudaSuccess) {
+    CK(device_malloc(&dx, std::max<int64_t>(1, n) * sizeof(double)));
+    if (device_malloc(&dy, std::max<int64_t>(1, n) * sizeof(double)) != cudaSuccess) {
         cudaFree(dx);
         return fail(h, SW2D_E_CUDA, "cudaMalloc");
     }

@@ -657,7 +657,7 @@ int tiles_make(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<
         using T = typename std::remove_reference<decltype(vec)>::type::value_type;
         void* p = nullptr;
         const size_t bytes = std::max<size_t>(1, vec.size()) * sizeof(T);
-        if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(h, SW2D_E_CUDA, "cudaMalloc (tiles)");
+        if (device_malloc(&p, bytes) != cudaSuccess) return fail(h, SW2D_E_CUDA, "cudaMalloc (tiles)");
         allocs.push_back(p);
         if (!vec.empty() && cudaMemcpyAsync(p, vec.data(), vec.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream) !=
                                 cudaSuccess)

@@ -54,3 +54,57 @@ def test_cells_without_internal_edges(pkg, n, scheme, friction):
         assert _same_state(a, oracle) and _same_state(b, oracle) and a.time == b.time
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("scheme", ["muscl_evr", "godunov"])
+def test_no_memory_for_the_tiles(pkg, scheme):
+    """Each of the run kernel's allocations fails in turn: the step's kernels take the steps, no error
+    stays behind, and the option set again tries again."""
+    case = pkg.workloads.dam_break(n_cells=3000, scheme=scheme)
+    want = pkg.SpModel(case)
+    fails = want.lib.sw2d_test_fail_allocations
+    fails(0, 0)
+    want.set_option("run_kernel", 1)
+    want.step(40)
+    n = fails(0, 0)
+    assert n > 0 and want.get_option("run_steps") == 40
+    for skip in range(n):
+        m = pkg.SpModel(case)
+        m.set_option("run_kernel", 1)
+        fails(skip, 1)
+        try:
+            assert m.step(40) == 40
+        finally:
+            fails(0, 0)
+        assert m.get_option("run_steps") == 0 and _same_state(m, want) and m.time == want.time
+        m.prepare()
+        assert m.step(1) == 1 and m.get_option("run_steps") == 0
+        m.set_option("run_kernel", 1)
+        m.step(3)
+        assert m.get_option("run_steps") == 3
+        m.close()
+    want.step(4)
+    assert want.lib.sw2d_last_error(want.handle) == b""
+    want.close()
+
+
+def test_tiles_that_do_not_fit_hold_no_memory(pkg):
+    """Under the size limit the tiles are built before their shared memory turns out too large (cells of
+    six neighbours)."""
+    import torch
+
+    from tests.test_gpu_polygons import _case, merged_mesh
+
+    case = _case(pkg, merged_mesh(pkg, 720, 170, 72.0, 34.0, 2))
+    assert 60000 < case.mesh.cell_nb <= 66000
+    m = pkg.SpModel(case)
+    torch.cuda.synchronize()
+    m.set_option("run_kernel", 1)
+    m.set_option("run_kernel", 0)
+    m.step(40)                       # graph and modules
+    free0 = torch.cuda.mem_get_info(0)[0]
+    m.set_option("run_kernel", 1)
+    m.step(40)
+    assert m.get_option("run_steps") == 0
+    assert torch.cuda.mem_get_info(0)[0] == free0
+    m.close()
