@@ -33,16 +33,24 @@ inline size_t request_bytes(size_t bytes)
     return kNoDeviceHolds;
 }
 
+// The error of a request that failed goes to the caller and is not left behind as CUDA's last error,
+// where the next launch's check would find it although the caller did without the memory.
+inline cudaError_t taken(cudaError_t e)
+{
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
 template <class T>
 cudaError_t device_malloc(T** p, size_t bytes)
 {
-    return cudaMalloc(p, request_bytes(bytes));
+    return taken(cudaMalloc(p, request_bytes(bytes)));
 }
 
 template <class T>
 cudaError_t pinned_malloc(T** p, size_t bytes)
 {
-    return cudaMallocHost(p, request_bytes(bytes));
+    return taken(cudaMallocHost(p, request_bytes(bytes)));
 }
 
 }  // namespace sw2d

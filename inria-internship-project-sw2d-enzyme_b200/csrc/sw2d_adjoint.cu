@@ -1057,7 +1057,6 @@ void more_segments(sw2d_handle* h, int64_t seg)
     if (adj_alloc(h, L, n * (seg + 1) * nc, &a->more_st) || adj_alloc(h, L, n * seg * nc, &a->more_bal) ||
         (a->seg_slope && adj_alloc(h, L, n * seg * nc, &a->more_slope)) ||
         adj_alloc(h, L, n * seg * h->ni * 5, &a->more_rs)) {
-        cudaGetLastError();
         drop_more(a);
         h->err.clear();
         return;
@@ -1096,7 +1095,6 @@ int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
             a->n_steps = 0;
             return rc;
         }
-        cudaGetLastError();
         h->err.clear();
     }
     // each step's slopes and Riemann states, kept by the segment's forward recompute for the
