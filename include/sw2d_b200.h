@@ -452,8 +452,12 @@ const char* sw2d_phase_name(int i);
  * Riemann states for the reverse steps when they fit in half of the free device memory.
  * "adjoint_kept_segments" (at least 1): sw2d_adjoint on a trajectory whose checkpoints a change of
  * the parameters has outdated runs it first, and keeps the steps of its last segments meanwhile
- * instead of recomputing them: this many at most, and what an eighth of the free device memory
- * and, over all handles, 1/32 of the device's holds (the default).  The same bits either way.  Takes effect at the next sw2d_record.
+ * instead of recomputing them: this many at most, and what an eighth of the free device memory holds
+ * (the default).  The same bits either way.  Takes effect at the next sw2d_record, which allocates
+ * and clears the memory.  This memory and that of the slopes which sw2d_assim_gradient keeps is at
+ * most 1/32 of the device's over all handles, and any allocation of the library that finds the device
+ * full takes it back from the handles not using it; their next gradients take it again, or recompute.
+ * "kept_bytes" (read only): what the handle holds of it.
  * "run_kernel" (0/1, default 1): sw2d_step_n and sw2d_execute take the steps of a small SP or DIP
  * mesh (one whose cells fit the chip's shared memory) in one launch; 0 takes them kernel by kernel, as
  * is done where there is no memory for the mesh's tiles.  "run_steps" (read only): steps taken so.
@@ -463,8 +467,8 @@ const char* sw2d_phase_name(int i);
  * (sw2d_adjoint_trace). */
 int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value);
 /* Current value of "fused_step", "flux_variant", "tile_cells" (0 without tiles),
- * "record_fluxes", "record_wave_speeds", "run_kernel" or "run_steps".  No counterpart in the
- * reference. */
+ * "record_fluxes", "record_wave_speeds", "run_kernel", "run_steps" or "kept_bytes".  No counterpart
+ * in the reference. */
 int sw2d_get_option(sw2d_handle* h, const char* name, int64_t* value);
 
 /* For tests: of the memory requests (device and pinned) that the library makes next in the calling

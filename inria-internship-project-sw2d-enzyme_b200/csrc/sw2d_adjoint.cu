@@ -40,7 +40,6 @@
 
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -75,9 +74,13 @@ struct AdjointState {
     double2* seg_rs = nullptr;           // every * ni * 5: each step's Riemann states (when memory allows)
     double4 *more_st = nullptr, *more_bal = nullptr;  // the buffers after the first
     double2 *more_slope = nullptr, *more_rs = nullptr;
-    std::vector<void*> more_allocs;
-    size_t more_bytes = 0;
-    bool more_busy = false;              // a gradient is using them
+    OptionalMemory more{this, [](void* a) { static_cast<AdjointState*>(a)->forget_more(); }};
+    void forget_more()
+    {
+        more_st = more_bal = nullptr;
+        more_slope = more_rs = nullptr;
+        n_seg = 1;
+    }
     double2* eside = nullptr;            // 3 * ni: {z_b}, {b}, {phi} of each internal edge's (L, R) cells
     // adjoint buffers
     double4* lam = nullptr;              // nc: adjoint of the state {h, q, r, -}
@@ -984,97 +987,36 @@ int reverse_sweep(sw2d_handle* h, int64_t kept)
     return SW2D_OK;
 }
 
-// The handles that hold buffers for more segments than the first, and the bytes of them all: at most
-// 1/32 of the device's memory, so that ensembles of handles leave each other room, and given back
-// when a trajectory's own arrays find none.
-struct MorePool {
-    std::mutex mu;
-    std::vector<AdjointState*> holders;
-    size_t bytes = 0;
-};
-MorePool& more_pool()
-{
-    static MorePool* p = new MorePool;
-    return *p;
-}
-
-// with the pool's mutex held
-void drop_more(AdjointState* a)
-{
-    MorePool& p = more_pool();
-    free_list(a->more_allocs);
-    p.bytes -= a->more_bytes;
-    p.holders.erase(std::remove(p.holders.begin(), p.holders.end(), a), p.holders.end());
-    a->more_bytes = 0;
-    a->more_st = a->more_bal = nullptr;
-    a->more_slope = a->more_rs = nullptr;
-    a->n_seg = 1;
-}
-
-// frees the buffers that no gradient is using; whether there were any
-bool give_back_more()
-{
-    MorePool& p = more_pool();
-    std::lock_guard<std::mutex> lock(p.mu);
-    const std::vector<AdjointState*> all = p.holders;
-    bool any = false;
-    for (AdjointState* a : all)
-        if (!a->more_busy) {
-            drop_more(a);
-            any = true;
-        }
-    return any;
-}
-
-// keeps a handle's buffers from being given back meanwhile
-struct MoreUse {
-    AdjointState* a;
-    explicit MoreUse(AdjointState* a_) : a(a_) { set(true); }
-    ~MoreUse() { set(false); }
-    void set(bool on)
-    {
-        std::lock_guard<std::mutex> lock(more_pool().mu);
-        a->more_busy = on;
-    }
-};
-
 // Buffers for more of the trajectory's last segments (each costs what the first one does): as many
-// as an eighth of the free device memory and the pool's share hold
-void more_segments(sw2d_handle* h, int64_t seg)
+// as an eighth of the free device memory and the share of all handles (OptionalMemory) hold
+int more_segments(sw2d_handle* h)
 {
     AdjointState* a = h->adj;
-    const int64_t nc = h->nc;
-    MorePool& p = more_pool();
-    std::lock_guard<std::mutex> lock(p.mu);
-    size_t free_b = 0, total_b = 0;
-    if (!a->seg_rs || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return;
-    const size_t one = (size_t)(2 * seg + 1) * nc * sizeof(double4) +
-                       (size_t)seg * ((a->seg_slope ? nc : 0) + 5 * h->ni) * sizeof(double2);
-    const size_t share = std::min(free_b / 8, total_b / 32 - std::min(p.bytes, total_b / 32));
-    const int64_t n = std::min({a->n_ck - 1, (int64_t)(share / one), h->adj_kept_segments - 1});
-    if (n <= 0) return;
-    std::vector<void*>& L = a->more_allocs;
-    if (adj_alloc(h, L, n * (seg + 1) * nc, &a->more_st) || adj_alloc(h, L, n * seg * nc, &a->more_bal) ||
-        (a->seg_slope && adj_alloc(h, L, n * seg * nc, &a->more_slope)) ||
-        adj_alloc(h, L, n * seg * h->ni * 5, &a->more_rs)) {
-        drop_more(a);
-        h->err.clear();
-        return;
-    }
-    p.holders.push_back(a);
-    a->more_bytes = n * one;
-    p.bytes += a->more_bytes;
+    const size_t nc = h->nc, ni = h->ni, seg = std::min(a->every, a->n_requested);
+    const size_t st = sizeof(double4) * nc, sl = a->seg_slope ? sizeof(double2) * nc : 0, rs = 5 * sizeof(double2) * ni;
+    const OptionalMemory::Use use(a->more);
+    a->more.drop();
+    if (!a->seg_rs) return SW2D_OK;
+    const size_t one = (2 * seg + 1) * st + seg * (sl + rs);
+    const int64_t n = std::min({a->n_ck - 1, (int64_t)(OptionalMemory::room(8) / one), h->adj_kept_segments - 1});
+    if (n <= 0) return SW2D_OK;
+    const std::vector<size_t> sizes{n * (seg + 1) * st, n * seg * st, n * seg * rs, n * seg * sl};
+    std::vector<void*> p;
+    if (!a->more.take({sizes.begin(), sizes.end() - (sl ? 0 : 1)}, p)) return SW2D_OK;
+    for (size_t i = 0; i < p.size(); i++) CK(cudaMemsetAsync(p[i], 0, sizes[i], h->stream));
+    a->more_st = static_cast<double4*>(p[0]);
+    a->more_bal = static_cast<double4*>(p[1]);
+    a->more_rs = static_cast<double2*>(p[2]);
+    a->more_slope = sl ? static_cast<double2*>(p[3]) : nullptr;
     a->n_seg = 1 + n;
+    return SW2D_OK;
 }
 
 int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
 {
     AdjointState* a = h->adj;
     free_list(a->traj_allocs);
-    {
-        std::lock_guard<std::mutex> lock(more_pool().mu);
-        drop_more(a);
-    }
+    a->more.drop();
     a->ck_valid = false;
     a->n_requested = 0;
     a->n_steps = n_steps;
@@ -1083,19 +1025,14 @@ int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
     const int64_t nc = h->nc, seg = std::min(every, n_steps);
     auto& L = a->traj_allocs;
     int rc = SW2D_OK;
-    for (bool again = true;; again = false) {
-        if (!(rc = adj_alloc(h, L, (a->n_ck + 1) * nc, &a->ck_st)) &&
-            !(rc = adj_alloc(h, L, (a->n_ck + 1) * a->nslot, &a->ck_slot)) &&
-            !(rc = adj_alloc(h, L, a->n_ck + 1, &a->ck_ctrl)) && !(rc = adj_alloc(h, L, (seg + 1) * nc, &a->seg_st)) &&
-            !(rc = adj_alloc(h, L, seg * nc, &a->seg_bal)) && !(rc = adj_alloc(h, L, n_steps, &a->d_dt_seq)) &&
-            !(rc = adj_alloc(h, L, n_steps, &a->d_t_seq)))
-            break;
+    if ((rc = adj_alloc(h, L, (a->n_ck + 1) * nc, &a->ck_st)) ||
+        (rc = adj_alloc(h, L, (a->n_ck + 1) * a->nslot, &a->ck_slot)) ||
+        (rc = adj_alloc(h, L, a->n_ck + 1, &a->ck_ctrl)) || (rc = adj_alloc(h, L, (seg + 1) * nc, &a->seg_st)) ||
+        (rc = adj_alloc(h, L, seg * nc, &a->seg_bal)) || (rc = adj_alloc(h, L, n_steps, &a->d_dt_seq)) ||
+        (rc = adj_alloc(h, L, n_steps, &a->d_t_seq))) {
         free_list(a->traj_allocs);
-        if (!again || !give_back_more()) {
-            a->n_steps = 0;
-            return rc;
-        }
-        h->err.clear();
+        a->n_steps = 0;
+        return rc;
     }
     // each step's slopes and Riemann states, kept by the segment's forward recompute for the
     // reverse steps, when they fit in half of the free device memory (else rebuilt there)
@@ -1115,9 +1052,8 @@ int alloc_trajectory(sw2d_handle* h, int64_t n_steps, int64_t every)
             h->err.clear();
         }
     }
-    more_segments(h, seg);
     a->n_requested = n_steps;
-    return SW2D_OK;
+    return more_segments(h);
 }
 
 // The CFL-driven run from checkpoint 0 that fixes the trajectory's dt sequence (sw2d_record,
@@ -1164,15 +1100,13 @@ int record_from_start(sw2d_handle* h, int64_t* steps_done)
 
 namespace sw2d {
 
+int64_t adjoint_kept_bytes(const sw2d_handle* h) { return h->adj ? (int64_t)h->adj->more.bytes() : 0; }
+
 void adjoint_release(sw2d_handle* h)
 {
     if (!h || !h->adj) return;
     cudaFree(h->adj->d_trace);
     free_list(h->adj->traj_allocs);
-    {
-        std::lock_guard<std::mutex> lock(more_pool().mu);
-        drop_more(h->adj);
-    }
     free_list(h->adj->obs_allocs);
     free_list(h->adj->fixed_allocs);
     delete h->adj;
@@ -1454,9 +1388,10 @@ int sw2d_adjoint(sw2d_handle* h, double* J, const sw2d_gradient* grad)
     CK(cudaSetDevice(h->device));
     AdjointState* a = h->adj;
     if ((rc = check_observations(h))) return rc;
-    const MoreUse use(a);
+    const OptionalMemory::Use use(a->more);
     int64_t kept = 0;
     if (!a->ck_valid) {
+        if (a->more.lost() && (rc = more_segments(h))) return rc;
         if ((rc = run_keeping(h))) return rc;
         if ((rc = read_status(h))) return rc;
         a->ck_valid = true;

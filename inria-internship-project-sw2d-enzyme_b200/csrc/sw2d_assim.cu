@@ -106,6 +106,7 @@ struct AssimState {
     double4* seg_st = nullptr;       // (seg_cap + 1) * nc
     double4* seg_bal = nullptr;      // seg_cap * nc
     double2* seg_slope = nullptr;    // seg_cap * nc: each step's slopes (MUSCL-EVR, when memory allows)
+    OptionalMemory slopes{this, [](void* a) { static_cast<AssimState*>(a)->seg_slope = nullptr; }};
     double4 *lam = nullptr, *lamb = nullptr, *ctb = nullptr;
     double2* cts = nullptr;
     double *znb = nullptr, *gzb = nullptr;
@@ -1165,24 +1166,24 @@ int seg_buffers(sw2d_handle* h)
     AssimState* a = h->assim;
     int64_t longest = 0;
     for (const auto& s : a->segs) longest = std::max(longest, s.n);
-    if (longest <= a->seg_cap) return SW2D_OK;
-    free_list(a->seg_allocs);
-    a->seg_cap = 0;
-    int rc = SW2D_OK;
-    if ((rc = adj_alloc(h, a->seg_allocs, (longest + 1) * h->nc, &a->seg_st)) ||
-        (rc = adj_alloc(h, a->seg_allocs, longest * h->nc, &a->seg_bal)))
-        return rc;
-    // the slopes too, when they fit in half of the free device memory (else the reverse steps rebuild
-    // them: 10k cells, 134 steps, 0.7 ms more per gradient)
-    a->seg_slope = nullptr;
-    size_t free_b = 0, total_b = 0;
-    if (h->p.scheme == SW2D_SCHEME_MUSCL_EVR && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-        (size_t)longest * h->nc * sizeof(double2) < free_b / 2 &&
-        adj_alloc(h, a->seg_allocs, longest * h->nc, &a->seg_slope)) {
-        a->seg_slope = nullptr;
-        h->err.clear();
+    const bool grows = longest > a->seg_cap;
+    if (grows) {
+        free_list(a->seg_allocs);
+        a->slopes.drop();
+        a->seg_cap = 0;
+        int rc = SW2D_OK;
+        if ((rc = adj_alloc(h, a->seg_allocs, (longest + 1) * h->nc, &a->seg_st)) ||
+            (rc = adj_alloc(h, a->seg_allocs, longest * h->nc, &a->seg_bal)))
+            return rc;
+        a->seg_cap = longest;
     }
-    a->seg_cap = longest;
+    // the slopes too, within half of the free device memory and the share of all handles (else the
+    // reverse steps rebuild them: 10k cells, 134 steps, 0.7 ms more per gradient)
+    const size_t bytes = (size_t)a->seg_cap * h->nc * sizeof(double2);
+    std::vector<void*> p;
+    if (h->p.scheme == SW2D_SCHEME_MUSCL_EVR && (grows || a->slopes.lost()) && bytes <= OptionalMemory::room(2) &&
+        a->slopes.take({bytes}, p))
+        a->seg_slope = static_cast<double2*>(p[0]);
     return SW2D_OK;
 }
 
@@ -1271,6 +1272,8 @@ int require(sw2d_handle* h, bool need_record)
 }  // namespace
 
 namespace sw2d {
+
+int64_t assim_kept_bytes(const sw2d_handle* h) { return h->assim ? (int64_t)h->assim->slopes.bytes() : 0; }
 
 void assim_release(sw2d_handle* h)
 {
@@ -1453,6 +1456,7 @@ int sw2d_assim_gradient(sw2d_handle* h, const double* m, int64_t stride, double*
     CK(cudaMemsetAsync(a->g_k2, 0, nc * sizeof(double), h->stream));
     CK(cudaMemsetAsync(a->g_w, 0, nc * sizeof(double), h->stream));
     CK(cudaMemsetAsync(a->gzb, 0, nc * sizeof(double), h->stream));
+    const OptionalMemory::Use use(a->slopes);
     if (K > 0 && (rc = seg_buffers(h))) return rc;
     if (K > 0 && h->assim_chained && (rc = chain_states(h))) return rc;
     // tiles: tile_top[k] = the last segment of a tile (the adjoint restarts from 0 before it)

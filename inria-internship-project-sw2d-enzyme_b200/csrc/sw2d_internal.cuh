@@ -564,8 +564,10 @@ int closure_set_ctas(sw2d_handle* h, int per_sm);  // resident CTAs per SM of th
 
 // Releases the adjoint buffers of the handle (sw2d_adjoint.cu).
 void adjoint_release(sw2d_handle* h);
+int64_t adjoint_kept_bytes(const sw2d_handle* h);
 // Releases the assimilation buffers of the handle (sw2d_assim.cu).
 void assim_release(sw2d_handle* h);
+int64_t assim_kept_bytes(const sw2d_handle* h);
 // Called when the physical parameters or the state change under a recorded trajectory.
 void adjoint_invalidate(sw2d_handle* h);
 

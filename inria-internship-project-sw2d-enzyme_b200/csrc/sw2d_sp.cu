@@ -1562,6 +1562,7 @@ int sw2d_get_option(sw2d_handle* h, const char* name, int64_t* value)
     else if (std::strcmp(name, "flux_variant") == 0) *value = h->flux_variant;
     else if (std::strcmp(name, "run_kernel") == 0) *value = h->run_kernel;
     else if (std::strcmp(name, "run_steps") == 0) *value = h->run_taken;
+    else if (std::strcmp(name, "kept_bytes") == 0) *value = adjoint_kept_bytes(h) + assim_kept_bytes(h);
     else if (std::strcmp(name, "update_reverse") == 0) *value = h->m.rev_update;
     else if (std::strcmp(name, "fused_slopes") == 0) *value = h->fused_slopes;
     else if (std::strcmp(name, "tile_cells") == 0) *value = h->tiles.tile_cells;

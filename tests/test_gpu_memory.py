@@ -81,3 +81,113 @@ def test_porosity_gradient(pkg, scheme):
         return [model.assim_gradient(case.phi, 6)[0], np.float64(model.assim_replay_cost(case.phi))]
 
     assert _failing_in_turn(pkg, make, act) >= (1 if scheme == "muscl_evr" else 0)
+
+
+def _recorded(pkg, case):
+    model = pkg.SpModel(case)
+    model.record(20, 6)
+    model.set_observations([3, 50], [10, 20], np.full((2, 2), 1.0))
+    return model
+
+
+def _gradient(model, friction):
+    model.set_param("friction", friction)
+    J, g = model.adjoint()
+    return [np.float64(J)] + [g[k] for k in sorted(g)]
+
+
+def _assimilating(pkg, case, dt):
+    model = pkg.SpModel(case)
+    model.assim_configure(phi_transform="none", cost_normalize=True)
+    model.assim_set_gauges([8 * dt, 16 * dt], [3, 50], np.ones(2), np.full((2, 2), 1.0))
+    return model
+
+
+def test_kept_memory_gives_way(pkg):
+    """The kept steps of one handle and the kept slopes of another go to whatever finds no room: a
+    model's creation, a record, a network's training buffers.  The next gradients take them again, with
+    the same results; those of a handle that cannot, too."""
+    case = pkg.workloads.dam_break(n_cells=600)
+    free = pkg.workloads.dam_break(n_cells=600, friction="none")
+    probe = pkg.SpModel(free)
+    probe.step(3)
+    dt = probe.dt
+    probe.close()
+    free.opts = dict(free.opts, t_max=20 * dt)
+    fails = pkg.capi.load_library().sw2d_test_fail_allocations
+    a, b = _recorded(pkg, case), _assimilating(pkg, free, dt)
+    want_a, want_b = _gradient(a, case.friction[0] * 1.1), b.assim_gradient(free.phi, 6)[0]
+    held = a.get_option("kept_bytes"), b.get_option("kept_bytes")
+    assert held[0] > 0 and held[1] > 0
+    net = pkg.closure.MLP(pkg.closure.init_params(0))
+    x, t = np.zeros((300, 10), np.float32), np.zeros((300, 2), np.float32)
+
+    others = [(0, lambda: pkg.SpModel(case).close()), (0, lambda: _recorded(pkg, case).close()),
+              (1, lambda: net.loss_grad(x, t))]     # its first request is for host memory
+    for skip, other in others:
+        fails(skip, 1)
+        try:
+            other()
+        finally:
+            fails(0, 0)
+        assert (a.get_option("kept_bytes"), b.get_option("kept_bytes")) == (0, 0)
+        got = _gradient(a, case.friction[0] * 1.1)
+        assert all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(got, want_a))
+        assert np.array_equal(_bits(b.assim_gradient(free.phi, 6)[0]), _bits(want_b))
+        assert (a.get_option("kept_bytes"), b.get_option("kept_bytes")) == held
+    # taken back and not to be had again: every segment recomputed, the slopes rebuilt
+    fails(0, 1)
+    pkg.SpModel(case).close()
+    for model, act, want in ((a, lambda: _gradient(a, case.friction[0] * 1.1), want_a),
+                             (b, lambda: [b.assim_gradient(free.phi, 6)[0]], [want_b])):
+        n = fails(0, 0)
+        act()
+        n = fails(0, 0)                  # the gradient's requests, the kept memory's among them
+        fails(0, 1)
+        pkg.SpModel(case).close()
+        fails(0, n)
+        try:
+            got = act()
+        finally:
+            fails(0, 0)
+        assert model.get_option("kept_bytes") == 0
+        assert all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(got, want))
+    net.close()
+    a.close()
+    b.close()
+
+
+def test_kept_memory_of_several_threads(pkg):
+    """Gradients of several handles in threads, while others' allocations take what is idle."""
+    import threading
+
+    case = pkg.workloads.dam_break(n_cells=600)
+    fails = pkg.capi.load_library().sw2d_test_fail_allocations
+    models = [_recorded(pkg, case) for _ in range(4)]
+    want = _gradient(models[0], case.friction[0] * 1.1)
+    bad = []
+
+    def gradients(m):
+        for _ in range(30):
+            got = _gradient(m, case.friction[0] * 1.1)
+            if not all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(got, want)):
+                bad.append(m)
+
+    def creations():
+        for _ in range(30):
+            fails(0, 1)
+            try:
+                pkg.SpModel(case).close()
+            except pkg.Sw2dError:
+                pass                     # nothing was idle
+            finally:
+                fails(0, 0)
+
+    threads = [threading.Thread(target=gradients, args=(m,)) for m in models] + [threading.Thread(target=creations)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not bad
+    for m in models:
+        m.close()
