@@ -705,25 +705,39 @@ int ensure_cap(sw2d_mlp* m, int64_t n)
 // floats of the result buffer of a batch of n rows: gradient, loss partials (256 rows each), status
 size_t result_floats(int64_t n) { return (size_t)sw2d::kNParams + (size_t)((n + 255) / 256) + 1; }
 
-// training buffers for n rows (the pinned copy is replaced together with the device buffer)
+// Training buffers for n rows: the new ones first, so that a batch they cannot be had for leaves the old
+// ones to smaller batches, then the old ones freed
 int ensure_train(sw2d_mlp* m, int64_t n)
 {
     using namespace sw2d;
     if (n <= m->tcap) return SW2D_OK;
-    int rc;
-    if (m->host) MCK(cudaFreeHost(m->host));
-    m->host = nullptr;
-    MCK(sw2d::pinned_malloc(&m->host, result_floats(n) * sizeof(float)));
-    float* grad = nullptr;
-    const int64_t parts = std::min<int64_t>((n + kTileM - 1) / kTileM, m->sms);  // one per CTA
-    if (parts > m->parts) {
-        if ((rc = malloc_dev(m, parts * kPartStride, &m->part))) return rc;
-        m->parts = parts;
-    }
-    if ((rc = malloc_dev(m, n * kIn, &m->traw)) || (rc = malloc_dev(m, n * kOut, &m->t)) ||
-        (rc = malloc_dev(m, n, &m->se)) || (rc = malloc_dev(m, result_floats(n), &grad)))
+    const int64_t parts = std::max(m->parts, std::min<int64_t>((n + kTileM - 1) / kTileM, m->sms));  // one per CTA
+    const size_t first = m->allocs.size();
+    float *host = nullptr, *part = nullptr, *traw = nullptr, *t = nullptr, *se = nullptr, *grad = nullptr;
+    MCK(pinned_malloc(&host, result_floats(n) * sizeof(float)));
+    int rc = SW2D_OK;
+    if ((parts > m->parts && (rc = malloc_dev(m, parts * kPartStride, &part))) || (rc = malloc_dev(m, n * kIn, &traw)) ||
+        (rc = malloc_dev(m, n * kOut, &t)) || (rc = malloc_dev(m, n, &se)) || (rc = malloc_dev(m, result_floats(n), &grad))) {
+        for (size_t i = first; i < m->allocs.size(); i++) cudaFree(m->allocs[i]);
+        m->allocs.resize(first);
+        cudaFreeHost(host);
         return rc;
-    m->grad = grad;
+    }
+    auto replace = [&](float*& old, float* now) {
+        if (old) {
+            m->allocs.erase(std::remove(m->allocs.begin(), m->allocs.end(), static_cast<void*>(old)), m->allocs.end());
+            cudaFree(old);
+        }
+        old = now;
+    };
+    if (part) replace(m->part, part);
+    replace(m->traw, traw);
+    replace(m->t, t);
+    replace(m->se, se);
+    replace(m->grad, grad);
+    if (m->host) cudaFreeHost(m->host);
+    m->host = host;
+    m->parts = parts;
     m->tcap = n;
     return SW2D_OK;
 }

@@ -191,3 +191,47 @@ def test_kept_memory_of_several_threads(pkg):
     assert not bad
     for m in models:
         m.close()
+
+
+def test_training_buffers(pkg):
+    """A batch too large for the memory there is: reported, and batches of the sizes before train on, with
+    the gradient of the last one for the next step.  Growing batches keep one set of buffers."""
+    import torch
+
+    C = pkg.closure
+    fails = pkg.capi.load_library().sw2d_test_fail_allocations
+    rng = np.random.default_rng(1)
+    x, t = rng.normal(size=(60000, 10)).astype(np.float32), rng.normal(size=(60000, 2)).astype(np.float32)
+
+    def step(net, n):
+        loss, g = net.loss_grad(x[:n], t[:n])
+        net.adam_step(1e-3)
+        return [np.float64(loss), np.asarray(g, np.float64), np.asarray(net.params, np.float64)]
+
+    net, ref = C.MLP(C.init_params(3)), C.MLP(C.init_params(3))
+    assert all(np.array_equal(a, b) for a, b in zip(step(net, 300), step(ref, 300)))
+    fails(0, 0)
+    C.MLP(C.init_params(3)).loss_grad(x[:1], t[:1])
+    n = fails(0, 0)
+    tried = 0
+    for skip in range(n):
+        fails(skip, 1)
+        try:
+            net.loss_grad(x[:5000], t[:5000])
+            break                        # fewer requests than a first batch makes
+        except RuntimeError:
+            tried += 1
+        finally:
+            fails(0, 0)
+        net.adam_step(1e-3)              # the gradient of the last batch is still there
+        ref.adam_step(1e-3)
+        assert np.array_equal(net.params, ref.params)
+        assert all(np.array_equal(a, b) for a, b in zip(step(net, 300), step(ref, 300)))
+    assert tried >= 5
+    free = []
+    for k in range(6):
+        net.loss_grad(x[:50000 + 1000 * k], t[:50000 + 1000 * k])
+        free.append(torch.cuda.mem_get_info(0)[0])
+    assert free[0] - free[-1] <= 4 << 20       # the last set is 10 % larger than the first, no more
+    net.close()
+    ref.close()
