@@ -436,6 +436,20 @@ int tiles_make(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<
 // tiles are built the first time), the launches of n steps, another try at tiles that found no memory,
 // the release.
 int run_ready(sw2d_handle* h, bool* ready);
+// A call that takes steps of a mesh the run kernel can take (`ready`), from its start to its end: whether
+// it takes them in the run kernel, which the calls in progress in other threads decide with it
+class RunTurn {
+public:
+    RunTurn(const sw2d_handle* h, bool ready);
+    ~RunTurn();
+    RunTurn(const RunTurn&) = delete;
+    RunTurn& operator=(const RunTurn&) = delete;
+    bool run() const { return run_; }
+
+private:
+    int device_, tiles_;
+    bool run_;
+};
 int run_steps(sw2d_handle* h, int64_t n);
 void run_retry(sw2d_handle* h);
 void run_release(sw2d_handle* h);

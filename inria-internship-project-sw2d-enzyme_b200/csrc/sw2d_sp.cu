@@ -985,7 +985,8 @@ int sw2d_step_n(sw2d_handle* h, int64_t n_steps, int64_t* steps_done)
     CK(cudaSetDevice(h->device));
     bool run = false;
     if (const int rc = run_ready(h, &run)) return rc;
-    if (run) {  // a small mesh: all steps in one launch, the control block copied out before and after it
+    const RunTurn turn(h, run);
+    if (turn.run()) {  // a small mesh: all steps in one launch, the control block copied out before and after it
         Ctrl* host = h->ctrl_host;
         CK(cudaMemcpyAsync(host + 1, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
         if (const int rc = run_steps(h, n_steps)) return rc;

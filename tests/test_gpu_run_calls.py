@@ -108,3 +108,40 @@ def test_tiles_that_do_not_fit_hold_no_memory(pkg):
     assert m.get_option("run_steps") == 0
     assert torch.cuda.mem_get_info(0)[0] == free0
     m.close()
+
+
+@pytest.mark.parametrize("cells,threads,shares", [(20000, 4, False), (5000, 6, False), (500, 4, True)])
+def test_handles_in_several_threads(pkg, cells, threads, shares):
+    """Handles stepped from threads: where their tiles do not share the chip, the step's kernels of all of
+    them do, and no handle holds it alone; where they do, each takes the run kernel.  The bits are those
+    of a handle alone."""
+    import threading
+
+    case = pkg.workloads.dam_break(n_cells=cells)
+    alone = pkg.SpModel(case)
+    alone.prepare()
+    alone.step(64)
+    assert alone.get_option("run_steps") == 64
+    models = [pkg.SpModel(case) for _ in range(threads)]
+    for m in models:
+        m.prepare()
+    start = threading.Barrier(threads)
+
+    def work(m):
+        start.wait()
+        for _ in range(40):
+            m.step(64)
+
+    pool = [threading.Thread(target=work, args=(m,)) for m in models]
+    for th in pool:
+        th.start()
+    for th in pool:
+        th.join()
+    alone.step(64 * 39)
+    share = sum(m.get_option("run_steps") for m in models) / (threads * 40 * 64)
+    assert share > 0.9 if shares else share < 0.5      # a first and last calls, that others do not overlap
+    assert all(_same_state(m, alone) and m.time == alone.time for m in models)
+    models[0].step(64)                                 # alone again
+    assert models[0].get_option("run_steps") >= 64
+    for m in models + [alone]:
+        m.close()
