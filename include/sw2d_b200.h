@@ -369,8 +369,9 @@ int sw2d_result_close(sw2d_handle* h);
 
 /* Advances at most n_steps passes of the body of swSp::execute's time loop
  * (swSp.cpp:522-589: hypCompute, friction, singular head loss, correctVelocity, t += dt),
- * stopping once t >= t_max.  The loop runs on the device (CUDA graph); the host does not
- * synchronise between steps.  *steps_done receives the number of steps taken (may be NULL). */
+ * stopping once t >= t_max.  The loop runs on the device, in a CUDA graph of the step's kernels or,
+ * for small meshes, in one launch (option "run_kernel"); the host does not synchronise between
+ * steps.  *steps_done receives the number of steps taken (may be NULL). */
 int sw2d_step_n(sw2d_handle* h, int64_t n_steps, int64_t* steps_done);
 /* Saves the run's point on the device (state, the balance slots that carry the fluxes of edges
  * left dry from step to step, time, dt and step count); sw2d_restore_point returns the run to
@@ -378,9 +379,12 @@ int sw2d_step_n(sw2d_handle* h, int64_t n_steps, int64_t* steps_done);
  * handle (saving again replaces it).  SP and DIP models.  No counterpart in the reference. */
 int sw2d_save_point(sw2d_handle* h);
 int sw2d_restore_point(sw2d_handle* h);
-/* Captures and instantiates the CUDA graph sw2d_step_n launches (32 steps, or the result file's
- * chunk), without taking a step, so that a timed run does not include the capture; the graph is
- * captured again after an option or launch configuration changes.  No counterpart in the
+/* Prepares what sw2d_step_n launches, without taking a step, so that a timed run does not include it:
+ * the CUDA graph of the step's kernels (32 steps, or the result file's chunk), captured again after
+ * an option or launch configuration changes, or for small meshes the tiles of the run kernel, once per
+ * handle (0.2 ms at 2,000 cells, 1.3 ms at 20,000, 3.8 ms at 60,000).  Without this call the graph is
+ * made by the first call that needs it, the tiles once the handle has been asked for as many steps as
+ * pay for them (8 to 32, from 8,192 cells on a 256th of the cells).  No counterpart in the
  * reference. */
 int sw2d_prepare_steps(sw2d_handle* h);
 
@@ -460,7 +464,9 @@ const char* sw2d_phase_name(int i);
  * "kept_bytes" (read only): what the handle holds of it.
  * "run_kernel" (0/1, default 1): sw2d_step_n and sw2d_execute take the steps of a small SP or DIP
  * mesh (one whose cells fit the chip's shared memory) in one launch; 0 takes them kernel by kernel, as
- * is done where there is no memory for the mesh's tiles.  "run_steps" (read only): steps taken so.
+ * is done where there is no memory for the mesh's tiles, before a new handle's steps are worth them
+ * (sw2d_prepare_steps; not once the option has been set to 1) and while several threads step handles
+ * whose tiles do not share the chip.  "run_steps" (read only): steps taken in one launch.
  * "run_wait_polls": the poll limit of that launch's waits, after which it gives up with an error
  * status (negative: the default).
  * "adjoint_trace" (0/1): record the state adjoint's magnitude per reverse step

@@ -351,7 +351,9 @@ struct sw2d_handle {
     int flux_variant = 0;               // launch variant of k_flux (sw2d_autotune)
     sw2d::RunState* run = nullptr;      // run kernel of small meshes
     int run_kernel = 1;                 // option "run_kernel"
+    bool run_eager = false;             // set to 1 by the caller: tiles built at the first call
     int64_t run_polls = -1;             // option "run_wait_polls" (< 0: the default)
+    int64_t run_asked = 0;              // steps asked for before the run kernel's tiles were built
     int64_t run_taken = 0;              // steps the run kernel has taken (option "run_steps")
     std::string err;
 };
@@ -432,10 +434,10 @@ int tiles_make(sw2d_handle* h, const std::vector<int2>& coff, const std::vector<
                const std::vector<int>& bcell, int tile_cells, bool own_slopes, int least, TileMesh& tm,
                std::vector<void*>& allocs, std::string& why);
 
-// The run kernel of small meshes (sw2d_run.cu): whether the handle's next steps may take it (its
-// tiles are built the first time), the launches of n steps, another try at tiles that found no memory,
-// the release.
-int run_ready(sw2d_handle* h, bool* ready);
+// The run kernel of small meshes (sw2d_run.cu): whether the handle's next `steps` steps may take it, its
+// tiles built when its steps are worth them (`steps` < 0: in any case), the launches of n steps, another
+// try at tiles that found no memory, the release.
+int run_ready(sw2d_handle* h, int64_t steps, bool* ready);
 // A call that takes steps of a mesh the run kernel can take (`ready`), from its start to its end: whether
 // it takes them in the run kernel, which the calls in progress in other threads decide with it
 class RunTurn {

@@ -984,7 +984,7 @@ int sw2d_step_n(sw2d_handle* h, int64_t n_steps, int64_t* steps_done)
     if (!h || n_steps < 0) return fail(h, SW2D_E_ARG, "invalid arguments");
     CK(cudaSetDevice(h->device));
     bool run = false;
-    if (const int rc = run_ready(h, &run)) return rc;
+    if (const int rc = run_ready(h, n_steps, &run)) return rc;
     const RunTurn turn(h, run);
     if (turn.run()) {  // a small mesh: all steps in one launch, the control block copied out before and after it
         Ctrl* host = h->ctrl_host;
@@ -1049,7 +1049,7 @@ int sw2d_prepare_steps(sw2d_handle* h)
     if (!h) return fail(h, SW2D_E_ARG, "invalid handle");
     CK(cudaSetDevice(h->device));
     bool run = false;
-    int rc = run_ready(h, &run);
+    int rc = run_ready(h, -1, &run);
     if (!rc && !run) rc = ensure_graph(h, h->result ? result_chunk(h) : kGraphSteps);
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->stream));
@@ -1525,6 +1525,7 @@ int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value)
         // launch (sw2d_run.cu); 0: by the step's kernels (the same results).  Set again, it also
         // tries again for a mesh that found no memory for its tiles.
         h->run_kernel = value ? 1 : 0;
+        h->run_eager = value != 0;
         run_retry(h);
     } else if (std::strcmp(name, "run_wait_polls") == 0) {
         // poll limit of the run kernel's waits (< 0: the default)

@@ -145,3 +145,31 @@ def test_handles_in_several_threads(pkg, cells, threads, shares):
     assert models[0].get_option("run_steps") >= 64
     for m in models + [alone]:
         m.close()
+
+
+def test_first_steps_of_a_handle(pkg):
+    """A model that takes a few steps does not pay for the run kernel's tiles; one that goes on, is prepared,
+    or is told to, has them."""
+    case = pkg.workloads.dam_break(n_cells=20000)
+    models = [pkg.SpModel(case) for _ in range(4)]
+    calls = (1, 30, 40, 10, 5)                     # 78 steps pay for the tiles of 20,000 cells
+    taken = []
+    models[1].prepare()
+    models[2].set_option("run_kernel", 1)
+    models[3].set_option("run_kernel", 0)
+    for m in models:
+        row = []
+        for n in calls:
+            assert m.step(n) == n
+            row.append(m.get_option("run_steps"))
+        taken.append(row)
+    assert taken == [[0, 0, 0, 10, 15], [1, 31, 71, 81, 86], [1, 31, 71, 81, 86], [0] * 5]
+    assert all(_same_state(m, models[0]) and m.time == models[0].time for m in models[1:])
+    for m in models:
+        m.close()
+    m = pkg.SpModel(pkg.workloads.dam_break(n_cells=500))
+    m.step(7)                                      # 8 steps pay for the tiles of 500 cells
+    assert m.get_option("run_steps") == 0
+    m.step(1)
+    assert m.get_option("run_steps") == 1
+    m.close()
