@@ -495,7 +495,9 @@ int sw2d_autotune(sw2d_handle* h, int iters, char* report, int capacity);
  * 512 cells when n_tile_sizes is 0), for MUSCL-EVR with the slopes inside k_flux and with
  * k_slopes first, each at its fastest launch variant (k_update, the same in every form, is left
  * out of the sums); then sets the fastest form ("fused_step", "fused_slopes", "tile_cells",
- * "flux_variant" and the launch config can be read back to persist it).  The run continues with
+ * "flux_variant" and the launch config can be read back to persist it).  A small mesh that the run
+ * kernel takes (option "run_kernel") keeps it unless the fastest form with its update is faster than
+ * a step of it, also timed; else "fused_step" would turn it off.  The run continues with
  * the same bits, as for sw2d_autotune.  DDP handles: sw2d_autotune. */
 int sw2d_autotune_step(sw2d_handle* h, int iters, const int* tile_sizes, int n_tile_sizes, char* report,
                        int capacity);

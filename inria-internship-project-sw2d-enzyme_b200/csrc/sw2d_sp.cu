@@ -1258,6 +1258,71 @@ int sw2d_autotune(sw2d_handle* h, int iters, char* report, int capacity)
     return SW2D_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// ms a step of the run kernel against `form_ms` of another form's step without its update; *run tells
+// whether the run kernel is the faster.  The state, slots, slopes and control block are put back.
+template <class Time>
+int time_run_kernel(sw2d_handle* h, int steps, cudaEvent_t e0, cudaEvent_t e1, double form_ms, Time&& time_it,
+                    std::string& rep, bool* run)
+{
+    DevMesh& m = h->m;
+    struct Part {
+        void* p;
+        size_t bytes;
+    } parts[] = {{m.st, h->nc * sizeof(double4)},
+                 {m.slot, (size_t)h->h_coff.back().y * sizeof(Slot)},
+                 {m.slope, h->nc * sizeof(double2)},
+                 {h->ctrl, sizeof(Ctrl)}};
+    size_t total = 0;
+    for (const Part& p : parts) total += p.bytes;
+    char* saved = nullptr;
+    if (device_malloc(&saved, total) != cudaSuccess) return SW2D_OK;  // not timed: the run kernel stays
+    auto copy_all = [&](bool back) {
+        cudaError_t e = cudaSuccess;
+        char* at = saved;
+        for (const Part& p : parts) {
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(back ? p.p : at, back ? at : p.p, p.bytes, cudaMemcpyDeviceToDevice, h->stream);
+            at += p.bytes;
+        }
+        return e;
+    };
+    double update_ms = 0.0;
+    float run_ms = 0.f;
+    auto measure = [&]() -> int {
+        CK(copy_all(false));
+        update_ms = time_it([&] { launch_update_s<false>(h, m); });
+        CK(copy_all(true));
+        Ctrl c;
+        CK(cudaMemcpyAsync(&c, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        c.t_max = 1.0e300;  // every step is taken, also at the end of the run
+        CK(cudaMemcpyAsync(h->ctrl, &c, sizeof(Ctrl), cudaMemcpyHostToDevice, h->stream));
+        if (const int rc = run_steps(h, 1)) return rc;
+        CK(cudaEventRecord(e0, h->stream));
+        if (const int rc = run_steps(h, steps)) return rc;
+        CK(cudaEventRecord(e1, h->stream));
+        CK(cudaEventSynchronize(e1));
+        CK(cudaEventElapsedTime(&run_ms, e0, e1));
+        CK(copy_all(true));
+        CK(cudaStreamSynchronize(h->stream));
+        return SW2D_OK;
+    };
+    const int rc = measure();
+    cudaFree(saved);
+    if (rc) return rc;
+    rep += "k_update=" + std::to_string(update_ms) + "ms run-kernel=" + std::to_string(run_ms / steps) + "ms ";
+    *run = run_ms / steps < form_ms + update_ms;
+    return SW2D_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 int sw2d_autotune_step(sw2d_handle* h, int iters, const int* tile_sizes, int n_tile_sizes, char* report,
                        int capacity)
 {
@@ -1349,8 +1414,18 @@ int sw2d_autotune_step(sw2d_handle* h, int iters, const int* tile_sizes, int n_t
             if (pre + bf < best.ms) best = {pre + bf, 1, fs, tile_sizes[k], bv};
         }
     }
+    // the run kernel of a small mesh: whole steps, against those of the best form above with its update,
+    // from the live state, which is put back
+    bool run = false;
+    const int prev_fused = h->fused;
+    h->fused = 0;
+    int rc_run = run_ready(h, -1, &run);
+    if (!rc_run && run) rc_run = time_run_kernel(h, std::max(iters, 32), e0, e1, best.ms, time_it, rep, &run);
+    h->fused = prev_fused;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (rc_run) return rc_run;
+    if (run) best = {0.0, 0, prev_fs, prev_tile, h->flux_variant};
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));
     // the chosen form (tiles rebuilt for it; the previous tiles, if any, when the four-kernel
@@ -1377,7 +1452,7 @@ int sw2d_autotune_step(sw2d_handle* h, int iters, const int* tile_sizes, int n_t
         rep += "chosen fused" + std::string(muscl ? (best.fused_slopes ? "" : "/slopes-first") : "") + " tile " +
                std::to_string(best.tile) + " k_flux/" + flux_variant_label(best.flux_v);
     else
-        rep += "chosen four-kernel k_slopes/" + std::to_string(kVariants[slope_v].block) + "x" +
+        rep += std::string("chosen ") + (run ? "run kernel, else four-kernel k_slopes/" : "four-kernel k_slopes/") + std::to_string(kVariants[slope_v].block) + "x" +
                std::to_string(kVariants[slope_v].minb) + " k_edges/" + std::to_string(kVariants[edge_v].block) + "x" +
                std::to_string(kVariants[edge_v].minb);
     if (report && capacity > 0) {

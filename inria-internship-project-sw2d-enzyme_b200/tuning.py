@@ -7,8 +7,9 @@ choice is stored in a JSON file keyed by GPU, scheme, options, step kind, tile s
 size (power-of-two bucket), and reused by later runs without timing again.
 
 ``autotune_step(model)`` (sw2d_autotune_step) also chooses the step form: the four-kernel step
-or the fused step, its tile size and, for MUSCL-EVR, where the slopes are computed; its cache
-key leaves out the step kind and tile size, which are what it chooses.
+or the fused step, its tile size and, for MUSCL-EVR, where the slopes are computed, or neither for
+a small mesh whose steps the run kernel takes faster; its cache key leaves out the step kind and
+tile size, which are what it chooses.
 """
 from __future__ import annotations
 
@@ -88,7 +89,7 @@ def autotune_step(model, iters: int = 10, device: int = 0, tile_sizes=(), cache_
                   force: bool = False) -> dict:
     """Chooses the step form, tile size and launch variants for `model` (sw2d_autotune_step);
     returns {"fused", "fused_slopes", "tile", "slopes", "edges", "flux", "report", "cached"}."""
-    key = "|".join(_base_key(model, device) + ["step"])
+    key = "|".join(_base_key(model, device) + [f"step-run{model.get_option('run_kernel')}"])
     db = _load(cache_path) if cache_path else {}
     if not force and key in db:
         e = db[key]

@@ -173,3 +173,31 @@ def test_first_steps_of_a_handle(pkg):
     m.step(1)
     assert m.get_option("run_steps") == 1
     m.close()
+
+
+@pytest.mark.parametrize("scheme", ["muscl_evr", "godunov"])
+@pytest.mark.parametrize("cells", [800, 20000])
+def test_autotuning_times_the_run_kernel(pkg, cells, scheme, tmp_path):
+    """The step's autotuner measures the run kernel of a small mesh beside the other forms, keeps it unless
+    one of them is faster, and leaves the run's bits alone; with the option 0 it is no candidate."""
+    case = pkg.workloads.channel_features(n_cells=cells, scheme=scheme)
+    a, b, c = (pkg.SpModel(case) for _ in range(3))
+    for m in (a, b, c):
+        m.step(25)
+    cache = str(tmp_path / "tune.json")
+    rep = pkg.tuning.autotune_step(a, iters=2, tile_sizes=(96, 256), cache_path=cache)
+    ms = {k: float(v.rstrip("ms")) for k, v in (w.split("=") for w in rep["report"].split() if "=" in w)}
+    rest = min(v for k, v in ms.items() if k.startswith(("four-kernel", "fused")))
+    kept = ms["run-kernel"] < rest + ms["k_update"]
+    assert kept == ("chosen run kernel" in rep["report"]) and (not kept or not rep["fused"])
+    before = a.get_option("run_steps")
+    assert a.step(50) == b.step(50) == 50
+    assert a.get_option("run_steps") - before == (0 if rep["fused"] else 50)
+    assert _same_state(a, b) and a.time == b.time
+    for name in ("slope_x", "slope_y"):
+        if scheme == "muscl_evr" and not rep["fused"]:
+            assert np.array_equal(_bits(a.array(name)), _bits(b.array(name)))
+    c.set_option("run_kernel", 0)
+    assert "run-kernel" not in pkg.tuning.autotune_step(c, iters=2, tile_sizes=(96,), cache_path=cache)["report"]
+    for m in (a, b, c):
+        m.close()
