@@ -468,7 +468,9 @@ const char* sw2d_phase_name(int i);
  * (sw2d_prepare_steps; not once the option has been set to 1) and while several threads step handles
  * whose tiles do not share the chip.  "run_steps" (read only): steps taken in one launch.
  * "run_wait_polls": the poll limit of that launch's waits, after which it gives up with an error
- * status (negative: the default).
+ * status (negative: the default, seconds of polling; all tiles are resident at once, so that only a
+ * device that stops making progress reaches it).  The state is then undefined until it is set, with
+ * the time, or restored.
  * "adjoint_trace" (0/1): record the state adjoint's magnitude per reverse step
  * (sw2d_adjoint_trace). */
 int sw2d_set_option(sw2d_handle* h, const char* name, int64_t value);

@@ -994,7 +994,13 @@ int sw2d_step_n(sw2d_handle* h, int64_t n_steps, int64_t* steps_done)
         CK(cudaStreamSynchronize(h->stream));
         h->run_taken += host[0].steps - host[1].steps;
         if (steps_done) *steps_done = host[0].steps - host[1].steps;
-        return status_to_code(h, host[0].status);
+        const unsigned status = host[0].status;
+        if (status & kStatusRunWait) {  // reported once: with a state set or restored the handle goes on
+            host[0].status &= ~kStatusRunWait;
+            CK(cudaMemcpyAsync(h->ctrl, host, sizeof(Ctrl), cudaMemcpyHostToDevice, h->stream));
+            CK(cudaStreamSynchronize(h->stream));
+        }
+        return status_to_code(h, status);
     }
     CK(cudaMemcpyAsync(h->ctrl_host, h->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));

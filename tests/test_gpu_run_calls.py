@@ -201,3 +201,22 @@ def test_autotuning_times_the_run_kernel(pkg, cells, scheme, tmp_path):
     assert "run-kernel" not in pkg.tuning.autotune_step(c, iters=2, tile_sizes=(96,), cache_path=cache)["report"]
     for m in (a, b, c):
         m.close()
+
+
+def test_a_wait_that_ran_out_is_reported_once(pkg):
+    """With the state and the time set again the handle goes on, also without a saved point."""
+    case = pkg.workloads.dam_break(n_cells=4000)
+    a, b = pkg.SpModel(case), pkg.SpModel(case)
+    for m in (a, b):
+        m.prepare()
+    a.set_option("run_wait_polls", 0)
+    with pytest.raises(pkg.Sw2dError, match="run kernel ran out"):
+        a.step(20)
+    a.set_option("run_wait_polls", -1)
+    for m in (a, b):
+        m.set_state(case.h0 * 1.01, case.q0, case.r0)
+        m.set_time(1.0, 0.01)
+        assert m.step(20) == 20
+    assert _same_state(a, b) and a.time == b.time
+    a.close()
+    b.close()
