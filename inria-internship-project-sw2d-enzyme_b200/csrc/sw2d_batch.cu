@@ -187,7 +187,7 @@ int sw2d_batch_create(sw2d_handle* const* members, int n_members, sw2d_batch** o
     if (queue_eligible(members, n_members, why)) {
         int64_t cells = 0;
         for (sw2d_handle* h : b->members) cells += h->nc;
-        b->q_cells = b->q_edges = queue_tile_rule(cells);
+        b->q_cells = b->q_edges = queue_tile_rule(cells, b->q_variant);
         if (queue_build(b->queue, members, n_members, b->q_variant, b->q_cells, b->q_edges, why) == SW2D_OK) b->mode = 1;
         else return bail(bfail(b, SW2D_E_CUDA, why));
     }

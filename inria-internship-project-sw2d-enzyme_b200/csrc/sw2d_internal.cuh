@@ -415,7 +415,7 @@ unsigned queue_read_status(QueueState* q);
 void queue_clear_status(QueueState* q);
 void queue_release(QueueState* q);
 int queue_variants();
-int queue_tile_rule(int64_t cells);
+int queue_tile_rule(int64_t cells, int variant);
 std::string queue_variant_label(int v);
 void queue_set_polls(QueueState* q, long long polls);
 int queue_grid(const QueueState* q);

@@ -384,16 +384,22 @@ int queue_build(QueueState*& q, sw2d_handle* const* members, int n, int variant,
     return SW2D_OK;
 }
 
-// Cells (edges) per tile for an ensemble of `cells` cells in all: a power of two near one tile per
-// resident CTA and phase, 128 .. 4096.  Smaller tiles pay a CTA's item overhead too often, larger ones
-// make each phase of a member a serial chain: 424k cells in 24 members, us per step with tiles of
-// 128 / 256 / 512 / 1024 / 4096: 137 / 111 / 105 / 161 / 457; 21k cells in 6 members: 30 / 40 / 60 / 99 /
-// 323; 1.7M cells in 100 members: 559 / 446 / 395 / 369 / 598; 12.2M cells in 256 members: 4096.
-int queue_tile_rule(int64_t cells)
+// Cells (edges) per tile for an ensemble of `cells` cells in all under launch variant v: a power of two,
+// 128 .. 4096, of one to two tiles per resident CTA and phase.  Smaller tiles pay a CTA's item overhead too
+// often, larger ones make each phase of a member a serial chain, which weighs more the smaller the tile: up
+// to 1.5 tiles per CTA below tiles of 1024, 2 from there.  us per step (B200, 128 x 6), tiles of
+// 128 / 256 / 512 / 1024 / 2048 / 4096, [] the rule's:
+//   22k cells [32] / 43 / 64 / 107 / 190 / 344; 424k 141 / 114 / [109] / 172 / 279 / 497; 600k 256: 157 /
+//   [139] / 181; 866k 512: 207 / [206] / 329; 1.2M 512: 271 / [254] / 338; 1.7M 512: 385 / [359] / 373 / 621;
+//   2.5M 1024: 521 / [506] / 649; 3.4M 1024: 757 / [731] / 760; 5.0M 2048: 996 / [986]; 12.2M 2500 / [2451].
+int queue_tile_rule(int64_t cells, int v)
 {
-    const int64_t ctas = 148 * 6;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
+    const int64_t ctas = (int64_t)sms * kQueueVariants[v].minb;
     int tile = 128;
-    while (tile < 4096 && (int64_t)tile * ctas * 3 < cells * 2) tile *= 2;
+    while (tile < 4096 && 2 * cells > (tile < 1024 ? 3 : 4) * tile * ctas) tile *= 2;
     return tile;
 }
 

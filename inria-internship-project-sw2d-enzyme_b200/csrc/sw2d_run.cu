@@ -623,6 +623,10 @@ const void* run_fn(const sw2d_handle* h, bool pairs)
 }
 
 constexpr int64_t kRunCellsMax = 66000;  // above it no tile fits (see the figures at the top)
+// Least cells of a tile: fewer take more SMs (and the exchanges more readers) for a shorter chain per CTA.
+// us per step with least tiles of 32 / 64 / 96 / 128 cells: MUSCL-EVR 500 cells 7.3 / 7.4 / 8.0 / 8.3, 2,000
+// 7.8 / 7.8 / 8.4 / 9.0, 5,000 8.1 / 8.1 / 8.9 / 9.3; Godunov 2,000 5.9 / 5.8 / 6.2 / 6.2, 5,000 6.2 / 5.9 / 6.5 /
+// 6.7.  At 64 up to four meshes of 2,000 cells share the chip.
 constexpr int kRunTileLeast = 64;
 constexpr int kRunSmemMax = 220 * 1024;
 
