@@ -81,29 +81,20 @@ public:
         return std::min(free_b / part, share);
     }
 
-    // a buffer of each size on the current device, in place of what it held; false: none of them
-    bool take(const std::vector<size_t>& sizes, std::vector<void*>& out)
+    // a buffer of `bytes` on the current device in place of what it held, or null
+    void* take(size_t bytes)
     {
         std::lock_guard<std::mutex> lock(pool().mu);
         free_all();
-        out.clear();
-        size_t free_b = 0, share = 0, sum = 0;
-        for (size_t n : sizes) sum += n;
-        if (cudaGetDevice(&device_) != cudaSuccess || !share_left(device_, free_b, share) || sum > share) return false;
+        size_t free_b = 0, share = 0;
+        if (cudaGetDevice(&device_) != cudaSuccess || !share_left(device_, free_b, share) || bytes > share) return nullptr;
+        void* p = nullptr;
+        if (taken(cudaMalloc(&p, request_bytes(bytes))) != cudaSuccess) return nullptr;
         pool().holders.push_back(this);
-        for (size_t n : sizes) {
-            void* p = nullptr;
-            if (taken(cudaMalloc(&p, request_bytes(n))) != cudaSuccess) {
-                free_all();
-                out.clear();
-                return false;
-            }
-            buffers_.push_back(p);
-            bytes_ += n;
-            out.push_back(p);
-        }
+        buffer_ = p;
+        bytes_ = bytes;
         lost_ = false;
-        return true;
+        return p;
     }
 
     void drop()
@@ -167,15 +158,16 @@ private:
     {
         auto& all = pool().holders;
         all.erase(std::remove(all.begin(), all.end(), this), all.end());
-        for (void* p : buffers_) cudaFree(p);
-        if (!buffers_.empty()) forget_(owner_);
-        buffers_.clear();
+        if (!buffer_) return;
+        cudaFree(buffer_);
+        forget_(owner_);
+        buffer_ = nullptr;
         bytes_ = 0;
     }
 
     void* owner_;
     void (*forget_)(void*);
-    std::vector<void*> buffers_;
+    void* buffer_ = nullptr;
     size_t bytes_ = 0;
     int device_ = 0;
     int uses_ = 0;

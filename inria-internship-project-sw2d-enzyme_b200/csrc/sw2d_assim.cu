@@ -1180,10 +1180,8 @@ int seg_buffers(sw2d_handle* h)
     // the slopes too, within half of the free device memory and the share of all handles (else the
     // reverse steps rebuild them: 10k cells, 134 steps, 0.7 ms more per gradient)
     const size_t bytes = (size_t)a->seg_cap * h->nc * sizeof(double2);
-    std::vector<void*> p;
-    if (h->p.scheme == SW2D_SCHEME_MUSCL_EVR && (grows || a->slopes.lost()) && bytes <= OptionalMemory::room(2) &&
-        a->slopes.take({bytes}, p))
-        a->seg_slope = static_cast<double2*>(p[0]);
+    if (h->p.scheme == SW2D_SCHEME_MUSCL_EVR && (grows || a->slopes.lost()) && bytes <= OptionalMemory::room(2))
+        a->seg_slope = static_cast<double2*>(a->slopes.take(bytes));
     return SW2D_OK;
 }
 

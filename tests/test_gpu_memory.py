@@ -57,8 +57,8 @@ def test_gradient(pkg, scheme):
         J, g = model.adjoint()
         return [np.float64(J)] + [g[k] for k in sorted(g)]
 
-    # slopes (MUSCL-EVR), Riemann states, the edges' sides, and the kept segments' arrays
-    assert _failing_in_turn(pkg, lambda: pkg.SpModel(case), act) >= (3 + 4 if scheme == "muscl_evr" else 2 + 3)
+    # slopes (MUSCL-EVR), Riemann states, the edges' sides, and the kept segments
+    assert _failing_in_turn(pkg, lambda: pkg.SpModel(case), act) >= (3 + 1 if scheme == "muscl_evr" else 2 + 1)
 
 
 @pytest.mark.parametrize("scheme", ["muscl_evr", "godunov"])
@@ -151,6 +151,8 @@ def test_kept_memory_gives_way(pkg):
         finally:
             fails(0, 0)
         assert model.get_option("kept_bytes") == 0
+        act()                            # and later it is
+        assert model.get_option("kept_bytes") == held[model is b]
         assert all(np.array_equal(_bits(x), _bits(y)) for x, y in zip(got, want))
     net.close()
     a.close()
@@ -235,3 +237,17 @@ def test_training_buffers(pkg):
     assert free[0] - free[-1] <= 4 << 20       # the last set is 10 % larger than the first, no more
     net.close()
     ref.close()
+
+
+def test_kept_segments_are_one_allocation(pkg):
+    case = pkg.workloads.dam_break(n_cells=600)
+    fails = pkg.capi.load_library().sw2d_test_fail_allocations
+    requests = []
+    for kept in (1, 3):
+        model = pkg.SpModel(case)
+        model.set_option("adjoint_kept_segments", kept)
+        fails(0, 0)
+        model.record(20, 6)
+        requests.append(fails(0, 0))
+        model.close()
+    assert requests[1] == requests[0] + 1
