@@ -241,10 +241,8 @@ struct sw2d_mlp {
     long long first_wait = kWaitPolls;  // sw2d_mlp_set_wait_polls
     int sms = 0;
     // fp32 master parameters, Adam moments; the gradient (result buffer of sw2d_mlp_loss_grad:
-    // gradient, loss partials, status word) and its host copy, pinned once the network trains on
-    float *p = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *pinned = nullptr;
-    std::vector<float> host;
-    int64_t batches = 0;
+    // gradient, loss partials, status word) and its pinned host copy
+    float *p = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr, *host = nullptr;
     float* part = nullptr;  // per-CTA partial gradients [parts x kPartStride]
     int64_t parts = 0;
     // bf16 operand copies: W1 [64 x 16] (inputs padded), W2 [64 x 64], W3 [16 x 64] (outputs padded),
@@ -707,20 +705,6 @@ int ensure_cap(sw2d_mlp* m, int64_t n)
 // floats of the result buffer of a batch of n rows: gradient, loss partials (256 rows each), status
 size_t result_floats(int64_t n) { return (size_t)sw2d::kNParams + (size_t)((n + 255) / 256) + 1; }
 
-// Where the result of n rows goes on the host.  Pinned memory takes 5 us off a batch (4,096 rows: 82 us
-// with ordinary memory) and 2.7 ms to allocate, twenty times a first batch, so it is had after kPinAfter
-// batches (36 KB: batches of up to 2^20 rows); without it ordinary memory serves.
-constexpr int64_t kPinAfter = 16;
-constexpr int64_t kPinnedRows = (int64_t)1 << 20;
-
-float* result_host(sw2d_mlp* m, int64_t n)
-{
-    if (n > kPinnedRows) return m->host.data();
-    if (++m->batches == kPinAfter && sw2d::pinned_malloc(&m->pinned, result_floats(kPinnedRows) * sizeof(float)) != cudaSuccess)
-        m->pinned = nullptr;
-    return m->pinned ? m->pinned : m->host.data();
-}
-
 // Training buffers for n rows: the new ones first, so that a batch they cannot be had for leaves the old
 // ones to smaller batches, then the old ones freed
 int ensure_train(sw2d_mlp* m, int64_t n)
@@ -729,12 +713,14 @@ int ensure_train(sw2d_mlp* m, int64_t n)
     if (n <= m->tcap) return SW2D_OK;
     const int64_t parts = std::max(m->parts, std::min<int64_t>((n + kTileM - 1) / kTileM, m->sms));  // one per CTA
     const size_t first = m->allocs.size();
-    float *part = nullptr, *traw = nullptr, *t = nullptr, *se = nullptr, *grad = nullptr;
+    float *host = nullptr, *part = nullptr, *traw = nullptr, *t = nullptr, *se = nullptr, *grad = nullptr;
+    MCK(pinned_malloc(&host, result_floats(n) * sizeof(float)));
     int rc = SW2D_OK;
     if ((parts > m->parts && (rc = malloc_dev(m, parts * kPartStride, &part))) || (rc = malloc_dev(m, n * kIn, &traw)) ||
         (rc = malloc_dev(m, n * kOut, &t)) || (rc = malloc_dev(m, n, &se)) || (rc = malloc_dev(m, result_floats(n), &grad))) {
         for (size_t i = first; i < m->allocs.size(); i++) cudaFree(m->allocs[i]);
         m->allocs.resize(first);
+        cudaFreeHost(host);
         return rc;
     }
     auto replace = [&](float*& old, float* now) {
@@ -749,7 +735,8 @@ int ensure_train(sw2d_mlp* m, int64_t n)
     replace(m->t, t);
     replace(m->se, se);
     replace(m->grad, grad);
-    m->host.resize(result_floats(n));
+    if (m->host) cudaFreeHost(m->host);
+    m->host = host;
     m->parts = parts;
     m->tcap = n;
     return SW2D_OK;
@@ -835,7 +822,7 @@ int sw2d_mlp_destroy(sw2d_mlp* m)
     cudaSetDevice(m->device);
     if (m->stream) cudaStreamSynchronize(m->stream);
     for (void* p : m->allocs) cudaFree(p);
-    if (m->pinned) cudaFreeHost(m->pinned);
+    if (m->host) cudaFreeHost(m->host);
     if (m->stream) cudaStreamDestroy(m->stream);
     delete m;
     return SW2D_OK;
@@ -935,19 +922,18 @@ int sw2d_mlp_loss_grad(sw2d_mlp* m, const float* features, const float* targets,
     const int nbp = (kNParams + 255) / 256, nbl = (int)((n + 255) / 256);
     k_mlp_reduce<<<nbp + nbl, 256, 0, m->stream>>>(m->part, grid, nbp, m->se, n, m->grad, m->status, nbl);
     MCK(cudaGetLastError());
-    float* host = result_host(m, n);
-    MCK(cudaMemcpyAsync(host, m->grad, result_floats(n) * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+    MCK(cudaMemcpyAsync(m->host, m->grad, result_floats(n) * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
     MCK(cudaStreamSynchronize(m->stream));
     unsigned st = 0;
-    std::memcpy(&st, host + kNParams + nbl, sizeof(st));
+    std::memcpy(&st, m->host + kNParams + nbl, sizeof(st));
     if (st) {
         // reported once: the kernel that ran out freed its TMEM, and the object stays usable
         MCK(cudaMemset(m->status, 0, sizeof(unsigned)));
         return mlp_fail(m, SW2D_E_CUDA, "tensor-core wait ran out");
     }
-    if (grad_out) std::memcpy(grad_out, host, kNParams * sizeof(float));
+    if (grad_out) std::memcpy(grad_out, m->host, kNParams * sizeof(float));
     double s = 0.0;
-    for (int i = 0; i < nbl; i++) s += host[kNParams + i];
+    for (int i = 0; i < nbl; i++) s += m->host[kNParams + i];
     if (loss) *loss = s / (double)(n * kOut);
     return SW2D_OK;
 }
