@@ -122,10 +122,8 @@ def test_kept_memory_gives_way(pkg):
     net = pkg.closure.MLP(pkg.closure.init_params(0))
     x, t = np.zeros((300, 10), np.float32), np.zeros((300, 2), np.float32)
 
-    others = [(0, lambda: pkg.SpModel(case).close()), (0, lambda: _recorded(pkg, case).close()),
-              (1, lambda: net.loss_grad(x, t))]     # its first request is for host memory
-    for skip, other in others:
-        fails(skip, 1)
+    for other in (lambda: pkg.SpModel(case).close(), lambda: _recorded(pkg, case).close(), lambda: net.loss_grad(x, t)):
+        fails(0, 1)
         try:
             other()
         finally:
@@ -251,3 +249,24 @@ def test_kept_segments_are_one_allocation(pkg):
         requests.append(fails(0, 0))
         model.close()
     assert requests[1] == requests[0] + 1
+
+
+def test_training_without_pinned_memory(pkg):
+    """A first batch requests five device buffers, then pinned memory for its result, which ordinary memory
+    replaces where there is none; a larger batch asks again."""
+    C = pkg.closure
+    fails = pkg.capi.load_library().sw2d_test_fail_allocations
+    rng = np.random.default_rng(2)
+    x, t = rng.normal(size=(900, 10)).astype(np.float32), rng.normal(size=(900, 2)).astype(np.float32)
+    a, b = C.MLP(C.init_params(3)), C.MLP(C.init_params(3))
+    for n in (300, 200, 900):
+        out = []
+        for net, first in ((a, 5), (b, 0)):
+            fails(first, 1 if net is a and n == 300 else 0)
+            loss, g = net.loss_grad(x[:n], t[:n])
+            assert fails(0, 0) == {300: 6, 200: 0}.get(n, 6)
+            net.adam_step(1e-3)
+            out.append((loss, g, net.params))
+        assert out[0][0] == out[1][0] and all(np.array_equal(u, v) for u, v in zip(out[0][1:], out[1][1:]))
+    a.close()
+    b.close()
