@@ -1,7 +1,7 @@
 // sw2d_mlp.cu — the learned momentum-exchange closure: an MLP of 10 inputs -> 64 -> 64 -> 2
 // (GELU) whose inference and training run on the 5th-generation tensor cores (tcgen05, BF16
-// operands, FP32 accumulators in TMEM): one hand-written GEMM kernel for training and
-// stand-alone inference, and the DIP cell-update kernel with the network inside
+// operands, FP32 accumulators in TMEM): a GEMM kernel for stand-alone inference (k_umma_gemm), a
+// training kernel (k_mlp_train), and the DIP cell-update kernel with the network inside
 // (k_update_closure, further down) for the closure in a model's step.
 //
 // k_umma_gemm (stand-alone inference) computes, for a tile of 128 rows per CTA, D = A * B^T with

@@ -16,8 +16,10 @@
 //   - A state is read before its owner can write the next one: the owner first needs the next step's
 //     minimum of every CTA, which each publishes after it has read its rings: one slot.
 // Every wait is bounded; a wait that runs out sets the status word and ends the launch, and the call
-// reports it (the state is then undefined until it is set or restored).  The arithmetic is that of the four kernels (sp_phases.cuh,
-// tile_phases.cuh), operand for operand, so the results are the same bits.
+// reports it (the state is then undefined until it is set or restored).  The arithmetic is that of the
+// four kernels (sp_phases.cuh, tile_phases.cuh), operand for operand, so the results are the same bits,
+// and the four kernels serve wherever this one does not: no memory for the tiles or no room for them on
+// chip, a new handle's first steps (run_worth), other handles' calls in progress (RunTurn).
 //
 // A pair of lanes takes each slope and each internal edge while a tile's edges then still fit one pass
 // of the CTA (up to about 20k cells on 148 SMs): one component of the slope, one side's Riemann state.
