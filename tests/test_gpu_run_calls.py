@@ -139,7 +139,7 @@ def test_handles_in_several_threads(pkg, cells, threads, shares):
         th.join()
     alone.step(64 * 39)
     share = sum(m.get_option("run_steps") for m in models) / (threads * 40 * 64)
-    assert share > 0.9 if shares else share < 0.5      # a first and last calls, that others do not overlap
+    assert share > 0.9 if shares else share < 0.8      # first and last calls overlap fewer others
     assert all(_same_state(m, alone) and m.time == alone.time for m in models)
     models[0].step(64)                                 # alone again
     assert models[0].get_option("run_steps") >= 64
