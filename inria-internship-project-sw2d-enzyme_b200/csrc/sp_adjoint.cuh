@@ -783,12 +783,14 @@ SW2D_HD void slopes_rev_t(double zc, int n, const SlopeNbr* nb, double sxb, doub
         const bool sel_left = under ? mn_left : mx_left;
         const double f = under ? fmn : fmx;
         const double den = rec - zc;
-        const double rden = 1.0 / den;
-        const double fac = (f - zc) * rden;
+        // A factor of zero (the cell itself holds the bound) passes nothing on through den, also where the
+        // reciprocal or num_bar overflows: the products are ordered so that no 0 * inf arises there
+        const double rden = 1.0 / den, num = f - zc;
+        const double fac = num == 0.0 ? 0.0 : num * rden;
         const double fac_bar = sxb * sx0 + syb * sy0;
         double sx0_bar = sxb * fac, sy0_bar = syb * fac;
         const double num_bar = fac_bar * rden;
-        const double den_bar = -num_bar * fac;
+        const double den_bar = fac == 0.0 ? 0.0 : -fac_bar * fac * rden;
         // f = zL or zR ; num = f - zc ; den = rec - zc ; rec = zc + ax sx0 + ay sy0
         const bool f_is_c = sel_left ? !nb[k].c_is_r : nb[k].c_is_r;
         if (f_is_c) zc_bar += num_bar;
